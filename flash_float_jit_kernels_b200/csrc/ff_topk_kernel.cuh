@@ -90,6 +90,10 @@ __device__ __forceinline__ uint32_t dsmem_atomic_add_u32(uint32_t addr, uint32_t
   return old;
 }
 
+// The two halves of a cluster barrier (all threads of all CTAs execute both, in turn).
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 // ---- bulk asynchronous copies global -> shared, completion on an mbarrier -----
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -1687,6 +1691,12 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
       FF_TRACE(p, 21);
     }
   }
+  // A row of one cluster that is swept with a guess touches a peer's shared memory (the gather's
+  // reservation) without a histogram merge, and so without a cluster barrier, in front of it: every
+  // peer must have started and set its counters up by then.  Arrived here, waited for behind the sweep.
+  const bool hinted_cluster = kHinted && use_hint && C > 1 && G == 1;
+  bool peers_may_leave = true;   // false: a peer may still read this CTA's shared memory (see leave_cluster)
+  if (hinted_cluster) cluster_arrive();
   if (kHinted && use_hint) {
     stream_pass(ts, [&](uint32_t tile, int tt, int units) {
       collect_tile<T>(tile, units, chunk.fb + tt * kTileUnits, chunk.mis, hint, stage, kSortCap, &sh.stage_count);
@@ -1701,6 +1711,7 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
     }
     __syncthreads();
     FF_TRACE(p, 3);
+    if (hinted_cluster) cluster_wait();
     gather_stage(sh.stage_count, true);
     FF_TRACE(p, 4);
     int total;
@@ -1722,6 +1733,7 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
     } else if (C > 1) {
       cluster.sync();
       total = static_cast<int>(dsmem_ld_u32(dsmem_addr(smem_addr(&sh.sort_count), 0)));
+      peers_may_leave = false;
     } else {
       total = sh.sort_count;
     }
@@ -1739,11 +1751,17 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
       // a caller's guess that did not fit is reported; the row's own guess is its own business
       if (!self_seeded && p.status != nullptr && tid == 0 && my_share == 0) atomicOr(p.status, 8);
       if (C > 1 && G == 1) cluster.sync();   // every CTA has read the count before it is cleared
+      peers_may_leave = true;
       if (tid == 0) sh.sort_count = 0;
     }
     if (tid == 0) sh.stage_count = 0;
     __syncthreads();
   }
+  // The count was read from rank 0's shared memory: rank 0 must not exit before every CTA has read it.
+  if (kHinted && !peers_may_leave) cluster_arrive();
+  auto leave_cluster = [&]() {
+    if (kHinted && !peers_may_leave) cluster_wait();
+  };
 
   if (!hinted_done) {
   // ---- level 0: 13-bit histogram of the whole chunk -----------------------
@@ -2044,6 +2062,7 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
     }
     FF_TRACE(p, 25);
     leave_scratch();
+    leave_cluster();
     return sx_done;
   }
 
@@ -2239,6 +2258,7 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
   }
   FF_TRACE(p, 25);
   leave_scratch();
+  leave_cluster();
   return sx_done;
 }
 

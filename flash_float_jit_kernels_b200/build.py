@@ -158,8 +158,38 @@ def build_tvmffi_module(force: bool = False) -> Path:
     return out
 
 
+HOST_MODULE_NAME = "ff_host.so"   # CPython module: the operators' host path, bound to the libraries by address
+
+
+def host_module_path() -> Path:
+    return CSRC / HOST_MODULE_NAME
+
+
+def build_host_module(force: bool = False) -> Path:
+    """Compile ``csrc/ff_host.cc`` (host code, g++, torch headers) into the CPython module ``csrc/ff_host.so``."""
+    import sysconfig
+
+    import torch
+    out = host_module_path()
+    src = CSRC / "ff_host.cc"
+    deps = [src, INCLUDE / "ff_topk.h", INCLUDE / "ff_indexer_logits.h"]
+    if not force and out.exists() and all(d.stat().st_mtime <= out.stat().st_mtime for d in deps if d.exists()):
+        return out
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parent.parent
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-o", str(out), str(src),
+           f"-I{root / 'include'}", f"-I{root / 'include/torch/csrc/api/include'}", f"-I{sysconfig.get_paths()['include']}",
+           f"-I{cuda / 'include'}", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           f"-L{root / 'lib'}", "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10", f"-Wl,-rpath,{root / 'lib'}"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
+    return out
+
+
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_host_module(force="--force" in sys.argv))
     print(build_indexer_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
     print(build_tvmffi_module(force="--force" in sys.argv))
     if "--checked" in sys.argv:

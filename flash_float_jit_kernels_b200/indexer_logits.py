@@ -16,6 +16,7 @@ from typing import Optional
 
 import torch
 
+from . import _host
 from .build import indexer_lib_path
 from ._lib import LibraryMissingError
 from .topk_indexer import TopkArgumentError, _ptr, _require, _stream_ptr
@@ -51,6 +52,12 @@ def load() -> ctypes.CDLL:
         fn.restype = restype
         fn.argtypes = argtypes
     return lib
+
+
+def raise_error(rc: int) -> None:
+    """Turns a non-zero return code of the library into the exception the operator documents."""
+    message = f"indexer_logits_fp8: {load().ff_indexer_last_error_string().decode()}"
+    raise TopkArgumentError(message) if rc < 0 else RuntimeError(message)
 
 
 def new_handover(B: int, device) -> torch.Tensor:
@@ -91,6 +98,9 @@ def indexer_logits_fp8(q: torch.Tensor, k: torch.Tensor, w: torch.Tensor, length
         (B, L) float32; positions ``>= lengths[b]`` that fall into a processed 128-key tile hold
         ``-inf``, later ones keep what ``out`` held (a fresh result is filled with ``-inf``).
     """
+    result = _host.logits()(q, k, w, lengths, out, status, ctas_per_row, threshold_hint, handover)
+    if result is not None:
+        return result
     _require(q.is_cuda and k.is_cuda and w.is_cuda and lengths.is_cuda, "all tensors must be CUDA tensors")
     _require(q.element_size() == 1 and k.element_size() == 1, "q and k must be fp8 (one byte per element)")
     _require(q.dim() == 3 and q.shape[1:] == (HEADS, HEAD_DIM) and q.is_contiguous(), "q must be contiguous [B, 64, 128]")
@@ -117,10 +127,8 @@ def indexer_logits_fp8(q: torch.Tensor, k: torch.Tensor, w: torch.Tensor, length
             lengths.data_ptr(), out.data_ptr(), out.stride(0) if B > 1 else max(out.stride(0), L), B, L,
             int(ctas_per_row), None if handover is None else threshold_hint.data_ptr(), _ptr(handover),
             _ptr(status), _stream_ptr(q.device))
-    if rc < 0:
-        raise TopkArgumentError(f"indexer_logits_fp8: {lib.ff_indexer_last_error_string().decode()}")
-    if rc > 0:
-        raise RuntimeError(f"indexer_logits_fp8: {lib.ff_indexer_last_error_string().decode()}")
+    if rc != 0:
+        raise_error(rc)
     return out
 
 

@@ -21,7 +21,7 @@ from typing import Optional
 
 import torch
 
-from . import _lib
+from . import _host, _lib
 
 
 class TopkArgumentError(AssertionError, ValueError):
@@ -131,6 +131,10 @@ def fast_topk_v3(
         (B, topk) int32 indices in (value desc, index asc) order, ``-1``
         padded for rows shorter than ``topk``.
     """
+    result = _host.topk()(score, lengths, topk, row_starts, out, status, threshold_hint, index_dtype, handover)
+    if result is not None:
+        return result
+    # not plain valid arguments: the full checks raise, or the call is made from here
     _check_common(score, lengths, topk, row_starts, dtypes=tuple(_SCORE_DTYPES))
     lib = _lib.load()
     B, L = score.size(0), score.size(1)
@@ -209,6 +213,8 @@ def fast_topk_transform_fused(
     whose ``cu_seqlens_q`` interval contains row ``i``.  ``k`` is
     ``dst_page_table.size(1)`` (the reference fixes it to 2048).
     """
+    if _host.transform()(score, lengths, dst_page_table, row_starts, src_page_table, cu_seqlens_q, None):
+        return
     _require(dst_page_table.dim() == 2 and dst_page_table.is_contiguous(),
              "dst_page_table must be contiguous 2-D")
     topk = int(dst_page_table.size(1))
@@ -251,6 +257,8 @@ def fast_topk_transform_ragged_fused(
     Mirrors ``fast_topk_transform_ragged_interface``
     (``topk_indexer_radix.cu:1602-1639``).
     """
+    if _host.transform()(score, lengths, topk_indices_ragged, row_starts, None, None, topk_indices_offset):
+        return
     _require(topk_indices_ragged.dim() == 2 and topk_indices_ragged.is_contiguous()
              and topk_indices_ragged.dtype == torch.int32,
              "topk_indices_ragged must be contiguous int32 2-D")

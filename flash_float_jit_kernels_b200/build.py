@@ -18,7 +18,7 @@ CSRC = Path(__file__).resolve().parent / "csrc"
 INCLUDE = Path(__file__).resolve().parent.parent / "include"
 LIB_NAME = "libff_topk.so"
 SOURCES = ["ff_topk.cu"]
-HEADERS = ["ff_topk_common.cuh", "ff_topk_kernel.cuh", "ff_cp_exchange.cuh"]
+HEADERS = ["ff_topk_common.cuh", "ff_topk_kernel.cuh", "ff_topk_rows.cuh", "ff_cp_exchange.cuh"]
 INDEXER_LIB_NAME = "libff_indexer.so"      # the logit producer: its own library and header
 INDEXER_SOURCES = ["ff_indexer_logits.cu"]
 

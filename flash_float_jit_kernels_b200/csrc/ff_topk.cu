@@ -11,6 +11,7 @@
 #include <mutex>
 
 #include "ff_topk_kernel.cuh"
+#include "ff_topk_rows.cuh"
 
 namespace {
 
@@ -106,6 +107,10 @@ int max_cluster_for(K kernel) {
   return 1;
 }
 
+using RowsKernel = void (*)(const ff::RowsParams);
+RowsKernel rows_kernel(int threads, int dtype, bool hints);
+int rows_smem(int threads, bool hints);
+
 void init_device(int device) {
   int prev = 0;
   cudaError_t e = cudaGetDevice(&prev);
@@ -123,6 +128,12 @@ void init_device(int device) {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ff::cp_merge_sorted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              ff::kMaxPeers * ff::kMaxK * static_cast<int>(sizeof(uint32_t)));
+  for (int threads : {256, 1024})
+    for (int dtype : {FF_DTYPE_F32, FF_DTYPE_BF16, FF_DTYPE_F16})
+      for (int hints : {0, 1})
+        if (e == cudaSuccess)
+          e = cudaFuncSetAttribute(rows_kernel(threads, dtype, hints != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   rows_smem(threads, hints != 0));
   if (e == cudaSuccess) {
     g_max_cluster[device] = max_cluster_for(ff::topk_cluster_kernel<false, ff::kModePlain>);
     for (int i = 0; i < 5; ++i)
@@ -161,10 +172,12 @@ int choose_cluster(int device, int32_t B, int64_t L_width, int32_t k) {
   if (c == 0) {
     // Measured on B200: the widest cluster is fastest at every row length down
     // to 4 Ki (the finish is shared out over the cluster), so take the largest
-    // size that keeps the whole batch in one wave of CTAs (one CTA per SM).
+    // size of which the device holds one for every row at the same time (fewer than the SM count
+    // says: a cluster lives inside one group of SMs.  8 rows of 120,000 columns in clusters of 16 took two waves,
+    // 26.5 us, and take 14 in clusters of 8).
     c = ff::kMaxCluster;
     int fit = 1;
-    while (fit * 2 * static_cast<int64_t>(B) <= g_sm_count[device] && fit < ff::kMaxCluster) fit *= 2;
+    for (int log2c = 1; log2c < 5 && B <= g_active_clusters[device][log2c]; ++log2c) fit = 1 << log2c;
     if (c > fit) c = fit;
   }
   if (c > ff::kMaxCluster) c = ff::kMaxCluster;
@@ -270,6 +283,79 @@ int launch(const ff::TopkParams& p, int cluster, cudaStream_t stream, int dtype 
   if (e != cudaSuccess) return fail_cuda(e, "cudaLaunchKernelEx(topk_cluster_kernel)");
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;
+}
+
+// The one-CTA-per-row kernels (ff_topk_rows.cuh), by score type, CTA size and guesses.
+// Lists of 2,560 and 3,072 survivors: k, a margin inside the threshold digit, room to spare; a caller's guess may
+// let 4,096 through.
+int rows_cap(int threads, bool hints) { return hints ? ff::kSortCap : threads == 256 ? 256 * 10 : 1024 * 3; }
+int rows_block(int threads, bool hints) { return threads == 256 && hints ? 512 : threads; }
+template <typename T>
+RowsKernel rows_kernel(int threads, bool hints) {
+  if (threads == 256) return hints ? ff::topk_rows_kernel<T, 512, 8, 2, true> : ff::topk_rows_kernel<T, 256, 10, 4, false>;
+  return hints ? ff::topk_rows_kernel<T, 1024, 4, 1, true> : ff::topk_rows_kernel<T, 1024, 3, 1, false>;
+}
+RowsKernel rows_kernel(int threads, int dtype, bool hints) {
+  return dtype == FF_DTYPE_BF16 ? rows_kernel<__nv_bfloat16>(threads, hints)
+                                : dtype == FF_DTYPE_F16 ? rows_kernel<__half>(threads, hints) : rows_kernel<float>(threads, hints);
+}
+int rows_smem(int threads, bool hints) { return ff::rows_smem_bytes(rows_cap(threads, hints)); }
+
+int launch_rows(const ff::TopkParams& p, int threads, cudaStream_t stream, int dtype) {
+  ff::RowsParams q = {};
+  q.scores = p.scores;
+  q.row_stride = p.row_stride;
+  q.lengths = p.lengths;
+  q.row_starts = p.row_starts;
+  q.out_idx = p.out_idx;
+  q.out_idx64 = p.out_idx64;
+  q.B = p.B;
+  q.k = p.k;
+  q.L_width = p.L_width;
+  q.epilogue = p.epilogue;
+  q.n_table_rows = p.n_table_rows;
+  q.table = p.table;
+  q.table_stride = p.table_stride;
+  q.cu_seqlens_q = p.cu_seqlens_q;
+  q.offsets = p.offsets;
+  q.status = p.status;
+  q.hint_in = p.hint_in;
+  q.hint_out = p.hint_out;
+  q.handover = p.handover;
+  q.trace = g_trace.load(std::memory_order_relaxed);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(p.B), 1, 1);
+  const bool hints = p.hint_in != nullptr || p.hint_out != nullptr;
+  cfg.blockDim = dim3(static_cast<unsigned>(rows_block(threads, hints)), 1, 1);
+  cfg.dynamicSmemBytes = static_cast<size_t>(rows_smem(threads, hints));
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  if (programmatic_launch_enabled()) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 1;
+  }
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, rows_kernel(threads, dtype, hints), q);
+  if (e != cudaSuccess) return fail_cuda(e, "cudaLaunchKernelEx(topk_rows_kernel)");
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return 0;
+}
+
+// CTA size of the one-CTA-per-row kernel for this batch, or 0: rows get a cluster or several (also whenever a
+// launch shape is forced).  Measured on B200 (k = 2048): up to one row per SM a CTA of 1024 threads, which takes
+// 8.6 us for 4 Ki columns, 9.6 for 16 Ki, 11.9 for 32 Ki and 16.0 for 64 Ki; a cluster takes 12.6 / 12.7 / 13.1 / 13.8
+// with sixteen CTAs, and more with the fewer CTAs that larger batches leave for a row (64 rows of 64 Ki: 18.6).
+// Beyond that four CTAs of 256 threads per SM (296 rows of 16 Ki: 15.0 us against 19.1), unless a second
+// row per SM is all there is and the rows are long (296 rows of 64 Ki: 41 against 38).
+int choose_rows_threads(int device, int32_t B, int64_t L_width) {
+  if (g_cluster_override.load() != 0 || g_groups_override.load() != 0) return 0;
+  const int sms = g_sm_count[device];
+  if (B <= sms) {
+    const int64_t longest = B <= 8 ? 40960 : B <= 18 ? 49152 : B <= 37 ? 40960 : B <= 74 ? 98304 : 0x7fffffff;
+    return L_width <= longest ? 1024 : 0;
+  }
+  return B <= 2 * sms && L_width > 49152 ? 1024 : 256;
 }
 
 // Built-in scratch for ff_topk_launch_static: enough for FF_TOPK_STATIC_MAX_ROWS
@@ -448,6 +534,8 @@ int transform_launch_impl(const void* scores_any, int dtype, int64_t row_stride,
     static_assert(FF_TOPK_HANDOVER_ROW_BYTES == ff::kHandoverRowBytes, "hand-over layout");
     p.handover = static_cast<unsigned char*>(handover);
   }
+  if (const int threads = choose_rows_threads(device, B, L_width))
+    return launch_rows(p, threads, static_cast<cudaStream_t>(stream), dtype);
   int cluster = choose_cluster(device, B, L_width, k);
   if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
     p.groups = choose_groups(device, B, L_width, workspace_bytes, &cluster, hint_in != nullptr);

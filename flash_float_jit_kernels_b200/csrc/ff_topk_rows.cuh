@@ -1,0 +1,780 @@
+// One CTA per row, several rows per SM: the exact select for batches of many rows (prefill) and for
+// short rows, where a cluster's barriers cost more than its CTAs save.
+//
+//   sweep 1   12-bit histogram of the row (plain 128-bit loads, one shared-memory add per score)
+//   threshold one suffix scan; every bin at or above the threshold digit keeps (elements above it, elements in it)
+//   sweep 2   scores not below a cut inside the threshold digit -> survivor list.  The cut is interpolated from
+//             the digit's count with a margin, so that little more than k survive; a cut that turns
+//             out too high is replaced by the digit's lower edge
+//   finish    counting sort of the survivors in one pass of bins: a survivor's bin is its EXPECTED rank
+//             (elements above its digit + its position inside the digit, interpolated), at two bins
+//             per survivor, so that buckets hold one or two entries whatever the scores' distribution;
+//             exact rank inside the bucket by counting; indices leave through shared memory
+//
+// What bounds it: latency of a dozen dependent shared-memory phases per row, so that registers and shared
+// memory are kept small enough for four rows per SM, and each phase issues a thread's loads together.
+#pragma once
+
+#include "ff_topk_kernel.cuh"
+
+namespace ff {
+
+struct RowsParams {
+  const void* scores;
+  int64_t row_stride;
+  const int32_t* lengths;
+  const int32_t* row_starts;
+  int32_t* out_idx;
+  int64_t* out_idx64;
+  int32_t B, k;
+  int64_t L_width;
+  int32_t epilogue;
+  int32_t n_table_rows;
+  const int32_t* table;
+  int64_t table_stride;
+  const int32_t* cu_seqlens_q;
+  const int32_t* offsets;
+  int32_t* status;
+  const float* hint_in;
+  float* hint_out;
+  unsigned char* handover;
+  unsigned long long* trace;   // stage stamps, as in TopkParams
+};
+
+constexpr int kRowsBits = 12;                     // first digit: sign, exponent, three mantissa bits
+constexpr int kRowsBins = 1 << kRowsBits;
+constexpr int kRowsShift = 32 - kRowsBits;
+
+// Shared memory of a CTA whose list holds `cap` survivors, in two regions:
+//   histogram, then the bucketed survivors (32 bits each)
+//   list (64 bits each), then two finish bins per survivor (32 bits each), then the ranked positions
+__host__ __device__ constexpr int rows_smem_bytes(int cap) { return kRowsBins * 4 + cap * 8; }
+static_assert(kRowsBins >= kSortCap, "the bucketed survivors take the histogram's place");
+
+struct RowsShared {
+  int warp_tot[3][32];
+  int t, above, total;     // threshold digit, elements above it, elements at or above it
+  int max_bin;             // largest bin at or above the threshold
+  int count;               // survivors listed
+  uint32_t value_bits;     // OR of the survivors' score bits
+  uint32_t kmin, kmax;     // bounds of the survivors' keys (rebuilt bins only)
+};
+
+// Sum of v over all threads of higher index; `total`: over all threads.  One barrier; calls that
+// follow each other without a barrier in between need different warp_tot arrays.
+template <int NT>
+__device__ __forceinline__ int suffix_exclusive(int v, int* warp_tot, int& total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int s = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int o = __shfl_down_sync(0xffffffffu, s, off);
+    if (lane + off < 32) s += o;
+  }
+  if (lane == 0) warp_tot[wid] = s;
+  __syncthreads();
+  const int w = lane < NT / 32 ? warp_tot[lane] : 0;
+  int ws = w;
+#pragma unroll
+  for (int off = 1; off < NT / 32; off <<= 1) {
+    const int o = __shfl_down_sync(0xffffffffu, ws, off);
+    if (lane + off < 32) ws += o;
+  }
+  total = __shfl_sync(0xffffffffu, ws, 0);
+  return s - v + __shfl_sync(0xffffffffu, ws - w, wid);
+}
+
+// key_of() in four instructions: the add maps -0.0 to +0.0 and every NaN to 0x7fffffff.
+__device__ __forceinline__ uint32_t fast_key(float x) {
+  const uint32_t u = __float_as_uint(__fadd_rn(x, 0.0f));
+  return u ^ (static_cast<uint32_t>(static_cast<int32_t>(u) >> 31) | 0x80000000u);
+}
+// Digit in sign-magnitude order, as the histogram is filled.
+__device__ __forceinline__ uint32_t rows_raw_digit(float x) { return __float_as_uint(__fadd_rn(x, 0.0f)) >> kRowsShift; }
+
+// A listed survivor: score bits and position.
+__device__ __forceinline__ uint64_t list_entry(float x, int pos) {
+  return (static_cast<uint64_t>(__float_as_uint(x)) << 32) | static_cast<uint32_t>(pos);
+}
+
+// A packed bin: twice the elements above it << 19 | twice the elements in it (cut: rows with so many in
+// one of the bins that matter do not use them).
+constexpr int kPackShift = 19;
+constexpr int kPackMax = (1 << (kPackShift - 1)) - 1;   // elements in a bin
+
+// Suffix scan of the bins in monotone order (raw: the array is in rows_raw_digit() order).  Every non-empty bin
+// with fewer than `limit` elements above it is packed in place, and the bin that reaches the limit
+// is published as sh.t with its counts.
+template <int NT>
+__device__ __forceinline__ void pack_bins(uint32_t* hist, bool raw, int limit, RowsShared& sh, int* warp_tot) {
+  constexpr int per = kRowsBins / NT;
+  const int tid = threadIdx.x;
+  const int m0 = tid * per;
+  const bool up = !raw || m0 >= kRowsBins / 2;   // the thread's bins lie in ascending order
+  const int base = !raw ? m0 : up ? m0 - kRowsBins / 2 : kRowsBins - per - m0;
+  int local = 0;
+#pragma unroll
+  for (int j = 0; j < per / 4; ++j) {            // rotated so that eight threads read eight different bank groups
+    const int q = (j + tid / (32 / per)) & (per / 4 - 1);
+    const uint4 v = *reinterpret_cast<const uint4*>(hist + base + 4 * q);
+    local += static_cast<int>(v.x + v.y + v.z + v.w);
+  }
+  int total;
+  int running = suffix_exclusive<NT>(local, warp_tot, total);
+  if (local > 0 && running < limit) {
+    uint32_t c[per];
+#pragma unroll
+    for (int q = 0; q < per / 4; ++q) {
+      const uint4 v = *reinterpret_cast<const uint4*>(hist + base + 4 * q);
+      c[4 * q] = v.x;
+      c[4 * q + 1] = v.y;
+      c[4 * q + 2] = v.z;
+      c[4 * q + 3] = v.w;
+    }
+    int largest = 0;
+#pragma unroll
+    for (int i = 0; i < per; ++i) {              // from the thread's largest digit down
+      const int n = static_cast<int>(up ? c[per - 1 - i] : c[i]);
+      if (n != 0 && running < limit) {
+        hist[base + (up ? per - 1 - i : i)] = (static_cast<uint32_t>(running) << (kPackShift + 1)) |
+                                              static_cast<uint32_t>(2 * min(n, kPackMax));
+        largest = max(largest, n);
+        if (running + n >= limit) {
+          sh.t = m0 + per - 1 - i;
+          sh.above = running;
+          sh.total = running + n;
+        }
+        running += n;
+      }
+    }
+    atomicMax(&sh.max_bin, largest);
+  }
+  __syncthreads();
+}
+
+// A row's scores in groups of 16 per thread (four units of 4 or two units of 8), NT threads apart.
+// FULL: every unit of the group is inside the row.
+template <typename T, int NT>
+struct RowGroup {
+  static constexpr int kPU = Elem<T>::kPerUnit;
+  static constexpr int kUnits = 16 / kPU;
+  static constexpr int kStep = NT * kUnits;
+  uint4 w[kUnits];
+  template <bool FULL>
+  __device__ __forceinline__ void load(const Chunk<T>& c, int u0) {
+    const uint4* p4 = reinterpret_cast<const uint4*>(c.abase) + (u0 + static_cast<int>(threadIdx.x));
+#pragma unroll
+    for (int i = 0; i < kUnits; ++i)
+      if (FULL || u0 + static_cast<int>(threadIdx.x) + i * NT < c.fe) w[i] = __ldg(p4 + i * NT);
+  }
+  __device__ __forceinline__ void load(const Chunk<T>& c, int u0) {
+    if (u0 + kStep <= c.fe) load<true>(c, u0); else load<false>(c, u0);
+  }
+  // f(score, element of the group) for every score that is there
+  template <bool FULL, typename F>
+  __device__ __forceinline__ void each(const Chunk<T>& c, int u0, F&& f) const {
+#pragma unroll
+    for (int i = 0; i < kUnits; ++i) {
+      if (FULL || u0 + static_cast<int>(threadIdx.x) + i * NT < c.fe) {
+        float x[kPU];
+        unpack_unit<T>(w[i], x);
+#pragma unroll
+        for (int e = 0; e < kPU; ++e) f(x[e], kPU * i + e);
+      }
+    }
+  }
+  // Position of element 0; element e lies at a constant distance from it.
+  static __device__ __forceinline__ int position(const Chunk<T>& c, int u0) {
+    return kPU * (u0 + static_cast<int>(threadIdx.x)) - c.mis;
+  }
+  static __device__ __forceinline__ constexpr int distance(int e) { return (e / kPU) * kPU * NT + (e & (kPU - 1)); }
+};
+
+// Where to cut inside the threshold digit so that a few more than the `wanted` largest of its `in_bin` scores are
+// kept: the density of scores is taken as linear over the digit, from its own count and the next
+// digit's (c0, c1): above a point x of the way down lie (c0 + c1) / 2 x + (c0 - c1) / 2 x^2 of them,
+// solved for the wanted count plus a margin (the steps of scores rounded to bf16,
+// sixteen to a digit, and four standard deviations).  Returns key bits above the digit's lower edge;
+// keep: how many are expected (less than wanted: they do not fit in `room`); linear: how many there would be
+// if the scores were spread evenly over the digit, as the finish takes them to be.
+__device__ __forceinline__ uint32_t cut_in_digit(const uint32_t* packed, int t, int in_bin, int wanted, int room, int& keep, int& linear) {
+  const float c0 = static_cast<float>(in_bin);
+  const int margin = (in_bin >> 4) + static_cast<int>(2.f * sqrtf(c0)) + 8;
+  keep = min(in_bin, wanted + margin);
+  if (keep > room) keep = room >= wanted + (margin >> 1) ? room : -1;
+  const int up = t + 1;
+  float c1 = static_cast<float>((packed[up >= kRowsBins / 2 ? up - kRowsBins / 2 : kRowsBins - 1 - up] &
+                                 ((1u << kPackShift) - 1u)) >> 1);
+  if ((up & 7) == 0) c1 *= up >= kRowsBins / 2 ? 0.5f : 2.f;   // the next digit spans a step of another width
+  c1 = fminf(c1, 3.f * c0);
+  const float b = 0.5f * (c0 + c1), a = 0.5f * (c0 - c1), want = static_cast<float>(keep);
+  const float x = 2.f * want / (b + sqrtf(fmaxf(b * b + 4.f * a * want, 0.f)));
+  const bool all = keep >= in_bin || !(x < 1.f);
+  linear = all ? in_bin : min(in_bin, static_cast<int>(x * c0) + 2);
+  return all ? 0u : static_cast<uint32_t>((1.f - x) * static_cast<float>(1 << kRowsShift));
+}
+
+// The rare rows whose survivors do not fit the list (heavy ties, scores crowded into one digit): further
+// digits of the composite, one sweep each, until they fit.  Returns the smallest composite that
+// goes to the finish.
+__host__ __device__ constexpr int rows_level_bits(int l) { return l <= 2 ? 10 : l == 5 ? 10 : 11; }
+__host__ __device__ constexpr int rows_level_shift(int l) { return l == 0 ? 52 : l == 1 ? 42 : l == 2 ? 32 : l == 3 ? 21 : l == 4 ? 10 : 0; }
+template <typename T, int NT>
+__device__ __noinline__ uint64_t deeper_digits(const Chunk<T>& c, uint32_t* hist, int k, int cap, RowsShared& sh, int32_t* status) {
+  const int tid = threadIdx.x;
+  uint64_t prefix = static_cast<uint64_t>(sh.t);
+  int r = k - sh.above;
+#pragma unroll 1
+  for (int level = 1;; ++level) {
+    const int bits = rows_level_bits(level), shift = rows_level_shift(level), above_shift = rows_level_shift(level - 1);
+    const uint32_t mask = (1u << bits) - 1u;
+    __syncthreads();
+    for (int i = tid; i < (1 << bits); i += NT) hist[i] = 0u;
+    __syncthreads();
+    const float vmin = prefilter_value(static_cast<uint32_t>((prefix << above_shift) >> 32));
+    auto count_one = [&](float x, int pos) {
+      const uint64_t comp = make_comp(fast_key(x), pos);
+      if ((comp >> above_shift) == prefix) atomicAdd(&hist[static_cast<uint32_t>(comp >> shift) & mask], 1u);
+    };
+#pragma unroll 1
+    for (int u0 = c.fb; u0 < c.fe; u0 += RowGroup<T, NT>::kStep) {
+      RowGroup<T, NT> g;
+      g.load(c, u0);
+      const int first = RowGroup<T, NT>::position(c, u0);
+      g.template each<false>(c, u0, [&](float x, int e) {
+        if (!(x < vmin)) count_one(x, first + RowGroup<T, NT>::distance(e));
+      });
+    }
+    float x = 0.f;
+    const int pos = partial_element(c, x);
+    if (pos >= 0) count_one(x, pos);
+    __syncthreads();
+    // the crossing: at most 2048 bins, a few consecutive ones per thread
+    const int per = (1 << bits) > NT ? (1 << bits) / NT : 1;
+    const int first = tid * per;
+    int local = 0;
+    if (first < (1 << bits))
+      for (int e = 0; e < per; ++e) local += static_cast<int>(hist[first + e]);
+    int total;
+    int running = suffix_exclusive<NT>(local, sh.warp_tot[1], total);
+    if (running < r && r <= running + local) {
+      for (int e = per - 1; e >= 0; --e) {
+        const int n = static_cast<int>(hist[first + e]);
+        if (running < r && r <= running + n) {
+          sh.t = first + e;
+          sh.above = running;
+          sh.total = (k - r) + running + n;
+        }
+        running += n;
+      }
+    }
+    __syncthreads();
+    if (total < r) {
+      if (status != nullptr && tid == 0) atomicOr(status, 4);
+      return ~0ull;
+    }
+    prefix = (prefix << bits) | static_cast<uint64_t>(sh.t);
+    r -= sh.above;
+    if (sh.total <= cap || level == kNumLevels - 1) return prefix << shift;
+  }
+}
+
+// Sweep 2: every score not below vmin (EXACT: whose composite is not below floor_comp) goes to the list.
+// `first` is the row's first group, still in registers.  A warp takes 512 scores at a time: the
+// lanes' hit counts are summed with five ballots and one shared atomic reserves the warp's slots.
+template <typename T, int NT, bool EXACT>
+__device__ __forceinline__ void collect_row(const Chunk<T>& c, const RowGroup<T, NT>* first, float vmin, uint64_t floor_comp,
+                                            uint64_t* list, int cap, RowsShared& sh) {
+  using Group = RowGroup<T, NT>;
+  const int lane = threadIdx.x & 31;
+  const uint32_t list_at = smem_addr(list);
+  auto take = [&](const Group& g, int u0, auto full) {
+    constexpr bool FULL = decltype(full)::value;
+    const int pos0 = Group::position(c, u0);
+    uint32_t hits = 0u;
+    g.template each<FULL>(c, u0, [&](float x, int e) {
+      bool hit = !(x < vmin);
+      if (EXACT) hit = hit && make_comp(fast_key(x), pos0 + Group::distance(e)) >= floor_comp;
+      if (hit) hits |= 1u << e;
+    });
+    if (!__any_sync(0xffffffffu, hits != 0u)) return;
+    const uint32_t n = static_cast<uint32_t>(__popc(hits));
+    const uint32_t lt = (1u << lane) - 1u;
+    int before = 0, total = 0;
+#pragma unroll
+    for (int b = 0; b < 5; ++b) {
+      const uint32_t plane = __ballot_sync(0xffffffffu, n & (1u << b));
+      before += __popc(plane & lt) << b;
+      total += __popc(plane) << b;
+    }
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&sh.count, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base + total > cap) return;
+    uint32_t at = list_at + 8u * static_cast<uint32_t>(base + before);
+    g.template each<FULL>(c, u0, [&](float x, int e) {
+      asm volatile(
+          "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p st.shared.v2.b32 [%0], {%1, %2};\n\t@p add.u32 %0, %0, 8;\n\t}"
+          : "+r"(at) : "r"(pos0 + Group::distance(e)), "r"(__float_as_uint(x)), "r"(hits & (1u << e)) : "memory");
+    });
+  };
+#pragma unroll 1
+  for (int u0 = c.fb; u0 < c.fe; u0 += Group::kStep) {
+    Group g;
+    if (first != nullptr && u0 == c.fb) g = *first; else g.load(c, u0);
+    if (u0 + Group::kStep <= c.fe) take(g, u0, std::true_type{}); else take(g, u0, std::false_type{});
+  }
+  float x = 0.f;
+  const int pos = partial_element(c, x);
+  if (pos >= 0 && !(x < vmin) && (!EXACT || make_comp(fast_key(x), pos) >= floor_comp)) {
+    const int at = atomicAdd(&sh.count, 1);
+    if (at < cap) list[at] = list_entry(x, pos);
+  }
+}
+
+template <typename T, int NT>
+__device__ __noinline__ void collect_row_exact(const Chunk<T>& c, uint64_t floor_comp, uint64_t* list, int cap, RowsShared& sh) {
+  collect_row<T, NT, true>(c, nullptr, prefilter_value(static_cast<uint32_t>(floor_comp >> 32)), floor_comp, list, cap, sh);
+}
+
+// How a survivor becomes an expected rank: its digit picks a packed bin (elements above, elements in it), and
+// its depth below the bin's upper end, as a 32-bit fraction, interpolates between the bin's ends.
+// The depth holds the key's bits below the digit, without the low ones in which no two survivors'
+// scores differ (rounded scores), and behind them the index, so that ties spread by index.  It orders the
+// survivors of a bin; two of them share a depth only if their keys are equal and their indices differ
+// in nothing but the low bits for which there was no room.
+struct DepthMap {
+  uint32_t key_mask;         // of the left-aligned key bits below the digit: those that tell survivors apart
+  int idx_left, idx_right;   // shift of the index behind them
+};
+__device__ __forceinline__ DepthMap depth_map(int shift, uint32_t value_bits, int len) {
+  int same = value_bits == 0u ? 31 : __ffs(static_cast<int>(value_bits)) - 1;   // low score bits that are zero everywhere
+  if (same > shift) same = shift;
+  const int free_bits = 32 - shift + same;                // below the key bits that count
+  const int idx_bits = 32 - __clz(len - 1);
+  DepthMap m;
+  m.key_mask = free_bits >= 32 ? 0u : ~((1u << free_bits) - 1u);
+  m.idx_left = free_bits > idx_bits ? free_bits - idx_bits : 0;
+  m.idx_right = idx_bits > free_bits ? idx_bits - free_bits : 0;
+  return m;
+}
+// below: the key's bits below the digit, left-aligned.  (A larger index lies deeper.)
+__device__ __forceinline__ uint32_t depth_of(const DepthMap& m, uint32_t below, int32_t idx) {
+  return (~below & m.key_mask) | ((static_cast<uint32_t>(idx) << m.idx_left) >> m.idx_right);
+}
+__device__ __forceinline__ uint32_t expected_rank2(uint32_t packed, uint32_t depth) {
+  return (packed >> kPackShift) + __umulhi(depth, packed & ((1u << kPackShift) - 1u));
+}
+
+// PER: survivors a thread holds in the finish (the list takes PER * NT); CTAS: CTAs per SM it is compiled for.
+template <typename T, int NT, int PER, int CTAS, bool HINTS>
+__global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ RowsShared sh;
+  using Group = RowGroup<T, NT>;
+  constexpr int kPU = Elem<T>::kPerUnit;
+  constexpr int kCap = PER * NT;
+  uint32_t* hist = reinterpret_cast<uint32_t*>(smem);
+  uint32_t* bucketed = hist;                                                 // depths, bucket by bucket
+  uint64_t* list = reinterpret_cast<uint64_t*>(smem + kRowsBins * 4);
+  uint32_t* bins = reinterpret_cast<uint32_t*>(list);                        // 2 * kCap finish bins
+  int32_t* ranked = reinterpret_cast<int32_t*>(list);                        // kCap positions
+  const int tid = threadIdx.x;
+  auto clear_words = [&](uint32_t* a, int n) {
+#pragma unroll 4
+    for (int i = 4 * tid; i < n; i += 4 * NT) *reinterpret_cast<uint4*>(a + i) = make_uint4(0u, 0u, 0u, 0u);
+  };
+  // set-up that reads nothing of the kernels in front, behind which it may run
+  clear_words(hist, kRowsBins);
+  if (tid == 0) {
+    sh.t = 0;
+    sh.above = 0;
+    sh.total = 0;
+    sh.max_bin = 0;
+    sh.count = 0;
+    sh.value_bits = 0u;
+    sh.kmin = 0xffffffffu;
+    sh.kmax = 0u;
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  FF_TRACE(p, 0);
+  const int row = static_cast<int>(blockIdx.x);
+  const int k = p.k;
+  const int rs = p.row_starts != nullptr ? p.row_starts[row] : 0;
+  int64_t l = p.lengths[row];
+  if (l > p.L_width - rs) l = p.L_width - rs;
+  const int len = l < 0 ? 0 : static_cast<int>(l);
+
+  // Writes the row's k results: index_of(j) is the window position of rank j, or -1.
+  auto write_all = [&](auto&& index_of) {
+    int table_row = row;
+    if (p.epilogue == 1 && p.cu_seqlens_q != nullptr) {
+      // prefill: request r with cu_seqlens_q[r] <= row < cu_seqlens_q[r+1]
+      int lo = 0, hi = p.n_table_rows;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (p.cu_seqlens_q[mid] <= row) lo = mid; else hi = mid;
+      }
+      table_row = lo;
+    }
+    const int32_t* table = p.epilogue == 1 ? p.table + static_cast<int64_t>(table_row) * p.table_stride : nullptr;
+    const int32_t offset = p.epilogue == 2 ? p.offsets[row] : 0;
+    auto result = [&](int j) -> int32_t {
+      const int32_t o = index_of(j);
+      return o < 0 ? -1 : table != nullptr ? __ldg(table + o) : o + offset;
+    };
+    const int64_t at = static_cast<int64_t>(row) * k;
+    if (p.out_idx64 != nullptr) {
+      int64_t* out = p.out_idx64 + at;
+#pragma unroll 4
+      for (int j = tid; j < k; j += NT) out[j] = result(j);
+    } else if (((k & 3) | (static_cast<int>(reinterpret_cast<uintptr_t>(p.out_idx)) & 15)) == 0) {
+      int4* out = reinterpret_cast<int4*>(p.out_idx + at);
+#pragma unroll 2
+      for (int j = tid; j < (k >> 2); j += NT) out[j] = make_int4(result(4 * j), result(4 * j + 1), result(4 * j + 2), result(4 * j + 3));
+    } else {
+      int32_t* out = p.out_idx + at;
+#pragma unroll 4
+      for (int j = tid; j < k; j += NT) out[j] = result(j);
+    }
+  };
+
+  uint32_t* header = nullptr;   // survivor list handed over by the producer of the scores
+  if (HINTS && p.handover != nullptr)
+    header = reinterpret_cast<uint32_t*>(p.handover + static_cast<int64_t>(row) * kHandoverRowBytes);
+
+  if (len <= k) {   // nothing to select
+    if (HINTS && tid == 0) {
+      if (header != nullptr) header[0] = header[1] = 0u;
+      if (p.hint_out != nullptr) p.hint_out[row] = __uint_as_float(0x7fffffffu);
+    }
+    write_all([&](int j) { return j < len ? j : -1; });
+    return;
+  }
+
+  const T* rowp = reinterpret_cast<const T*>(p.scores) + static_cast<int64_t>(row) * p.row_stride + rs;
+  // the row in 16-byte units on absolute addresses, partial ones at its ends
+  Chunk<T> chunk;
+  {
+    chunk.mis = static_cast<int>((reinterpret_cast<uintptr_t>(rowp) >> Elem<T>::kLog2Bytes) & (kPU - 1));
+    chunk.abase = rowp - chunk.mis;
+    chunk.len = len;
+    chunk.fb = chunk.mis != 0 ? 1 : 0;
+    chunk.tail_unit = static_cast<int>((static_cast<int64_t>(len) + chunk.mis) / kPU);
+    chunk.fe = max(chunk.tail_unit, chunk.fb);
+    chunk.head = chunk.mis != 0;
+    chunk.tail = ((len + chunk.mis) & (kPU - 1)) != 0 && chunk.tail_unit >= chunk.fb;
+  }
+  __syncthreads();   // set up
+
+  bool listed = false;          // the list holds survivors found with a guess
+  if constexpr (HINTS) {
+    const float hint = p.hint_in != nullptr ? p.hint_in[row] : __uint_as_float(0x7fffffffu);
+    const bool use = hint == hint;
+    if (header != nullptr) {
+      const int n = static_cast<int>(__ldcg(header));
+      if (use && n >= k && n <= kCap) {
+        const unsigned long long* given = reinterpret_cast<const unsigned long long*>(header + 16);
+#pragma unroll 4
+        for (int i = tid; i < n; i += NT) {
+          const uint64_t c = __ldcg(given + i);
+          list[i] = list_entry(__uint_as_float(bits_of_key(comp_key(c))), comp_index(c));
+        }
+        listed = true;
+      }
+      __syncthreads();
+      if (tid == 0) {
+        if (listed) sh.count = n;
+        else if (use && p.status != nullptr) atomicOr(p.status, 8);
+        header[0] = header[1] = 0u;   // empty for the producer's next launch
+      }
+    } else if (use) {
+      collect_row<T, NT, false>(chunk, nullptr, hint, 0ull, list, kCap, sh);
+      __syncthreads();
+      const int n = sh.count;
+      listed = n >= k && n <= kCap;
+      __syncthreads();
+      if (!listed && tid == 0) {
+        sh.count = 0;
+        if (p.status != nullptr) atomicOr(p.status, 8);
+      }
+    }
+    __syncthreads();
+  }
+
+  bool rebuild = listed;        // the packed bins do not fit the list: they are rebuilt from it
+  int span = 0;                 // expected ranks are below this
+  if (!listed) {
+    // ---- sweep 1 ----
+    auto count_one = [&](float x, int) {
+      const uint32_t d = rows_raw_digit(x);
+      if (FF_IN_RANGE(p, d, kRowsBins, 11)) atomicAdd(&hist[d], 1u);
+    };
+    Group first;
+    first.load(chunk, chunk.fb);
+    Group g = first;
+#pragma unroll 1
+    for (int u0 = chunk.fb;;) {
+      if (u0 + Group::kStep <= chunk.fe) g.template each<true>(chunk, u0, count_one);
+      else g.template each<false>(chunk, u0, count_one);
+      u0 += Group::kStep;
+      if (u0 >= chunk.fe) break;
+      g.load(chunk, u0);
+    }
+    if (chunk.head || chunk.tail) {   // (uniform)
+      float x = 0.f;
+      if (partial_element(chunk, x) >= 0) count_one(x, 0);
+    }
+    __syncthreads();
+    FF_TRACE(p, 1);
+    // ---- threshold ----
+    pack_bins<NT>(hist, true, k, sh, sh.warp_tot[0]);
+    FF_TRACE(p, 2);
+    // ---- sweep 2 ----
+    const int above = sh.above, in_bin = sh.total - above;
+    const uint32_t bin_key = static_cast<uint32_t>(sh.t) << kRowsShift;
+    int keep, linear;
+    const uint32_t cut = bin_key + cut_in_digit(hist, sh.t, in_bin, k - above, kCap - above, keep, linear);
+    bool exact = bin_key > 0xff800000u || sh.max_bin > kPackMax || keep < k - above ||
+                 (sh.total > kCap && 8 * sh.max_bin > 7 * sh.total);
+    if (!exact) {
+      collect_row<T, NT, false>(chunk, &first, prefilter_value(cut), 0ull, list, kCap, sh);
+      __syncthreads();
+      const int n = sh.count;
+      span = min(above + linear, kCap);
+      if (n < k || n > kCap) {   // the interpolation was off
+        __syncthreads();
+        if (tid == 0) sh.count = 0;
+        __syncthreads();
+        exact = n > kCap || sh.total > kCap;
+        if (!exact) {
+          collect_row<T, NT, false>(chunk, &first, prefilter_value(bin_key), 0ull, list, kCap, sh);
+          span = sh.total;
+          __syncthreads();
+        }
+      }
+      rebuild = 8 * sh.max_bin > 7 * sh.total;   // one digit holds nearly all: it says little about their ranks
+    }
+    if (exact) {
+      rebuild = true;
+      const uint64_t floor_comp = sh.total <= kCap ? static_cast<uint64_t>(sh.t) << rows_level_shift(0)
+                                                   : deeper_digits<T, NT>(chunk, hist, k, kCap, sh, p.status);
+      collect_row_exact<T, NT>(chunk, floor_comp, list, kCap, sh);
+      __syncthreads();
+    }
+  }
+  FF_TRACE(p, 3);
+  const int n = min(sh.count, kCap);
+  if (rebuild) span = n;
+
+  // ---- finish ----
+  // A thread keeps its survivors in registers; where[] is in turn a survivor's packed bin, finish bin and
+  // arrival in it, bucket (first slot << 16 | size), and rank.  Loads and stores are kept in loops of their
+  // own, so that a phase's loads are in flight together.  The second half of the places is skipped
+  // by the whole CTA when n leaves it empty.
+  constexpr int kHalf = (PER + 1) / 2;
+  uint32_t depth[PER], where[PER];
+  int32_t pos[PER];                      // window position, or -1: no survivor
+  auto mine = [&](auto&& f) {
+#pragma unroll
+    for (int j = 0; j < kHalf; ++j) f(j);
+    if (n > kHalf * NT) {
+#pragma unroll
+      for (int j = kHalf; j < PER; ++j) f(j);
+    }
+  };
+#pragma unroll
+  for (int j = 0; j < PER; ++j) pos[j] = -1;
+  {
+    uint32_t value_bits = 0u;
+    mine([&](int j) {
+      if (tid + j * NT < n) {
+        const uint64_t e = list[tid + j * NT];
+        value_bits |= static_cast<uint32_t>(e >> 32);
+        pos[j] = static_cast<int32_t>(e);
+        depth[j] = __float_as_uint(__fadd_rn(__uint_as_float(static_cast<uint32_t>(e >> 32)), 0.0f));
+        if (!rebuild) where[j] = hist[depth[j] >> kRowsShift];
+      }
+    });
+    value_bits = __reduce_or_sync(0xffffffffu, value_bits);
+    if ((tid & 31) == 0) atomicOr(&sh.value_bits, value_bits);
+  }
+  auto key_bits = [](uint32_t u) { return u ^ (static_cast<uint32_t>(static_cast<int32_t>(u) >> 31) | 0x80000000u); };
+  uint32_t base = 0u;
+  int shift = kRowsShift;
+  if (rebuild) {
+    // digits of the survivors' own key range instead of the row's first digit
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
+    if (!listed) clear_words(hist, kRowsBins);
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      if (pos[j] >= 0) {
+        kmin = min(kmin, key_bits(depth[j]));
+        kmax = max(kmax, key_bits(depth[j]));
+      }
+    }
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if ((tid & 31) == 0) {
+      atomicMin(&sh.kmin, kmin);
+      atomicMax(&sh.kmax, kmax);
+    }
+    __syncthreads();
+    base = sh.kmin;
+    const uint32_t range = sh.kmax - sh.kmin;
+    shift = range >= static_cast<uint32_t>(kRowsBins) ? 32 - __clz(static_cast<int>(range)) - kRowsBits : 0;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const uint32_t d = (key_bits(depth[j]) - base) >> shift;
+      if (pos[j] >= 0 && FF_IN_RANGE(p, d, kRowsBins, 15)) atomicAdd(&hist[d], 1u);
+    }
+    __syncthreads();
+    pack_bins<NT>(hist, false, n, sh, sh.warp_tot[2]);
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (pos[j] >= 0) where[j] = hist[(key_bits(depth[j]) - base) >> shift];
+  } else {
+    __syncthreads();   // the list has been read
+  }
+  clear_words(bins, 2 * span);
+  const DepthMap map = depth_map(shift, sh.value_bits, len);
+  const uint32_t last_bin = 2u * static_cast<uint32_t>(span) - 1u;
+  if (rebuild) {
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const uint32_t below = shift == 0 ? 0u : (key_bits(depth[j]) - base) << (32 - shift);
+      depth[j] = depth_of(map, below, pos[j]);
+      where[j] = min(expected_rank2(where[j], depth[j]), last_bin);
+    }
+  } else {
+    mine([&](int j) {
+      depth[j] = depth_of(map, (depth[j] ^ static_cast<uint32_t>(static_cast<int32_t>(depth[j]) >> 31)) << kRowsBits, pos[j]);
+      where[j] = min(expected_rank2(where[j], depth[j]), last_bin);
+    });
+  }
+  __syncthreads();   // the bins are clear
+  mine([&](int j) {
+    if (pos[j] >= 0 && FF_IN_RANGE(p, where[j], 2 * kCap, 12)) where[j] |= atomicAdd(&bins[where[j]], 1u) << 16;
+  });
+  __syncthreads();
+  FF_TRACE(p, 22);
+  {
+    // counts -> (first slot << 16 | size)
+    constexpr int per = 2 * PER;
+    constexpr int kQuads = (per + 3) / 4;
+    uint4* quads = reinterpret_cast<uint4*>(bins);
+    const int q0 = tid * kQuads;
+    const int q_end = (2 * span + 3) >> 2;
+    uint4 v[kQuads];
+    uint32_t local = 0u;
+#pragma unroll
+    for (int q = 0; q < kQuads; ++q) {
+      v[q] = q0 + q < q_end ? quads[q0 + q] : make_uint4(0u, 0u, 0u, 0u);
+      local += (v[q].x + v[q].y) + (v[q].z + v[q].w);
+    }
+    int total;
+    const int after = suffix_exclusive<NT>(static_cast<int>(local), sh.warp_tot[1], total);
+    uint32_t start = static_cast<uint32_t>(total - after) - local;
+#pragma unroll
+    for (int q = 0; q < kQuads; ++q) {
+      const uint32_t s1 = start + v[q].x, s2 = s1 + v[q].y, s3 = s2 + v[q].z;
+      if (q0 + q < q_end)
+        quads[q0 + q] = make_uint4((start << 16) | v[q].x, (s1 << 16) | v[q].y, (s2 << 16) | v[q].z, (s3 << 16) | v[q].w);
+      start = s3 + v[q].w;
+    }
+  }
+  __syncthreads();
+  FF_TRACE(p, 23);
+  {
+    uint32_t at[PER];
+    mine([&](int j) {
+      if (pos[j] >= 0) {
+        const uint32_t w = bins[where[j] & 0xffffu];
+        at[j] = (w >> 16) + (where[j] >> 16);
+        where[j] = w;
+      }
+    });
+    mine([&](int j) {
+      if (pos[j] >= 0 && FF_IN_RANGE(p, at[j], kCap, 13)) bucketed[at[j]] = depth[j];
+    });
+  }
+  __syncthreads();
+  FF_TRACE(p, 24);
+  mine([&](int j) {
+    if (pos[j] >= 0) {
+      const uint32_t size = where[j] & 0xffffu;
+      uint32_t rank = where[j] >> 16;
+      const uint32_t* bucket = bucketed + rank;
+      if (FF_IN_RANGE(p, static_cast<int>(rank + size) - 1, kCap, 17)) {
+        rank += (bucket[0] < depth[j] ? 1u : 0u) + (bucket[size > 1u ? 1 : 0] < depth[j] ? 1u : 0u);   // most buckets have no more
+#pragma unroll 1
+        for (uint32_t q = 2; q < size; ++q) rank += bucket[q] < depth[j] ? 1u : 0u;
+      }
+      where[j] = rank;
+    }
+  });
+  mine([&](int j) {
+    if (pos[j] >= 0) ranked[where[j]] = pos[j];
+  });
+  __syncthreads();
+  // Survivors of one depth have taken the same rank; all but one of them find another's position there.
+  uint32_t beaten = 0u;
+  mine([&](int j) {
+    if (pos[j] >= 0 && ranked[where[j]] != pos[j]) beaten |= 1u << j;
+  });
+  if (__syncthreads_or(beaten != 0u ? 1 : 0)) {
+    // Each moves down by the positions below its own that share its rank.
+    int32_t* tied_pos = reinterpret_cast<int32_t*>(hist);
+    uint32_t* tied_rank = reinterpret_cast<uint32_t*>(ranked + kCap);
+    if (tid == 0) sh.count = 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      if (beaten & (1u << j)) {
+        const int at = atomicAdd(&sh.count, 1);
+        tied_pos[at] = pos[j];
+        tied_rank[at] = where[j];
+      }
+    }
+    __syncthreads();
+    const int m = sh.count;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      if (pos[j] >= 0) {
+        uint32_t below = ranked[where[j]] < pos[j] ? 1u : 0u;
+#pragma unroll 1
+        for (int q = 0; q < m; ++q) below += tied_rank[q] == where[j] && tied_pos[q] < pos[j] ? 1u : 0u;
+        where[j] += below;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (pos[j] >= 0) ranked[where[j]] = pos[j];
+    __syncthreads();
+  }
+  FF_TRACE(p, 31);
+  write_all([&](int j) { return ranked[j]; });
+  FF_TRACE(p, 25);
+  if constexpr (HINTS) {
+    if (p.hint_out != nullptr) {
+      // Next call's guess: the score of rank hint_target_rank(k), or, with fewer survivors, a linear
+      // extrapolation below the smallest one from the ranks n / 2 and n.
+      const int want = hint_target_rank(k);
+      const int rank_a = min(n, want) - 1, rank_m = n >> 1;
+      if (tid == 0) {
+        const float va = Elem<T>::to_float(rowp[ranked[rank_a]]), vm = Elem<T>::to_float(rowp[ranked[rank_m]]);
+        float guess = va;
+        if (n < want && rank_a > rank_m) {
+          const float lower = va - (vm - va) * (static_cast<float>(want - 1 - rank_a) / static_cast<float>(rank_a - rank_m));
+          if (lower == lower && fabsf(lower) <= 3.0e38f) guess = lower;
+        }
+        p.hint_out[row] = guess;
+      }
+    }
+  }
+}
+
+}  // namespace ff

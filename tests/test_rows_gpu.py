@@ -1,0 +1,76 @@
+"""The one-CTA-per-row select (short rows, batches of many rows) at the sizes where it changes its ways: rows that
+end inside, at and just behind a group of scores, lists that fill up, digits that say nothing, and
+neighbours that share key and depth; exact against the CPU oracle."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+KINDS = 10
+
+
+def _row(kind: int, L: int, g: torch.Generator) -> torch.Tensor:
+    x = torch.randn((L,), generator=g)
+    if kind == 1:
+        return x.to(torch.bfloat16).float()                    # heavy ties
+    if kind == 2:
+        return torch.full((L,), -2.5)                          # only the index decides
+    if kind == 3:
+        return x + 1000.0                                      # every score in one digit
+    if kind == 4:
+        return x[: (L + 7) // 8].repeat_interleave(8)[:L]      # equal keys with neighbouring indices, full mantissas
+    if kind == 5:
+        return -x.abs() - 0.5                                  # negative threshold
+    if kind == 6:
+        x[::7], x[1::7], x[2::9] = float("nan"), float("inf"), float("-inf")
+        return x
+    if kind == 7:
+        x[3] = 1e30                                            # one far outlier over a narrow rest
+        return x * 1e-3 + 1.0
+    if kind == 8:
+        return torch.round(x * 2)                              # about ten distinct values
+    if kind == 9:
+        return torch.sort(x).values                            # every winner at the end
+    return x
+
+
+def _check(oracle, s, lengths, k, rs=None, **kw):
+    from flash_float_jit_kernels_b200 import fast_topk_v3
+    dev = torch.device("cuda:0")
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    out = fast_topk_v3(s.to(dev), lengths.to(dev), k, None if rs is None else rs.to(dev), status=status, **kw)
+    torch.cuda.synchronize()
+    assert int(status.item()) & ~8 == 0
+    exp = oracle.topk_c(s.float().numpy(), lengths.numpy(), k, None if rs is None else rs.numpy())
+    got = out.cpu().numpy()
+    bad = np.argwhere((got != exp).any(axis=1)).ravel()
+    assert bad.size == 0, f"rows {bad[:8].tolist()} of kinds {[int(b) % KINDS for b in bad[:8]]}"
+
+
+# 16 scores per thread and group: 4,096 with 256 threads (more rows than SMs), 16,384 with 1,024 (fewer rows)
+@pytest.mark.parametrize("B,L,k", [(20, 2049, 2048), (20, 16383, 2048), (20, 16385, 512), (20, 33000, 2048), (20, 70, 1),
+                                   (160, 4095, 2048), (160, 4096, 1024), (160, 4097, 512), (160, 12289, 2048), (160, 70, 69),
+                                   (310, 9000, 2048), (300, 50001, 1024)])
+def test_rows_of_every_kind(oracle, B, L, k):
+    g = torch.Generator().manual_seed(L + k)
+    s = torch.stack([_row(i % KINDS, L, g) for i in range(B)])
+    lengths = torch.full((B,), L, dtype=torch.int32)
+    lengths[KINDS:2 * KINDS] = torch.randint(1, L + 1, (KINDS,), generator=g, dtype=torch.int32)
+    _check(oracle, s, lengths, k)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B", [30, 170])
+def test_windows_types_guesses_and_wide_indices(oracle, B, dtype):
+    from flash_float_jit_kernels_b200 import new_threshold_hint
+    g = torch.Generator().manual_seed(B)
+    L, k = 6011, 700
+    s = torch.stack([_row(i % KINDS, L, g) for i in range(B)]).to(dtype)
+    rs = torch.arange(B, dtype=torch.int32) % 19
+    lengths = torch.full((B,), L - 20, dtype=torch.int32) - (torch.arange(B, dtype=torch.int32) % 9)
+    _check(oracle, s, lengths, k, rs)
+    _check(oracle, s, lengths, k, rs, index_dtype=torch.int64)
+    hint = new_threshold_hint(B, "cuda")
+    for _ in range(3):
+        _check(oracle, s, lengths, k, rs, threshold_hint=hint)

@@ -14,7 +14,7 @@ from . import _lib
 from .build import host_module_path
 
 TOPK_FUNCTIONS = ("ff_topk_launch_typed", "ff_topk_launch_handover", "ff_topk_transform_launch", "ff_topk_workspace_bytes")
-LOGITS_FUNCTIONS = ("ff_indexer_logits_launch_handover",)
+LOGITS_FUNCTIONS = ("ff_indexer_logits_launch_fresh",)
 
 
 def _bind(module, lib, names) -> None:

@@ -31,7 +31,7 @@ decltype(&ff_topk_launch_typed) p_typed = nullptr;
 decltype(&ff_topk_launch_handover) p_handover = nullptr;
 decltype(&ff_topk_transform_launch) p_transform = nullptr;
 decltype(&ff_topk_workspace_bytes) p_workspace_bytes = nullptr;
-decltype(&ff_indexer_logits_launch_handover) p_logits = nullptr;
+decltype(&ff_indexer_logits_launch_fresh) p_logits = nullptr;
 PyObject* g_on_error = nullptr;   // Python callable (return code, operator name): raises
 
 using at::Tensor;
@@ -306,8 +306,12 @@ PyObject* logits(PyObject* py_q, PyObject* py_k, PyObject* py_w, PyObject* py_le
   }
   Tensor fresh;
   const Tensor* out;
+  bool fill = false;
   if (is_none(py_out)) {
-    fresh = at::full({B, L}, -std::numeric_limits<float>::infinity(), at::TensorOptions().dtype(at::kFloat).device(dev));
+    // the kernel writes the -inf behind the rows' ends itself where it can (a fill kernel of its own: 5 us for 64 x 128 Ki)
+    const auto options = at::TensorOptions().dtype(at::kFloat).device(dev);
+    fill = ctas_per_row == 0 && B <= FF_INDEXER_MAX_FILL_ROWS && keys->stride(0) < (int64_t{1} << 40);
+    fresh = fill ? at::empty({B, L}, options) : at::full({B, L}, -std::numeric_limits<float>::infinity(), options);
     out = &fresh;
   } else {
     out = cuda_tensor(py_out);
@@ -325,7 +329,7 @@ PyObject* logits(PyObject* py_q, PyObject* py_k, PyObject* py_w, PyObject* py_le
   float* out_ptr = static_cast<float*>(out->data_ptr());
   const int rc = without_gil([&] {
     return p_logits(q_ptr, k_ptr, k_stride, w_ptr, len_ptr, out_ptr, out_stride, static_cast<int32_t>(B),
-                    static_cast<int32_t>(L), static_cast<int32_t>(ctas_per_row), hint, handover, status, stream);
+                    static_cast<int32_t>(L), static_cast<int32_t>(ctas_per_row), fill ? 1 : 0, hint, handover, status, stream);
   });
   if (rc != 0) return report(rc, "indexer_logits_fp8");
   if (out == &fresh) return THPVariable_Wrap(std::move(fresh));
@@ -366,7 +370,7 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   else if (strcmp(name, "ff_topk_launch_handover") == 0) p_handover = reinterpret_cast<decltype(p_handover)>(p);
   else if (strcmp(name, "ff_topk_transform_launch") == 0) p_transform = reinterpret_cast<decltype(p_transform)>(p);
   else if (strcmp(name, "ff_topk_workspace_bytes") == 0) p_workspace_bytes = reinterpret_cast<decltype(p_workspace_bytes)>(p);
-  else if (strcmp(name, "ff_indexer_logits_launch_handover") == 0) p_logits = reinterpret_cast<decltype(p_logits)>(p);
+  else if (strcmp(name, "ff_indexer_logits_launch_fresh") == 0) p_logits = reinterpret_cast<decltype(p_logits)>(p);
   else {
     PyErr_SetString(PyExc_ValueError, "bind: unknown name");
     return nullptr;

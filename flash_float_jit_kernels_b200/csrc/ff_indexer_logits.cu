@@ -5,11 +5,14 @@
 // has no such kernel; the shape is the one its README gives for the indexer
 // (README.md:28) and the benchmark's ragged decode batch is generated this way.
 //
-// One CTA works on one row b and a strided share of its 128-key tiles:
+// Two kernels.  indexer_logits_run_kernel (the default): a persistent grid whose CTAs each take an equal run of
+// the batch's 128-key tiles, K arriving by tensor copies.  indexer_logits_kernel (a fixed number of CTAs per row on
+// request, and batches of more than 1,024 rows): one CTA works on one row b and a strided share of its tiles:
 //   * four producer warps copy a tile of K (128 keys x 128 bytes) into shared
 //     memory with 16-byte cp.async, writing the 128-byte-swizzled K-major layout
 //     the tensor core reads (16-byte chunk c of key r goes to chunk c ^ (r & 7));
-//     rows past the row's length are zero-filled, nothing outside K is read;
+//     rows past the row's length are zero-filled, nothing outside K is read.
+// Both:
 //   * one thread issues four tcgen05.mma (kind::f8f6f4, M = 128 keys, N = 64
 //     heads, K = 32 per instruction) per tile into one of two accumulator
 //     buffers in tensor memory (128 lanes x 64 fp32 columns each);
@@ -18,6 +21,7 @@
 //     fused multiply-adds (four interleaved partial sums), and store one score per key.
 // Stages are handed over with mbarriers; every wait is bounded and sets a status
 // bit instead of spinning for ever.
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -106,13 +110,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
   *gave_up = 1;
   return false;
-}
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t done;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-  return done != 0;
 }
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
@@ -389,40 +386,42 @@ __global__ void __launch_bounds__(kThreads, 2) indexer_logits_kernel(const Param
 }
 
 
-// ---- persistent variant ---------------------------------------------------------
-// The grid is two CTAs per SM whatever the batch; the work is cut into units of
-// kUnitTiles consecutive 128-key tiles of one row, numbered row by row (a prefix sum
-// over the rows' unit counts, computed by every CTA from the device-side lengths), and
-// CTA c takes units c, c + grid, c + 2 grid, ...  Barriers, tensor memory and the
-// pipeline state are set up once per CTA and run on across units; q is double buffered
-// (the next unit's q lands while the current unit's tiles are multiplied).
-constexpr int kUnitTiles = 8;
-constexpr int kPStages = 5;
-constexpr int kMaxRowsPersistent = 1024;
-constexpr int kPSmemQ = 0;                       // two q buffers
-constexpr int kPSmemK = 2 * kQBytes;
-constexpr int kPSmemBytes = 2 * kQBytes + kPStages * kTileBytes + 1024;
+// ---- the default kernel: a persistent grid, every CTA an equal run of tiles ----------------
+// The tiles of all rows are numbered row by row (a prefix sum over the rows' tile counts, computed by every CTA from
+// the device-side lengths) and CTA c of the G takes tiles [c T / G, (c + 1) T / G): one wave, the same number of
+// tiles for everyone whatever the lengths, and at most a row change or two per CTA on the way.
+//   * one thread asks for the K tiles with cp.async.bulk.tensor (128-byte swizzle done by the copy; keys
+//     past the tensor's end arrive as zero) and, at a row change, for the new row's q into the other q buffer;
+//   * one thread issues the tensor-core instructions;
+//   * four epilogue warps as above; in front of their first tile they also write the -inf of a fresh result.
+// Bound by the K bytes: 64 full rows of 131,072 keys 179.7 us (6.16 TB/s, 94 % of the measured copy peak), lengths
+// U[8192, 131072] 98.6 us (5.93 TB/s).  Shares of up to 32 tiles dealt out by the hardware (indexer_logits_kernel: each
+// share sets up barriers and tensor memory, loads q and fills its pipeline again, and the last wave is ragged)
+// took 180.8 and 114.9 us, and 14.5 instead of 10.7 us for 16 ragged rows of 40,000.
+constexpr int kRunStages = 5;
+constexpr int kRunMaxRows = FF_INDEXER_MAX_FILL_ROWS;
+constexpr int kRunThreads = (kEpilogueWarps + 2) * 32;
+constexpr int kRunProducerWarp = kEpilogueWarps + 1;
+constexpr int kRunSmemBytes = 2 * kQBytes + kRunStages * kTileBytes + 1024;
 
-struct PShared {
-  unsigned long long full[kPStages];
-  unsigned long long empty[kPStages];
+struct RunShared {
+  unsigned long long full[kRunStages];
+  unsigned long long empty[kRunStages];
   unsigned long long qfull[2];
   unsigned long long qempty[2];
   unsigned long long tfull[2];
   unsigned long long tempty[2];
   uint32_t tmem_base;
   int timed_out;
-  float w[kHeads];                       // head weights of the unit the epilogue is working on
-  int prefix[kMaxRowsPersistent + 1];    // units before row b
+  int prefix[kRunMaxRows + 1];           // tiles in front of row b
+  float w[2][kHeads];
+  unsigned long long handover[kEpilogueWarps][2][kHandoverWarpBuf];
 };
 
-// One unit of work and the position inside it; every role walks the same sequence.
-struct UnitCursor {
-  int u;        // unit number (global), advanced by the grid size
-  int n;        // how many units this CTA has started before this one
-  int row, len, tile0, ntile;
-  int i;        // tile inside the unit
-  int t;        // tiles this CTA has passed before this one (drives stages and phases)
+struct RunParams {
+  Params p;
+  int32_t B;
+  int32_t fill;            // 1: positions behind a row's last processed tile become -inf as well
 };
 
 __device__ __forceinline__ int clamp_len(const Params& p, int row) {
@@ -430,212 +429,242 @@ __device__ __forceinline__ int clamp_len(const Params& p, int row) {
   if (len > p.L_width) len = p.L_width;
   return len < 0 ? 0 : len;
 }
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
 
-__device__ __forceinline__ void cursor_load_unit(UnitCursor& c, const Params& p, const int* prefix, int B) {
-  int lo = 0, hi = B;   // last row with prefix[row] <= u
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (prefix[mid] <= c.u) lo = mid; else hi = mid;
+// A CTA's run of tiles, walked alike by every role.
+struct RunCursor {
+  int row, tile, n_tiles;  // tile of the row, tiles of the row
+  int rows_done;           // rows of this CTA before this one (drives the q buffers)
+  __device__ __forceinline__ void start(const int* prefix, int B, int first) {
+    int lo = 0, hi = B;    // last row with prefix[row] <= first (empty rows share a prefix with the next)
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (prefix[mid] <= first) lo = mid; else hi = mid;
+    }
+    row = lo;
+    tile = first - prefix[lo];
+    n_tiles = prefix[lo + 1] - prefix[lo];
+    rows_done = 0;
   }
-  c.row = lo;
-  c.len = clamp_len(p, lo);
-  const int tiles_row = (c.len + kTileKeys - 1) / kTileKeys;
-  c.tile0 = (c.u - prefix[lo]) * kUnitTiles;
-  c.ntile = min(kUnitTiles, tiles_row - c.tile0);
-  c.i = 0;
-}
-// Moves to the next tile; returns false when the CTA's units are used up.
-__device__ __forceinline__ bool cursor_next(UnitCursor& c, const Params& p, const int* prefix, int B, int total_units,
-                                            int stride) {
-  c.t += 1;
-  c.i += 1;
-  if (c.i < c.ntile) return true;
-  c.u += stride;
-  c.n += 1;
-  if (c.u >= total_units) return false;
-  cursor_load_unit(c, p, prefix, B);
-  return true;
-}
+  // Moves on by one tile; true at a row change.
+  __device__ __forceinline__ bool next(const int* prefix, int B) {
+    if (++tile < n_tiles) return false;
+    do ++row; while (row < B && prefix[row + 1] == prefix[row]);
+    tile = 0;
+    n_tiles = row < B ? prefix[row + 1] - prefix[row] : 0;
+    ++rows_done;
+    return true;
+  }
+};
 
-__global__ void __launch_bounds__(kThreads, 2) indexer_logits_persistent_kernel(const Params p, const int B) {
+__global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(const __grid_constant__ CUtensorMap k_map,
+                                                                          const __grid_constant__ CUtensorMap q_map,
+                                                                          const RunParams a) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ PShared sh;
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t q_s = smem_base + kPSmemQ;
-  const uint32_t k_s = smem_base + kPSmemK;
+  __shared__ RunShared sh;
+  const Params& p = a.p;
+  const int B = a.B;
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;   // swizzle atoms need 1024-byte alignment
+  const uint32_t q_s = smem_base;
+  const uint32_t k_s = smem_base + 2 * kQBytes;
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
 
-  // units per row -> exclusive prefix (one warp: each lane sums a contiguous run of rows)
-  for (int b = tid; b < B; b += kThreads) {
-    const int tiles = (clamp_len(p, b) + kTileKeys - 1) / kTileKeys;
-    sh.prefix[b + 1] = (tiles + kUnitTiles - 1) / kUnitTiles;
-  }
+  // set-up that reads nothing of the kernels in front, behind which it may run
   if (tid == 0) {
-    sh.prefix[0] = 0;
-    for (int s = 0; s < kPStages; ++s) {
-      mbar_init(smem_u32(&sh.full[s]), kProducerThreads);
+    for (int s = 0; s < kRunStages; ++s) {
+      mbar_init(smem_u32(&sh.full[s]), 1);
       mbar_init(smem_u32(&sh.empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
-      mbar_init(smem_u32(&sh.qfull[b]), kProducerThreads);
+      mbar_init(smem_u32(&sh.qfull[b]), 1);
       mbar_init(smem_u32(&sh.qempty[b]), 1);
       mbar_init(smem_u32(&sh.tfull[b]), 1);
       mbar_init(smem_u32(&sh.tempty[b]), kEpilogueWarps * 32);
     }
     sh.timed_out = 0;
+    sh.prefix[0] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncthreads();
-  if (warp == 0) {
-    const int per = (B + 31) / 32;
-    const int b0 = lane * per;
-    int sum = 0;
-    for (int j = 0; j < per; ++j)
-      if (b0 + j < B) sum += sh.prefix[b0 + j + 1];
-    int incl = sum;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += v;
-    }
-    int running = incl - sum;
-    for (int j = 0; j < per; ++j) {
-      if (b0 + j < B) {
-        running += sh.prefix[b0 + j + 1];
-        sh.prefix[b0 + j + 1] = running;
-      }
-    }
-  }
-  __syncthreads();
-  const int total_units = sh.prefix[B];
-  const int stride = static_cast<int>(gridDim.x);
-  if (static_cast<int>(blockIdx.x) >= total_units) return;   // uniform, before the allocation
-
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+  // tiles per row -> exclusive prefix (one warp sums 32 rows at a time)
+  if (warp == kRunProducerWarp) {
+    int running = 0;
+    for (int b0 = 0; b0 < B; b0 += 32) {
+      const int b = b0 + lane;
+      int incl = b < B ? (clamp_len(p, b) + kTileKeys - 1) / kTileKeys : 0;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += v;
+      }
+      if (b < B) sh.prefix[b + 1] = running + incl;
+      running += __shfl_sync(0xffffffffu, incl, 31);
+    }
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh.tmem_base;
+  const int64_t total = sh.prefix[B];
+  const int first = static_cast<int>(total * blockIdx.x / gridDim.x);
+  const int n_mine = static_cast<int>(total * (blockIdx.x + 1) / gridDim.x) - first;
+  RunCursor c;
+  if (n_mine > 0) c.start(sh.prefix, B, first);
 
-  UnitCursor c;
-  c.u = static_cast<int>(blockIdx.x);
-  c.n = 0;
-  c.t = 0;
-  cursor_load_unit(c, p, sh.prefix, B);
-
-  if (warp >= kProducerWarp0) {
-    // ---------------- producers ----------------
-    const int pt = tid - kProducerWarp0 * 32;
-    // Every tile is one copy group.  A tile is announced (its "full" barrier, and with a unit's
-    // first tile the unit's q) once its group has landed: normally when kPStages tiles are
-    // outstanding, the oldest is waited for; at the end, and before a wait that the tensor-core
-    // thread can only satisfy after seeing tiles still unannounced, everything outstanding is.
-    UnitCursor d = c;          // the next tile to announce
-    bool more = true;          // c points at a tile to issue
-    int lag = 0;               // tiles issued and not yet announced
-    auto announce_one = [&]() {
-      if (d.i == 0) mbar_arrive(smem_u32(&sh.qfull[d.n & 1]));
-      mbar_arrive(smem_u32(&sh.full[d.t % kPStages]));
-      lag -= 1;
-      (void)cursor_next(d, p, sh.prefix, B, total_units, stride);
-    };
-    auto announce_all = [&]() {
-      cp_async_wait<0>();
-      fence_async_proxy();
-      while (lag > 0) announce_one();
-    };
-    while (more) {
-      const int stage = c.t % kPStages;
-      if (c.t >= kPStages)
-        (void)mbar_wait(smem_u32(&sh.empty[stage]), static_cast<uint32_t>((c.t / kPStages - 1) & 1), &sh.timed_out);
-      if (c.i == 0) {   // first tile of a unit: its q goes into the same copy group
-        const int qb = c.n & 1;
-        if (c.n >= 2) {
-          // The buffer's previous unit (n - 2) must be multiplied.  After a short unit n - 1 some of
-          // its tiles may still be unannounced: announce them before waiting.
-          const uint32_t bar = smem_u32(&sh.qempty[qb]);
-          const uint32_t parity = static_cast<uint32_t>((c.n / 2 - 1) & 1);
-          if (!mbar_test(bar, parity)) {
-            announce_all();
-            (void)mbar_wait(bar, parity, &sh.timed_out);
-          }
+  if (warp == kRunProducerWarp) {
+    // ---------------- copies (one thread) ----------------
+    if (lane == 0) {
+      bool new_row = true;
+      for (int i = 0; i < n_mine; ++i) {
+        if (new_row) {
+          const int qb = c.rows_done & 1;
+          if (c.rows_done >= 2)   // the buffer's previous row must be multiplied
+            (void)mbar_wait(smem_u32(&sh.qempty[qb]), static_cast<uint32_t>((c.rows_done / 2 - 1) & 1), &sh.timed_out);
+          mbar_expect(smem_u32(&sh.qfull[qb]), kQBytes);
+          tma_load_3d(q_s + qb * kQBytes, &q_map, 0, 0, c.row, smem_u32(&sh.qfull[qb]));
         }
-        const uint8_t* qrow = p.q + static_cast<int64_t>(c.row) * kQBytes;
-        copy_rows_swizzled<kHeads>(q_s + qb * kQBytes, qrow, pt, kHeads);
-      }
-      const uint8_t* krow = p.k + static_cast<int64_t>(c.row) * p.k_row_stride;
-      const int key0 = (c.tile0 + c.i) * kTileKeys;
-      copy_rows_swizzled<kTileKeys>(k_s + stage * kTileBytes, krow + static_cast<int64_t>(key0) * kDim, pt,
-                                    c.len - key0);
-      cp_async_commit();
-      lag += 1;
-      more = cursor_next(c, p, sh.prefix, B, total_units, stride);
-      if (lag == kPStages) {
-        cp_async_wait<kPStages - 1>();   // the oldest of the kPStages outstanding groups has landed
-        fence_async_proxy();
-        announce_one();
+        const int stage = i % kRunStages;
+        if (i >= kRunStages)
+          (void)mbar_wait(smem_u32(&sh.empty[stage]), static_cast<uint32_t>((i / kRunStages - 1) & 1), &sh.timed_out);
+        mbar_expect(smem_u32(&sh.full[stage]), kTileBytes);
+        tma_load_3d(k_s + stage * kTileBytes, &k_map, 0, c.tile * kTileKeys, c.row, smem_u32(&sh.full[stage]));
+        new_row = c.next(sh.prefix, B);
       }
     }
-    announce_all();
   } else if (warp == kMmaWarp) {
     // ---------------- tensor-core issue (one thread) ----------------
     if (lane == 0) {
-      bool more = true;
-      while (more) {
-        const int stage = c.t % kPStages;
-        const int buf = c.t & 1;
-        const int qb = c.n & 1;
-        if (c.i == 0) (void)mbar_wait(smem_u32(&sh.qfull[qb]), static_cast<uint32_t>((c.n / 2) & 1), &sh.timed_out);
-        if (c.t >= 2) (void)mbar_wait(smem_u32(&sh.tempty[buf]), static_cast<uint32_t>((c.t / 2 - 1) & 1), &sh.timed_out);
-        (void)mbar_wait(smem_u32(&sh.full[stage]), static_cast<uint32_t>((c.t / kPStages) & 1), &sh.timed_out);
+      bool new_row = true;
+      for (int i = 0; i < n_mine; ++i) {
+        const int stage = i % kRunStages, buf = i & 1, qb = c.rows_done & 1;
+        if (new_row) (void)mbar_wait(smem_u32(&sh.qfull[qb]), static_cast<uint32_t>((c.rows_done / 2) & 1), &sh.timed_out);
+        if (i >= 2) (void)mbar_wait(smem_u32(&sh.tempty[buf]), static_cast<uint32_t>((i / 2 - 1) & 1), &sh.timed_out);
+        (void)mbar_wait(smem_u32(&sh.full[stage]), static_cast<uint32_t>((i / kRunStages) & 1), &sh.timed_out);
         tc_fence_after();
-        const uint32_t a_addr = k_s + stage * kTileBytes;
-        const uint32_t b_addr = q_s + qb * kQBytes;
+        const uint32_t a_addr = k_s + stage * kTileBytes, b_addr = q_s + qb * kQBytes;
 #pragma unroll
-        for (int ks = 0; ks < kDim / 32; ++ks)
+        for (int ks = 0; ks < kDim / 32; ++ks)   // 32 bytes of K per instruction, inside the swizzle atom
           mma_f8(tmem + buf * kHeads, smem_desc(a_addr + ks * 32), smem_desc(b_addr + ks * 32), ks > 0 ? 1u : 0u);
         mma_commit(smem_u32(&sh.empty[stage]));
         mma_commit(smem_u32(&sh.tfull[buf]));
-        if (c.i == c.ntile - 1) mma_commit(smem_u32(&sh.qempty[qb]));   // the unit's q buffer is free after these MMAs
-        more = cursor_next(c, p, sh.prefix, B, total_units, stride);
+        new_row = c.next(sh.prefix, B);
+        if (new_row) mma_commit(smem_u32(&sh.qempty[qb]));
       }
     }
   } else {
     // ---------------- epilogue: thread = key (tensor memory lane) ----------------
-    const int key_in_tile = warp * 32 + lane;
-    float w_next = p.w[static_cast<int64_t>(c.row) * kHeads + (tid & (kHeads - 1))];
-    bool more = true;
-    while (more) {
-      if (c.i == 0) {
-        // hand the head weights of this unit's row to all epilogue threads; the next unit's are fetched early
-        asm volatile("bar.sync 1, 128;" ::: "memory");   // everyone is done with the previous unit's weights
-        if (tid < kHeads) sh.w[tid] = w_next;
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        const int u_next = c.u + stride;
-        if (u_next < total_units) {
-          UnitCursor peek = c;
-          peek.u = u_next;
-          cursor_load_unit(peek, p, sh.prefix, B);
-          w_next = p.w[static_cast<int64_t>(peek.row) * kHeads + (tid & (kHeads - 1))];
-        }
+    auto load_w = [&](int row, int b) {
+      if (tid < kHeads) sh.w[b][tid] = p.w[static_cast<int64_t>(row) * kHeads + tid];
+    };
+    if (n_mine > 0) load_w(c.row, 0);
+    if (a.fill) {
+      // -inf behind the rows' last tiles, 4,096 scores at a time dealt out over the CTAs
+      constexpr int kChunk = 4096;
+      const int chunks = (p.L_width + kChunk - 1) / kChunk;
+      for (int64_t u = blockIdx.x; u < static_cast<int64_t>(B) * chunks; u += gridDim.x) {
+        const int row = static_cast<int>(u / chunks), c0 = static_cast<int>(u - static_cast<int64_t>(row) * chunks) * kChunk;
+        const int c1 = min(c0 + kChunk, p.L_width);
+        float* out = p.scores + static_cast<int64_t>(row) * p.score_stride;
+        const int j = max(c0, (sh.prefix[row + 1] - sh.prefix[row]) * kTileKeys);
+        if (j >= c1) continue;
+        const float ninf = __uint_as_float(0xff800000u);
+        const int j4 = min(c1, j + static_cast<int>((4 - ((reinterpret_cast<uintptr_t>(out + j) >> 2) & 3)) & 3));
+        for (int q = j + tid; q < j4; q += kEpilogueWarps * 32) out[q] = ninf;
+        const int n4 = (c1 - j4) / 4;
+        for (int q = tid; q < n4; q += kEpilogueWarps * 32) reinterpret_cast<float4*>(out + j4)[q] = make_float4(ninf, ninf, ninf, ninf);
+        for (int q = j4 + 4 * n4 + tid; q < c1; q += kEpilogueWarps * 32) out[q] = ninf;
       }
-      const int buf = c.t & 1;
-      (void)mbar_wait(smem_u32(&sh.tfull[buf]), static_cast<uint32_t>((c.t / 2) & 1), &sh.timed_out);
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");   // the weights are there
+    const int key_in_tile = warp * 32 + lane;
+    float hint = __uint_as_float(0x7fffffffu);   // NaN: no guess, nothing is handed over
+    unsigned char* row_base = nullptr;
+    int cur = 0, n_cur = 0, n_pending = 0;       // as in indexer_logits_kernel
+    uint32_t pending_base = 0u;
+    auto enter_row = [&]() {
+      if (p.hint != nullptr && p.handover != nullptr) {
+        hint = p.hint[c.row];
+        row_base = p.handover + static_cast<int64_t>(c.row) * FF_HANDOVER_ROW_BYTES;
+      }
+    };
+    auto leave_row = [&]() {
+      if (hint != hint) return;
+      __syncwarp();
+      if (n_pending > 0)
+        store_handover(row_base, sh.handover[warp][cur ^ 1], n_pending, __shfl_sync(0xffffffffu, pending_base, 0), lane);
+      if (n_cur > 0) {
+        uint32_t base = 0u;
+        if (lane == 0) base = atomicAdd(reinterpret_cast<uint32_t*>(row_base), static_cast<uint32_t>(n_cur));
+        store_handover(row_base, sh.handover[warp][cur], n_cur, __shfl_sync(0xffffffffu, base, 0), lane);
+      }
+      __syncwarp();
+      n_cur = n_pending = 0;
+    };
+    int len = 0;
+    if (n_mine > 0) {
+      len = clamp_len(p, c.row);
+      enter_row();
+    }
+    for (int i = 0; i < n_mine; ++i) {
+      const int buf = i & 1, wb = c.rows_done & 1;
+      (void)mbar_wait(smem_u32(&sh.tfull[buf]), static_cast<uint32_t>((i / 2) & 1), &sh.timed_out);
       tc_fence_after();
       const uint32_t taddr = tmem + (static_cast<uint32_t>(warp * 32) << 16) + buf * kHeads;
-      const float s = score_of_lane(taddr, sh.w);
+      const float s = score_of_lane(taddr, sh.w[wb]);
       tc_fence_before();
       mbar_arrive(smem_u32(&sh.tempty[buf]));
-      const int key = (c.tile0 + c.i) * kTileKeys + key_in_tile;
+      const int key = c.tile * kTileKeys + key_in_tile;
       if (key < p.L_width)
-        p.scores[static_cast<int64_t>(c.row) * p.score_stride + key] = key < c.len ? s : __uint_as_float(0xff800000u);
-      more = cursor_next(c, p, sh.prefix, B, total_units, stride);
+        p.scores[static_cast<int64_t>(c.row) * p.score_stride + key] = key < len ? s : __uint_as_float(0xff800000u);
+      if (hint == hint) {
+        if (n_pending > 0) {   // last tile's reservation has long arrived
+          store_handover(row_base, sh.handover[warp][cur ^ 1], n_pending, __shfl_sync(0xffffffffu, pending_base, 0), lane);
+          n_pending = 0;
+        }
+        const bool hit = key < len && !(s < hint);
+        const uint32_t votes = __ballot_sync(0xffffffffu, hit);
+        if (votes != 0u) {
+          if (hit)
+            sh.handover[warp][cur][n_cur + __popc(votes & ((1u << lane) - 1u))] =
+                (static_cast<unsigned long long>(monotone_key(s)) << 32) | static_cast<uint32_t>(~static_cast<uint32_t>(key));
+          n_cur += __popc(votes);
+          if (n_cur > kHandoverWarpBuf - 32) {   // the next tile might not fit: reserve list slots, switch buffers
+            __syncwarp();
+            if (lane == 0) pending_base = atomicAdd(reinterpret_cast<uint32_t*>(row_base), static_cast<uint32_t>(n_cur));
+            n_pending = n_cur;
+            cur ^= 1;
+            n_cur = 0;
+          }
+        }
+      }
+      if (c.next(sh.prefix, B)) {
+        // (c is at the next row; the lists still belong to the one left)
+        leave_row();
+        if (i + 1 < n_mine) {
+          load_w(c.row, c.rows_done & 1);
+          len = clamp_len(p, c.row);
+          enter_row();
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+        }
+      }
     }
+    if (n_mine > 0 && c.tile != 0) leave_row();   // the run ended inside a row
   }
   tc_fence_before();
   __syncthreads();
@@ -662,13 +691,33 @@ constexpr int kMaxDevices = 64;
 std::once_flag g_once[kMaxDevices];
 int g_rc[kMaxDevices];
 std::atomic<int64_t> g_launches{0};
+int g_sms[kMaxDevices];
+std::atomic<decltype(&cuTensorMapEncodeTiled)> g_encode{nullptr};   // from the driver, without linking against it
 void init_device(int device) {
   cudaError_t e = cudaFuncSetAttribute(ffl::indexer_logits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        ffl::kSmemBytes);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(ffl::indexer_logits_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             ffl::kPSmemBytes);
+    e = cudaFuncSetAttribute(ffl::indexer_logits_run_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ffl::kRunSmemBytes);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&g_sms[device], cudaDevAttrMultiProcessorCount, device);
+  if (e == cudaSuccess) {
+    void* entry = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &entry, 12000, cudaEnableDefault, &found);
+    if (e == cudaSuccess && (entry == nullptr || found != cudaDriverEntryPointSuccess)) e = cudaErrorSymbolNotFound;
+    if (e == cudaSuccess) g_encode.store(reinterpret_cast<decltype(&cuTensorMapEncodeTiled)>(entry));
+  }
   g_rc[device] = static_cast<int>(e);
+}
+
+// [n][rows][128] bytes, blocks `stride` bytes apart, in boxes of `box` rows with 128-byte swizzle.
+bool encode_map(CUtensorMap* map, const void* base, int64_t rows, int64_t n, int64_t stride, uint32_t box) {
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(ffl::kDim), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(n)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ffl::kDim), static_cast<cuuint64_t>(stride)};
+  const cuuint32_t boxes[3] = {static_cast<cuuint32_t>(ffl::kDim), box, 1};
+  const cuuint32_t steps[3] = {1, 1, 1};
+  return g_encode.load()(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, boxes, steps,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 }  // namespace
 
@@ -688,10 +737,20 @@ int ff_indexer_logits_launch_handover(const void* q_e4m3, const void* k_e4m3, in
                                       const float* w, const int32_t* lengths, float* scores, int64_t score_stride,
                                       int32_t B, int32_t L_width, int32_t ctas_per_row, const float* hint,
                                       void* handover, int32_t* status, void* stream) {
+  return ff_indexer_logits_launch_fresh(q_e4m3, k_e4m3, k_row_stride_bytes, w, lengths, scores, score_stride, B, L_width,
+                                        ctas_per_row, 0, hint, handover, status, stream);
+}
+
+int ff_indexer_logits_launch_fresh(const void* q_e4m3, const void* k_e4m3, int64_t k_row_stride_bytes, const float* w,
+                                   const int32_t* lengths, float* scores, int64_t score_stride, int32_t B,
+                                   int32_t L_width, int32_t ctas_per_row, int32_t fill, const float* hint,
+                                   void* handover, int32_t* status, void* stream) {
   if (B < 0 || L_width < 0) return fail(-2, "negative B or L_width");
   if ((hint == nullptr) != (handover == nullptr)) return fail(-3, "hint and handover go together");
   if (handover != nullptr && ((reinterpret_cast<uintptr_t>(handover) & 63u) != 0 || ctas_per_row < 0))
     return fail(-2, "the hand-over list must be 64-byte aligned and needs the default kernel (ctas_per_row >= 0)");
+  if (fill != 0 && (ctas_per_row != 0 || B > ffl::kRunMaxRows))
+    return fail(-2, "fill needs ctas_per_row == 0 and at most FF_INDEXER_MAX_FILL_ROWS rows");
   if (B == 0 || L_width == 0) return 0;
   if (q_e4m3 == nullptr || k_e4m3 == nullptr || w == nullptr || lengths == nullptr || scores == nullptr)
     return fail(-3, "q, k, w, lengths and scores must not be NULL");
@@ -721,29 +780,38 @@ int ff_indexer_logits_launch_handover(const void* q_e4m3, const void* k_e4m3, in
   p.status = status;
   p.hint = hint;
   p.handover = static_cast<unsigned char*>(handover);
-  if (ctas_per_row < 0) {
-    // The persistent kernel, two CTAs per SM, units of 8 tiles dealt out round robin.  Measured a few
-    // per cent slower than shares of 32 tiles per CTA (below), which is therefore the default.
-    if (B > ffl::kMaxRowsPersistent) return fail(-6, "the persistent kernel takes at most 1024 rows");
-    int sms = 148;
-    (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int64_t max_units = static_cast<int64_t>(B) * ((tiles + ffl::kUnitTiles - 1) / ffl::kUnitTiles);
-    const int grid = static_cast<int>(max_units < 2 * sms ? max_units : 2 * sms);
-    ffl::indexer_logits_persistent_kernel<<<grid, ffl::kThreads, ffl::kPSmemBytes, static_cast<cudaStream_t>(stream)>>>(p, B);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return fail_cuda(e, "indexer_logits_persistent_kernel");
+  // A K row stride that a tensor map cannot hold (2^40 bytes) goes to the other kernel too.
+  if (ctas_per_row <= 0 && B <= ffl::kRunMaxRows && k_row_stride_bytes < (1ll << 40)) {
+    // Two CTAs per SM, or one per tile where there are fewer tiles.
+    const int64_t most = static_cast<int64_t>(B) * tiles;
+    const ffl::RunParams a = {p, B, fill};
+    CUtensorMap k_map, q_map;
+    if (!encode_map(&k_map, k_e4m3, L_width, B, k_row_stride_bytes, ffl::kTileKeys) ||
+        !encode_map(&q_map, q_e4m3, ffl::kHeads, B, ffl::kQBytes, ffl::kHeads))
+      return fail(-2, "cuTensorMapEncodeTiled rejected q or K");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(most < 2 * g_sms[device] ? most : 2 * g_sms[device]), 1, 1);
+    cfg.blockDim = dim3(ffl::kRunThreads, 1, 1);
+    cfg.dynamicSmemBytes = ffl::kRunSmemBytes;
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // set up behind the running kernel, wait for it inside
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, ffl::indexer_logits_run_kernel, k_map, q_map, a);
+    if (e != cudaSuccess) return fail_cuda(e, "indexer_logits_run_kernel");
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return 0;
   }
-  // Default (ctas_per_row == 0): every row is cut into shares of about 32 tiles (512 KiB of K), but
+  if (ctas_per_row < 0) return fail(-6, "the persistent kernel takes at most 1024 rows");
+  // More rows than the persistent kernel numbers: every row is cut into shares of about 32 tiles (512 KiB of K), but
   // into at least so many that the batch has about four CTAs per SM when every row is full, so that
   // small batches still fill the device.  ctas_per_row > 0 fixes the number of CTAs of a full row.
   int per_row = ctas_per_row;
   int tiles_per_cta = 32;
   if (per_row <= 0) {
-    int sms = 148;
-    (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int want_ctas = (4 * sms + B - 1) / B;             // per row
+    const int want_ctas = (4 * g_sms[device] + B - 1) / B;             // per row
     if (tiles_per_cta * want_ctas > tiles) tiles_per_cta = (tiles + want_ctas - 1) / want_ctas;
     if (tiles_per_cta < 1) tiles_per_cta = 1;
     per_row = (tiles + tiles_per_cta - 1) / tiles_per_cta;

@@ -35,6 +35,11 @@ SIGNATURES = {
         [c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_int32, c_int32,
          c_void_p, c_void_p, c_void_p, c_void_p],
     ),
+    "ff_indexer_logits_launch_fresh": (
+        c_int,
+        [c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_int32, c_int32, c_int32,
+         c_void_p, c_void_p, c_void_p, c_void_p],
+    ),
     "ff_indexer_launch_count": (c_int64, []),
     "ff_indexer_last_error_string": (c_char_p, []),
 }

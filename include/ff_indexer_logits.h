@@ -58,6 +58,15 @@ int ff_indexer_logits_launch_handover(const void* q_e4m3, const void* k_e4m3, in
                                       int64_t score_stride, int32_t B, int32_t L_width, int32_t ctas_per_row,
                                       const float* hint, void* handover, int32_t* status, void* stream);
 
+/* The same for a `scores` buffer that holds nothing yet: with fill = 1 every position behind a row's last key is
+ * written as -inf, not only those inside a processed 128-key tile, so that the caller need not fill the
+ * buffer first.  fill needs ctas_per_row == 0 and B <= FF_INDEXER_MAX_FILL_ROWS; hint and handover may be NULL. */
+#define FF_INDEXER_MAX_FILL_ROWS 1024
+int ff_indexer_logits_launch_fresh(const void* q_e4m3, const void* k_e4m3, int64_t k_row_stride_bytes, const float* w,
+                                   const int32_t* lengths, float* scores, int64_t score_stride, int32_t B,
+                                   int32_t L_width, int32_t ctas_per_row, int32_t fill, const float* hint,
+                                   void* handover, int32_t* status, void* stream);
+
 int64_t ff_indexer_launch_count(void);
 const char* ff_indexer_last_error_string(void);
 

@@ -75,6 +75,26 @@ def test_logits_are_bit_exact_against_the_oracle(oracle, B, L, lens, ctas):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("B,L", [(1, 40000), (300, 257), (1024, 129), (1025, 300)])
+def test_runs_of_tiles_over_many_rows(oracle, B, L):
+    """Runs that start and end inside rows, cross several short or empty ones, and batches just within and
+    beyond the rows one launch numbers; a fresh result holds -inf behind every row's end."""
+    from flash_float_jit_kernels_b200.indexer_logits import indexer_logits_fp8
+    dev = torch.device("cuda:0")
+    q, k, w = _make(B, L, 3 * B, dev)
+    lengths = torch.randint(0, L + 1, (B,), generator=torch.Generator().manual_seed(B), dtype=torch.int32)
+    lengths[B // 2:B // 2 + 3] = 0
+    lengths[-1] = L
+    got = indexer_logits_fp8(q.to(dev), k.to(dev), w.to(dev), lengths.to(dev)).cpu().numpy()
+    for b in sorted({0, 1 % B, B // 3, B // 2 - 1, B // 2 + 1, B - 2, B - 1} & set(range(B))):
+        n = int(lengths[b])
+        exp, _ = oracle.indexer_logits(q[b].float().numpy(), k[b, :n].float().numpy(), w[b].numpy())
+        assert np.array_equal(got[b, :n].view(np.uint32), exp.view(np.uint32)), b
+    behind = np.arange(L)[None, :] >= lengths.numpy()[:, None]
+    assert np.all(np.isneginf(got[behind])) and np.all(np.isfinite(got[~behind]))
+
+
+@pytest.mark.gpu
 def test_logits_feed_the_indexer(oracle):
     """Producer and selector back to back: the top-k of the produced scores is the oracle's
     top-k of the oracle's scores."""

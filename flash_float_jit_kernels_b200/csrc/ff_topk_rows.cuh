@@ -89,18 +89,49 @@ __device__ __forceinline__ uint32_t fast_key(float x) {
   const uint32_t u = __float_as_uint(__fadd_rn(x, 0.0f));
   return u ^ (static_cast<uint32_t>(static_cast<int32_t>(u) >> 31) | 0x80000000u);
 }
-// Digit in sign-magnitude order, as the histogram is filled.
+// Digit in sign-magnitude order, as the histogram is filled, and the same place for a monotone digit.
+__device__ __forceinline__ int rows_raw_of(int m) { return m >= kRowsBins / 2 ? m - kRowsBins / 2 : kRowsBins - 1 - m; }
 __device__ __forceinline__ uint32_t rows_raw_digit(float x) { return __float_as_uint(__fadd_rn(x, 0.0f)) >> kRowsShift; }
 
-// A listed survivor: score bits and position.
-__device__ __forceinline__ uint64_t list_entry(float x, int pos) {
-  return (static_cast<uint64_t>(__float_as_uint(x)) << 32) | static_cast<uint32_t>(pos);
-}
+// The survivors in arrival order: a score and its window position, in turn.
+template <int CAP>
+struct RowList {
+  float* x;
+  __device__ __forceinline__ void put(int i, float score, int32_t pos) const {
+    reinterpret_cast<uint2*>(x)[i] = make_uint2(__float_as_uint(score), static_cast<uint32_t>(pos));
+  }
+};
 
 // A packed bin: twice the elements above it << 19 | twice the elements in it (cut: rows with so many in
 // one of the bins that matter do not use them).
 constexpr int kPackShift = 19;
 constexpr int kPackMax = (1 << (kPackShift - 1)) - 1;   // elements in a bin
+__device__ __forceinline__ uint32_t packed_bin(int above, int count) {
+  return (static_cast<uint32_t>(above) << (kPackShift + 1)) | static_cast<uint32_t>(2 * min(count, kPackMax));
+}
+
+// Where to cut inside the threshold digit so that a few more than the `wanted` largest of its `in_bin` scores are
+// kept: the density of scores is taken as linear over the digit, from its own count and the next
+// digit's (c0, c1): above a point x of the way down lie (c0 + c1) / 2 x + (c0 - c1) / 2 x^2 of them,
+// solved for the wanted count plus a margin (the steps of scores rounded to bf16,
+// sixteen to a digit, and four standard deviations).  Returns key bits above the digit's lower edge;
+// keep: how many are expected (less than wanted: they do not fit in `room`); spread: the count that the whole digit
+// would have at the kept part's density, which is what the finish interpolates with.
+__device__ __forceinline__ uint32_t cut_in_digit(const uint32_t* packed, int t, int in_bin, int wanted, int room, int& keep, int& spread) {
+  const float c0 = static_cast<float>(in_bin);
+  const int margin = (in_bin >> 4) + static_cast<int>(2.f * sqrtf(c0)) + 8;
+  keep = min(in_bin, wanted + margin);
+  if (keep > room) keep = room >= wanted + (margin >> 1) ? room : -1;
+  const int up = t + 1;
+  float c1 = static_cast<float>((packed[rows_raw_of(up)] & ((1u << kPackShift) - 1u)) >> 1);
+  if ((up & 7) == 0) c1 *= up >= kRowsBins / 2 ? 0.5f : 2.f;   // the next digit spans a step of another width
+  c1 = fminf(c1, 3.f * c0);
+  const float b = 0.5f * (c0 + c1), a = 0.5f * (c0 - c1), want = static_cast<float>(keep);
+  const float x = 2.f * want / (b + sqrtf(fmaxf(b * b + 4.f * a * want, 0.f)));
+  const bool all = keep >= in_bin || !(x < 1.f);
+  spread = all ? in_bin : static_cast<int>(fminf(want / x, static_cast<float>(kPackMax)));
+  return all ? 0u : static_cast<uint32_t>((1.f - x) * static_cast<float>(1 << kRowsShift));
+}
 
 // Suffix scan of the bins in monotone order (raw: the array is in rows_raw_digit() order).  Every non-empty bin
 // with fewer than `limit` elements above it is packed in place, and the bin that reaches the limit
@@ -136,8 +167,7 @@ __device__ __forceinline__ void pack_bins(uint32_t* hist, bool raw, int limit, R
     for (int i = 0; i < per; ++i) {              // from the thread's largest digit down
       const int n = static_cast<int>(up ? c[per - 1 - i] : c[i]);
       if (n != 0 && running < limit) {
-        hist[base + (up ? per - 1 - i : i)] = (static_cast<uint32_t>(running) << (kPackShift + 1)) |
-                                              static_cast<uint32_t>(2 * min(n, kPackMax));
+        hist[base + (up ? per - 1 - i : i)] = packed_bin(running, n);
         largest = max(largest, n);
         if (running + n >= limit) {
           sh.t = m0 + per - 1 - i;
@@ -189,30 +219,6 @@ struct RowGroup {
   }
   static __device__ __forceinline__ constexpr int distance(int e) { return (e / kPU) * kPU * NT + (e & (kPU - 1)); }
 };
-
-// Where to cut inside the threshold digit so that a few more than the `wanted` largest of its `in_bin` scores are
-// kept: the density of scores is taken as linear over the digit, from its own count and the next
-// digit's (c0, c1): above a point x of the way down lie (c0 + c1) / 2 x + (c0 - c1) / 2 x^2 of them,
-// solved for the wanted count plus a margin (the steps of scores rounded to bf16,
-// sixteen to a digit, and four standard deviations).  Returns key bits above the digit's lower edge;
-// keep: how many are expected (less than wanted: they do not fit in `room`); linear: how many there would be
-// if the scores were spread evenly over the digit, as the finish takes them to be.
-__device__ __forceinline__ uint32_t cut_in_digit(const uint32_t* packed, int t, int in_bin, int wanted, int room, int& keep, int& linear) {
-  const float c0 = static_cast<float>(in_bin);
-  const int margin = (in_bin >> 4) + static_cast<int>(2.f * sqrtf(c0)) + 8;
-  keep = min(in_bin, wanted + margin);
-  if (keep > room) keep = room >= wanted + (margin >> 1) ? room : -1;
-  const int up = t + 1;
-  float c1 = static_cast<float>((packed[up >= kRowsBins / 2 ? up - kRowsBins / 2 : kRowsBins - 1 - up] &
-                                 ((1u << kPackShift) - 1u)) >> 1);
-  if ((up & 7) == 0) c1 *= up >= kRowsBins / 2 ? 0.5f : 2.f;   // the next digit spans a step of another width
-  c1 = fminf(c1, 3.f * c0);
-  const float b = 0.5f * (c0 + c1), a = 0.5f * (c0 - c1), want = static_cast<float>(keep);
-  const float x = 2.f * want / (b + sqrtf(fmaxf(b * b + 4.f * a * want, 0.f)));
-  const bool all = keep >= in_bin || !(x < 1.f);
-  linear = all ? in_bin : min(in_bin, static_cast<int>(x * c0) + 2);
-  return all ? 0u : static_cast<uint32_t>((1.f - x) * static_cast<float>(1 << kRowsShift));
-}
 
 // The rare rows whose survivors do not fit the list (heavy ties, scores crowded into one digit): further
 // digits of the composite, one sweep each, until they fit.  Returns the smallest composite that
@@ -280,42 +286,47 @@ __device__ __noinline__ uint64_t deeper_digits(const Chunk<T>& c, uint32_t* hist
 }
 
 // Sweep 2: every score not below vmin (EXACT: whose composite is not below floor_comp) goes to the list.
-// `first` is the row's first group, still in registers.  A warp takes 512 scores at a time: the
-// lanes' hit counts are summed with five ballots and one shared atomic reserves the warp's slots.
-template <typename T, int NT, bool EXACT>
+// `first` is the row's first group, still in registers.  A warp takes 512 scores at a time: a scan over the lanes' hit
+// counts, one shared atomic for the warp's slots, and predicated stores (no hit mask: testing a score
+// again is one instruction, picking its bit out of a mask three).
+template <typename T, int NT, int CAP, bool EXACT>
 __device__ __forceinline__ void collect_row(const Chunk<T>& c, const RowGroup<T, NT>* first, float vmin, uint64_t floor_comp,
-                                            uint64_t* list, int cap, RowsShared& sh) {
+                                            RowList<CAP> list, RowsShared& sh) {
   using Group = RowGroup<T, NT>;
   const int lane = threadIdx.x & 31;
-  const uint32_t list_at = smem_addr(list);
+  const uint32_t list_at = smem_addr(list.x);
+  auto is_hit = [&](float x, int pos) { return !(x < vmin) && (!EXACT || make_comp(fast_key(x), pos) >= floor_comp); };
   auto take = [&](const Group& g, int u0, auto full) {
     constexpr bool FULL = decltype(full)::value;
     const int pos0 = Group::position(c, u0);
-    uint32_t hits = 0u;
-    g.template each<FULL>(c, u0, [&](float x, int e) {
-      bool hit = !(x < vmin);
-      if (EXACT) hit = hit && make_comp(fast_key(x), pos0 + Group::distance(e)) >= floor_comp;
-      if (hit) hits |= 1u << e;
-    });
-    if (!__any_sync(0xffffffffu, hits != 0u)) return;
-    const uint32_t n = static_cast<uint32_t>(__popc(hits));
-    const uint32_t lt = (1u << lane) - 1u;
-    int before = 0, total = 0;
+    int n = 0;
+    g.template each<FULL>(c, u0, [&](float x, int e) { n += is_hit(x, pos0 + Group::distance(e)) ? 1 : 0; });
+    int incl = n;
 #pragma unroll
-    for (int b = 0; b < 5; ++b) {
-      const uint32_t plane = __ballot_sync(0xffffffffu, n & (1u << b));
-      before += __popc(plane & lt) << b;
-      total += __popc(plane) << b;
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += v;
     }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    if (total == 0) return;
     int base = 0;
     if (lane == 0) base = atomicAdd(&sh.count, total);
     base = __shfl_sync(0xffffffffu, base, 0);
-    if (base + total > cap) return;
-    uint32_t at = list_at + 8u * static_cast<uint32_t>(base + before);
+    if (base + total > CAP) return;
+    uint32_t at = list_at + 8u * static_cast<uint32_t>(base + incl - n);
     g.template each<FULL>(c, u0, [&](float x, int e) {
-      asm volatile(
-          "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p st.shared.v2.b32 [%0], {%1, %2};\n\t@p add.u32 %0, %0, 8;\n\t}"
-          : "+r"(at) : "r"(pos0 + Group::distance(e)), "r"(__float_as_uint(x)), "r"(hits & (1u << e)) : "memory");
+      const int pos = pos0 + Group::distance(e);
+      if constexpr (EXACT) {
+        if (is_hit(x, pos)) {
+          asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(__float_as_uint(x)), "r"(pos) : "memory");
+          at += 8u;
+        }
+      } else {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.geu.f32 p, %1, %2;\n\t@p st.shared.v2.b32 [%0], {%4, %3};\n\t"
+            "@p add.u32 %0, %0, 8;\n\t}"
+            : "+r"(at) : "f"(x), "f"(vmin), "r"(pos), "r"(__float_as_uint(x)) : "memory");
+      }
     });
   };
 #pragma unroll 1
@@ -324,17 +335,21 @@ __device__ __forceinline__ void collect_row(const Chunk<T>& c, const RowGroup<T,
     if (first != nullptr && u0 == c.fb) g = *first; else g.load(c, u0);
     if (u0 + Group::kStep <= c.fe) take(g, u0, std::true_type{}); else take(g, u0, std::false_type{});
   }
-  float x = 0.f;
-  const int pos = partial_element(c, x);
-  if (pos >= 0 && !(x < vmin) && (!EXACT || make_comp(fast_key(x), pos) >= floor_comp)) {
-    const int at = atomicAdd(&sh.count, 1);
-    if (at < cap) list[at] = list_entry(x, pos);
+  if (c.head || c.tail) {   // (uniform)
+    float x = 0.f;
+    const int pos = partial_element(c, x);
+    if (pos >= 0 && is_hit(x, pos)) {
+      const int at = atomicAdd(&sh.count, 1);
+      if (at < CAP) {
+        list.put(at, x, pos);
+      }
+    }
   }
 }
 
-template <typename T, int NT>
-__device__ __noinline__ void collect_row_exact(const Chunk<T>& c, uint64_t floor_comp, uint64_t* list, int cap, RowsShared& sh) {
-  collect_row<T, NT, true>(c, nullptr, prefilter_value(static_cast<uint32_t>(floor_comp >> 32)), floor_comp, list, cap, sh);
+template <typename T, int NT, int CAP>
+__device__ __noinline__ void collect_row_exact(const Chunk<T>& c, uint64_t floor_comp, RowList<CAP> list, RowsShared& sh) {
+  collect_row<T, NT, CAP, true>(c, nullptr, prefilter_value(static_cast<uint32_t>(floor_comp >> 32)), floor_comp, list, sh);
 }
 
 // How a survivor becomes an expected rank: its digit picks a packed bin (elements above, elements in it), and
@@ -376,9 +391,9 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   constexpr int kCap = PER * NT;
   uint32_t* hist = reinterpret_cast<uint32_t*>(smem);
   uint32_t* bucketed = hist;                                                 // depths, bucket by bucket
-  uint64_t* list = reinterpret_cast<uint64_t*>(smem + kRowsBins * 4);
-  uint32_t* bins = reinterpret_cast<uint32_t*>(list);                        // 2 * kCap finish bins
-  int32_t* ranked = reinterpret_cast<int32_t*>(list);                        // kCap positions
+  const RowList<kCap> list = {reinterpret_cast<float*>(smem + kRowsBins * 4)};
+  uint32_t* bins = reinterpret_cast<uint32_t*>(list.x);                      // 2 * kCap finish bins
+  int32_t* ranked = reinterpret_cast<int32_t*>(list.x);                      // kCap positions
   const int tid = threadIdx.x;
   auto clear_words = [&](uint32_t* a, int n) {
 #pragma unroll 4
@@ -480,7 +495,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
 #pragma unroll 4
         for (int i = tid; i < n; i += NT) {
           const uint64_t c = __ldcg(given + i);
-          list[i] = list_entry(__uint_as_float(bits_of_key(comp_key(c))), comp_index(c));
+          list.put(i, __uint_as_float(bits_of_key(comp_key(c))), comp_index(c));
         }
         listed = true;
       }
@@ -491,7 +506,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
         header[0] = header[1] = 0u;   // empty for the producer's next launch
       }
     } else if (use) {
-      collect_row<T, NT, false>(chunk, nullptr, hint, 0ull, list, kCap, sh);
+      collect_row<T, NT, kCap, false>(chunk, nullptr, hint, 0ull, list, sh);
       __syncthreads();
       const int n = sh.count;
       listed = n >= k && n <= kCap;
@@ -535,22 +550,24 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     // ---- sweep 2 ----
     const int above = sh.above, in_bin = sh.total - above;
     const uint32_t bin_key = static_cast<uint32_t>(sh.t) << kRowsShift;
-    int keep, linear;
-    const uint32_t cut = bin_key + cut_in_digit(hist, sh.t, in_bin, k - above, kCap - above, keep, linear);
+    int keep, spread;
+    const uint32_t cut = bin_key + cut_in_digit(hist, sh.t, in_bin, k - above, kCap - above, keep, spread);
     bool exact = bin_key > 0xff800000u || sh.max_bin > kPackMax || keep < k - above ||
                  (sh.total > kCap && 8 * sh.max_bin > 7 * sh.total);
     if (!exact) {
-      collect_row<T, NT, false>(chunk, &first, prefilter_value(cut), 0ull, list, kCap, sh);
+      collect_row<T, NT, kCap, false>(chunk, &first, prefilter_value(cut), 0ull, list, sh);
+      if (tid == 0) hist[rows_raw_of(sh.t)] = packed_bin(above, spread);   // (read in the finish)
       __syncthreads();
       const int n = sh.count;
-      span = min(above + linear, kCap);
+      span = above + keep;
       if (n < k || n > kCap) {   // the interpolation was off
         __syncthreads();
         if (tid == 0) sh.count = 0;
         __syncthreads();
         exact = n > kCap || sh.total > kCap;
         if (!exact) {
-          collect_row<T, NT, false>(chunk, &first, prefilter_value(bin_key), 0ull, list, kCap, sh);
+          if (tid == 0) hist[rows_raw_of(sh.t)] = packed_bin(above, in_bin);
+          collect_row<T, NT, kCap, false>(chunk, &first, prefilter_value(bin_key), 0ull, list, sh);
           span = sh.total;
           __syncthreads();
         }
@@ -561,7 +578,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
       rebuild = true;
       const uint64_t floor_comp = sh.total <= kCap ? static_cast<uint64_t>(sh.t) << rows_level_shift(0)
                                                    : deeper_digits<T, NT>(chunk, hist, k, kCap, sh, p.status);
-      collect_row_exact<T, NT>(chunk, floor_comp, list, kCap, sh);
+      collect_row_exact<T, NT, kCap>(chunk, floor_comp, list, sh);
       __syncthreads();
     }
   }
@@ -591,10 +608,11 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     uint32_t value_bits = 0u;
     mine([&](int j) {
       if (tid + j * NT < n) {
-        const uint64_t e = list[tid + j * NT];
-        value_bits |= static_cast<uint32_t>(e >> 32);
-        pos[j] = static_cast<int32_t>(e);
-        depth[j] = __float_as_uint(__fadd_rn(__uint_as_float(static_cast<uint32_t>(e >> 32)), 0.0f));
+        const uint2 entry = reinterpret_cast<const uint2*>(list.x)[tid + j * NT];
+        const float x = __uint_as_float(entry.x);
+        pos[j] = static_cast<int32_t>(entry.y);
+        value_bits |= __float_as_uint(x);
+        depth[j] = __float_as_uint(__fadd_rn(x, 0.0f));   // (-0.0 and NaN as in the keys)
         if (!rebuild) where[j] = hist[depth[j] >> kRowsShift];
       }
     });
@@ -702,29 +720,39 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   }
   __syncthreads();
   FF_TRACE(p, 24);
+  // Rank inside the bucket by counting.  (The bins have been read: the ranked positions may take their place.)
+  bool tied = false;
   mine([&](int j) {
     if (pos[j] >= 0) {
-      const uint32_t size = where[j] & 0xffffu;
+      const uint32_t size = where[j] & 0xffffu, d = depth[j];
       uint32_t rank = where[j] >> 16;
       const uint32_t* bucket = bucketed + rank;
       if (FF_IN_RANGE(p, static_cast<int>(rank + size) - 1, kCap, 17)) {
-        rank += (bucket[0] < depth[j] ? 1u : 0u) + (bucket[size > 1u ? 1 : 0] < depth[j] ? 1u : 0u);   // most buckets have no more
+        // up to three entries without a loop; what is not there compares as the largest depth (a wrong "tied" does no harm)
+        const uint32_t b0 = bucket[0], b1 = size > 1u ? bucket[1] : 0xffffffffu, b2 = size > 2u ? bucket[2] : 0xffffffffu;
+        rank += (b0 < d ? 1u : 0u) + (b1 < d ? 1u : 0u) + (b2 < d ? 1u : 0u);
+        bool more = (b0 == d && b1 == d) || (b1 == d && b2 == d) || (b0 == d && b2 == d);
+        if (size > 3u) {
+          uint32_t same = (b0 == d ? 1u : 0u) + (b1 == d ? 1u : 0u) + (b2 == d ? 1u : 0u);
 #pragma unroll 1
-        for (uint32_t q = 2; q < size; ++q) rank += bucket[q] < depth[j] ? 1u : 0u;
+          for (uint32_t q = 3; q < size; ++q) {
+            rank += bucket[q] < d ? 1u : 0u;
+            same += bucket[q] == d ? 1u : 0u;
+          }
+          more = same > 1u;
+        }
+        tied |= more;
       }
       where[j] = rank;
+      if (FF_IN_RANGE(p, rank, kCap, 18)) ranked[rank] = pos[j];
     }
   });
-  mine([&](int j) {
-    if (pos[j] >= 0) ranked[where[j]] = pos[j];
-  });
-  __syncthreads();
-  // Survivors of one depth have taken the same rank; all but one of them find another's position there.
-  uint32_t beaten = 0u;
-  mine([&](int j) {
-    if (pos[j] >= 0 && ranked[where[j]] != pos[j]) beaten |= 1u << j;
-  });
-  if (__syncthreads_or(beaten != 0u ? 1 : 0)) {
+  if (__syncthreads_or(tied ? 1 : 0)) {
+    // Survivors of one depth have taken the same rank; all but one of them find another's position there.
+    uint32_t beaten = 0u;
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (pos[j] >= 0 && ranked[where[j]] != pos[j]) beaten |= 1u << j;
     // Each moves down by the positions below its own that share its rank.
     int32_t* tied_pos = reinterpret_cast<int32_t*>(hist);
     uint32_t* tied_rank = reinterpret_cast<uint32_t*>(ranked + kCap);

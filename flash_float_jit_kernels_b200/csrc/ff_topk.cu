@@ -46,6 +46,7 @@ int g_init_rc[kMaxDevices];
 int g_max_cluster[kMaxDevices];  // largest schedulable cluster size per device
 int g_sm_count[kMaxDevices];
 int g_active_clusters[kMaxDevices][5];  // co-resident clusters of size 1, 2, 4, 8, 16
+int g_rows_clusters_of_4[kMaxDevices];  // co-resident clusters of four CTAs of topk_rows_kernel, two on an SM
 
 int fail(int code, const char* msg) {
   snprintf(g_err, sizeof(g_err), "%s", msg);
@@ -65,11 +66,11 @@ cudaError_t prepare_kernel(K kernel) {
 }
 
 template <typename K>
-int active_clusters_for(K kernel, int c) {
+int active_clusters_for(K kernel, int c, int smem_bytes = ff::smem_bytes_for(ff::kMaxStages)) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(c, 1, 1);
   cfg.blockDim = dim3(ff::kThreads, 1, 1);
-  cfg.dynamicSmemBytes = ff::smem_bytes_for(ff::kMaxStages);
+  cfg.dynamicSmemBytes = smem_bytes;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = c;
@@ -108,8 +109,8 @@ int max_cluster_for(K kernel) {
 }
 
 using RowsKernel = void (*)(const ff::RowsParams);
-RowsKernel rows_kernel(int threads, int dtype, bool hints);
-int rows_smem(int threads, bool hints);
+RowsKernel rows_kernel(int shape, int dtype, bool hints);
+int rows_smem(int shape, bool hints);
 
 void init_device(int device) {
   int prev = 0;
@@ -128,16 +129,19 @@ void init_device(int device) {
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ff::cp_merge_sorted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              ff::kMaxPeers * ff::kMaxK * static_cast<int>(sizeof(uint32_t)));
-  for (int threads : {256, 1024})
+  for (int shape : {256, 1024, -20512})
     for (int dtype : {FF_DTYPE_F32, FF_DTYPE_BF16, FF_DTYPE_F16})
-      for (int hints : {0, 1})
+      for (int hints = 0; hints < (shape < 0 ? 1 : 2); ++hints) {
+        const RowsKernel kernel = rows_kernel(shape, dtype, hints != 0);
         if (e == cudaSuccess)
-          e = cudaFuncSetAttribute(rows_kernel(threads, dtype, hints != 0), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   rows_smem(threads, hints != 0));
+          e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_smem(shape, hints != 0));
+        if (e == cudaSuccess && shape < 0) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      }
   if (e == cudaSuccess) {
     g_max_cluster[device] = max_cluster_for(ff::topk_cluster_kernel<false, ff::kModePlain>);
     for (int i = 0; i < 5; ++i)
       g_active_clusters[device][i] = active_clusters_for(ff::topk_cluster_kernel<false, ff::kModePlain>, 1 << i);
+    g_rows_clusters_of_4[device] = active_clusters_for(rows_kernel(-40512, FF_DTYPE_F32, false), 4, rows_smem(-40512, false));
     int sms = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     g_sm_count[device] = sms > 0 ? sms : 148;
@@ -288,20 +292,25 @@ int launch(const ff::TopkParams& p, int cluster, cudaStream_t stream, int dtype 
 // The one-CTA-per-row kernels (ff_topk_rows.cuh), by score type, CTA size and guesses.
 // Lists of 2,560 and 3,072 survivors: k, a margin inside the threshold digit, room to spare; a caller's guess may
 // let 4,096 through.
-int rows_cap(int threads, bool hints) { return hints ? ff::kSortCap : threads == 256 ? 256 * 10 : 1024 * 3; }
-int rows_block(int threads, bool hints) { return threads == 256 && hints ? 512 : threads; }
+// A shape is the threads per CTA, negative and with the cluster size in front of it for a cluster per row
+// (-80512: eight CTAs of 512 threads).
+int shape_threads(int shape) { return (shape < 0 ? -shape : shape) % 10000; }
+int shape_cluster(int shape) { return shape < 0 ? -shape / 10000 : 1; }
+int rows_cap(int shape, bool hints) { return hints ? ff::kSortCap : shape_threads(shape) == 1024 ? 1024 * 3 : 256 * 10; }
+int rows_block(int shape, bool hints) { return shape_threads(shape) == 256 && hints ? 512 : shape_threads(shape); }
 template <typename T>
-RowsKernel rows_kernel(int threads, bool hints) {
-  if (threads == 256) return hints ? ff::topk_rows_kernel<T, 512, 8, 2, true> : ff::topk_rows_kernel<T, 256, 10, 4, false>;
-  return hints ? ff::topk_rows_kernel<T, 1024, 4, 1, true> : ff::topk_rows_kernel<T, 1024, 3, 1, false>;
+RowsKernel rows_kernel(int shape, bool hints) {
+  if (shape < 0) return ff::topk_rows_kernel<T, 512, 5, 2, false, true>;   // (rows with guesses have one CTA)
+  if (shape == 256) return hints ? ff::topk_rows_kernel<T, 512, 8, 2, true, false> : ff::topk_rows_kernel<T, 256, 10, 4, false, false>;
+  return hints ? ff::topk_rows_kernel<T, 1024, 4, 1, true, false> : ff::topk_rows_kernel<T, 1024, 3, 1, false, false>;
 }
-RowsKernel rows_kernel(int threads, int dtype, bool hints) {
-  return dtype == FF_DTYPE_BF16 ? rows_kernel<__nv_bfloat16>(threads, hints)
-                                : dtype == FF_DTYPE_F16 ? rows_kernel<__half>(threads, hints) : rows_kernel<float>(threads, hints);
+RowsKernel rows_kernel(int shape, int dtype, bool hints) {
+  return dtype == FF_DTYPE_BF16 ? rows_kernel<__nv_bfloat16>(shape, hints)
+                                : dtype == FF_DTYPE_F16 ? rows_kernel<__half>(shape, hints) : rows_kernel<float>(shape, hints);
 }
-int rows_smem(int threads, bool hints) { return ff::rows_smem_bytes(rows_cap(threads, hints)); }
+int rows_smem(int shape, bool hints) { return ff::rows_smem_bytes(rows_cap(shape, hints), shape < 0); }
 
-int launch_rows(const ff::TopkParams& p, int threads, cudaStream_t stream, int dtype) {
+int launch_rows(const ff::TopkParams& p, int shape, cudaStream_t stream, int dtype) {
   ff::RowsParams q = {};
   q.scores = p.scores;
   q.row_stride = p.row_stride;
@@ -323,39 +332,60 @@ int launch_rows(const ff::TopkParams& p, int threads, cudaStream_t stream, int d
   q.hint_out = p.hint_out;
   q.handover = p.handover;
   q.trace = g_trace.load(std::memory_order_relaxed);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(p.B), 1, 1);
   const bool hints = p.hint_in != nullptr || p.hint_out != nullptr;
-  cfg.blockDim = dim3(static_cast<unsigned>(rows_block(threads, hints)), 1, 1);
-  cfg.dynamicSmemBytes = static_cast<size_t>(rows_smem(threads, hints));
+  const int cluster = shape_cluster(shape);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(p.B) * cluster, 1, 1);
+  cfg.blockDim = dim3(static_cast<unsigned>(rows_block(shape, hints)), 1, 1);
+  cfg.dynamicSmemBytes = static_cast<size_t>(rows_smem(shape, hints));
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
   if (programmatic_launch_enabled()) {
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.numAttrs = 1;
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
   }
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, rows_kernel(threads, dtype, hints), q);
+  if (shape < 0) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, rows_kernel(shape, dtype, hints), q);
   if (e != cudaSuccess) return fail_cuda(e, "cudaLaunchKernelEx(topk_rows_kernel)");
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return 0;
 }
 
-// CTA size of the one-CTA-per-row kernel for this batch, or 0: rows get a cluster or several (also whenever a
-// launch shape is forced).  Measured on B200 (k = 2048): up to one row per SM a CTA of 1024 threads, which takes
-// 8.6 us for 4 Ki columns, 9.6 for 16 Ki, 11.9 for 32 Ki and 16.0 for 64 Ki; a cluster takes 12.6 / 12.7 / 13.1 / 13.8
-// with sixteen CTAs, and more with the fewer CTAs that larger batches leave for a row (64 rows of 64 Ki: 18.6).
-// Beyond that four CTAs of 256 threads per SM (296 rows of 16 Ki: 15.0 us against 19.1), unless a second
-// row per SM is all there is and the rows are long (296 rows of 64 Ki: 41 against 38).
-int choose_rows_threads(int device, int32_t B, int64_t L_width) {
+// Shape of topk_rows_kernel for this batch, or 0: the kernel of ff_topk_kernel.cuh (also whenever a launch shape is
+// forced; `split`: that one would split the row over several clusters).  Measured on B200, k = 2048:
+//   * more rows than SMs: four CTAs of 256 threads per SM (296 rows of 16 Ki: 14.6 us against 18.9 with one CTA of 1024),
+//     unless a second row per SM is all there is and the rows are long (296 rows of 64 Ki: 41 against 38);
+//   * one CTA of 1024 threads: 8.5 us for 4 Ki columns, 9.2 for 16 Ki, 11.4 for 32 Ki, 15.6 for 64 Ki, 23.6 for 128 Ki;
+//   * a cluster of 512-thread CTAs, four: 10.7 us for 32 Ki, 12.4 for 64 Ki, 15.3 for 128 Ki; eight: 11.2, 11.2, 12.9;
+//     sixteen: 12.5 for 128 Ki, 13.9 for 256 Ki, 16.2 for 512 Ki.  As many as the device holds with an SM for each CTA
+//     (two on an SM slow each other down: 32 rows of 64 Ki 13.8 us with four, 18.5 with eight), but four also for long
+//     rows of up to as many as fit two on an SM (64 ragged rows of 128 Ki: 20.8 us against 23.5 in clusters of two);
+//   * ff_topk_kernel.cuh: 13.8 us for 64 Ki, 14.3 for 128 Ki, 15.0 for 256 Ki, 16.8 for 512 Ki (sixteen CTAs; 12.4, 12.5 and
+//     12.9 split over clusters), 24.7 for 64 rows of 128 Ki; with guesses it is the faster one from 48 Ki columns up.
+int choose_rows_shape(int device, int32_t B, int64_t L_width, bool hints, bool split) {
   if (g_cluster_override.load() != 0 || g_groups_override.load() != 0) return 0;
   const int sms = g_sm_count[device];
-  if (B <= sms) {
-    const int64_t longest = B <= 8 ? 40960 : B <= 18 ? 49152 : B <= 37 ? 40960 : B <= 74 ? 98304 : 0x7fffffff;
-    return L_width <= longest ? 1024 : 0;
+  if (B > sms) return B <= 2 * sms && L_width > 49152 ? 1024 : 256;
+  const int* one_per_sm = g_active_clusters[device];   // of 1, 2, 4, 8, 16 CTAs
+  if (2 * B > sms) return 1024;
+  if (hints) return L_width <= (B <= 8 ? 40960 : B <= 18 ? 49152 : B <= 37 ? 65536 : 98304) ? 1024 : 0;
+  if (split || L_width > 524288) return 0;
+  if (B > one_per_sm[2]) {
+    if (L_width <= 81920) return 1024;
+    return L_width <= 131072 && B <= g_rows_clusters_of_4[device] ? -40512 : 0;
   }
-  return B <= 2 * sms && L_width > 49152 ? 1024 : 256;
+  if (L_width <= (B > one_per_sm[3] ? 32768 : 20480)) return 1024;
+  if (L_width <= (B > one_per_sm[3] ? 131072 : 40960)) return -40512;
+  if (B > one_per_sm[3]) return 0;
+  return L_width > 98304 && B <= one_per_sm[4] ? -160512 : -80512;
 }
 
 // Built-in scratch for ff_topk_launch_static: enough for FF_TOPK_STATIC_MAX_ROWS
@@ -444,6 +474,10 @@ int ff_topk_policy_launch_shape(int32_t B, int64_t L_width, int32_t k, int32_t h
   int groups = 1;
   if (has_workspace != 0)
     groups = choose_groups(device, B, L_width, ff_topk_workspace_bytes(B, L_width, k), &cluster, hinted != 0);
+  if (const int shape = choose_rows_shape(device, B, L_width, hinted != 0, groups > 1)) {
+    cluster = shape_cluster(shape);
+    groups = 1;
+  }
   out2[0] = cluster;
   out2[1] = groups;
   return 0;
@@ -534,13 +568,13 @@ int transform_launch_impl(const void* scores_any, int dtype, int64_t row_stride,
     static_assert(FF_TOPK_HANDOVER_ROW_BYTES == ff::kHandoverRowBytes, "hand-over layout");
     p.handover = static_cast<unsigned char*>(handover);
   }
-  if (const int threads = choose_rows_threads(device, B, L_width))
-    return launch_rows(p, threads, static_cast<cudaStream_t>(stream), dtype);
   int cluster = choose_cluster(device, B, L_width, k);
   if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
     p.groups = choose_groups(device, B, L_width, workspace_bytes, &cluster, hint_in != nullptr);
     p.workspace = static_cast<uint32_t*>(workspace);
   }
+  if (const int shape = choose_rows_shape(device, B, L_width, hint_in != nullptr || hint_out != nullptr, p.groups > 1))
+    return launch_rows(p, shape, static_cast<cudaStream_t>(stream), dtype);
   return launch<false>(p, cluster, static_cast<cudaStream_t>(stream), dtype);
 }
 
@@ -630,6 +664,8 @@ int ff_topk_launch_static(const float* scores, int64_t row_stride, const int32_t
   p.status = status;
   int cluster = choose_cluster(device, B, L_width, k);
   p.groups = choose_groups(device, B, L_width, FF_TOPK_STATIC_MAX_ROWS * row_bytes, &cluster);
+  if (const int shape = choose_rows_shape(device, B, L_width, false, p.groups > 1))
+    return launch_rows(p, shape, static_cast<cudaStream_t>(stream), FF_DTYPE_F32);
   p.workspace = scratch;
   if (p.groups > 1) {
     // Only rows split over several clusters touch the scratch.  The array keeps whatever the

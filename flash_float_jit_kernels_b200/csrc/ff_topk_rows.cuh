@@ -48,14 +48,59 @@ constexpr int kRowsShift = 32 - kRowsBits;
 // Shared memory of a CTA whose list holds `cap` survivors, in two regions:
 //   histogram, then the bucketed survivors (32 bits each)
 //   list (64 bits each), then two finish bins per survivor (32 bits each), then the ranked positions
-__host__ __device__ constexpr int rows_smem_bytes(int cap) { return kRowsBins * 4 + cap * 8; }
+// and in a cluster the row's histogram and this CTA's own list behind them.
+__host__ __device__ constexpr int rows_smem_bytes(int cap, bool cluster) {
+  return (kRowsBins * 4 + cap * 8) * (cluster ? 2 : 1);
+}
 static_assert(kRowsBins >= kSortCap, "the bucketed survivors take the histogram's place");
+
+// ---- a row shared by the CTAs of a cluster ----
+__device__ __forceinline__ uint32_t cluster_size() {
+  uint32_t n;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return n;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t n;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(n));
+  return n;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  cluster_arrive();
+  cluster_wait();
+}
+__device__ __forceinline__ void dsmem_red_add(uint32_t addr, uint32_t v) {
+  asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+// Adds this CTA's non-zero counts to every CTA's merged ones (n a multiple of 4; a power of two CTAs).  Everybody
+// pushes and nobody reads, so that one cluster barrier later each CTA holds the row's histogram.  The (bins,
+// peer) pairs are dealt out over the threads: a row's scores fall into few, neighbouring bins, and one thread
+// pushing its bins to all peers in turn took 1.2 us with two CTAs and 2.4 with eight; 0.7 and 1.3 this way.
+template <int NT>
+__device__ __forceinline__ void add_to_peers(const uint32_t* counts, uint32_t* merged, int n) {
+  const uint32_t C = cluster_size();
+  const int log2c = 31 - __clz(static_cast<int>(C));
+  const uint32_t at = dsmem_addr(smem_addr(merged), threadIdx.x & (C - 1u));
+#pragma unroll 4
+  for (int i = 4 * (static_cast<int>(threadIdx.x) >> log2c); i < n; i += 4 * (NT >> log2c)) {
+    const uint4 v = *reinterpret_cast<const uint4*>(counts + i);
+    if ((v.x | v.y | v.z | v.w) == 0u) continue;
+    const uint32_t to = at + 4u * static_cast<uint32_t>(i);
+    if (v.x != 0u) dsmem_red_add(to, v.x);
+    if (v.y != 0u) dsmem_red_add(to + 4u, v.y);
+    if (v.z != 0u) dsmem_red_add(to + 8u, v.z);
+    if (v.w != 0u) dsmem_red_add(to + 12u, v.w);
+  }
+}
 
 struct RowsShared {
   int warp_tot[3][32];
   int t, above, total;     // threshold digit, elements above it, elements at or above it
   int max_bin;             // largest bin at or above the threshold
   int count;               // survivors listed
+  int base;                // clusters: this CTA's first slot in the row's list
+  int reserved;            // clusters, first CTA: slots of the row's list given out
+  int gathered;            // clusters: survivors of all CTAs
   uint32_t value_bits;     // OR of the survivors' score bits
   uint32_t kmin, kmax;     // bounds of the survivors' keys (rebuilt bins only)
 };
@@ -225,8 +270,9 @@ struct RowGroup {
 // goes to the finish.
 __host__ __device__ constexpr int rows_level_bits(int l) { return l <= 2 ? 10 : l == 5 ? 10 : 11; }
 __host__ __device__ constexpr int rows_level_shift(int l) { return l == 0 ? 52 : l == 1 ? 42 : l == 2 ? 32 : l == 3 ? 21 : l == 4 ? 10 : 0; }
-template <typename T, int NT>
-__device__ __noinline__ uint64_t deeper_digits(const Chunk<T>& c, uint32_t* hist, int k, int cap, RowsShared& sh, int32_t* status) {
+template <typename T, int NT, bool CLUSTER>
+__device__ __noinline__ uint64_t deeper_digits(const Chunk<T>& c, uint32_t* hist, uint32_t* merged, int k, int cap,
+                                               RowsShared& sh, int32_t* status) {
   const int tid = threadIdx.x;
   uint64_t prefix = static_cast<uint64_t>(sh.t);
   int r = k - sh.above;
@@ -235,8 +281,12 @@ __device__ __noinline__ uint64_t deeper_digits(const Chunk<T>& c, uint32_t* hist
     const int bits = rows_level_bits(level), shift = rows_level_shift(level), above_shift = rows_level_shift(level - 1);
     const uint32_t mask = (1u << bits) - 1u;
     __syncthreads();
-    for (int i = tid; i < (1 << bits); i += NT) hist[i] = 0u;
+    for (int i = tid; i < (1 << bits); i += NT) {
+      hist[i] = 0u;
+      if (CLUSTER) merged[i] = 0u;
+    }
     __syncthreads();
+    if (CLUSTER) cluster_barrier();   // everyone's merged counts are clear
     const float vmin = prefilter_value(static_cast<uint32_t>((prefix << above_shift) >> 32));
     auto count_one = [&](float x, int pos) {
       const uint64_t comp = make_comp(fast_key(x), pos);
@@ -255,17 +305,22 @@ __device__ __noinline__ uint64_t deeper_digits(const Chunk<T>& c, uint32_t* hist
     const int pos = partial_element(c, x);
     if (pos >= 0) count_one(x, pos);
     __syncthreads();
+    if (CLUSTER) {
+      add_to_peers<NT>(hist, merged, 1 << bits);
+      cluster_barrier();
+    }
+    const uint32_t* counts = CLUSTER ? merged : hist;
     // the crossing: at most 2048 bins, a few consecutive ones per thread
     const int per = (1 << bits) > NT ? (1 << bits) / NT : 1;
     const int first = tid * per;
     int local = 0;
     if (first < (1 << bits))
-      for (int e = 0; e < per; ++e) local += static_cast<int>(hist[first + e]);
+      for (int e = 0; e < per; ++e) local += static_cast<int>(counts[first + e]);
     int total;
     int running = suffix_exclusive<NT>(local, sh.warp_tot[1], total);
     if (running < r && r <= running + local) {
       for (int e = per - 1; e >= 0; --e) {
-        const int n = static_cast<int>(hist[first + e]);
+        const int n = static_cast<int>(counts[first + e]);
         if (running < r && r <= running + n) {
           sh.t = first + e;
           sh.above = running;
@@ -347,6 +402,53 @@ __device__ __forceinline__ void collect_row(const Chunk<T>& c, const RowGroup<T,
   }
 }
 
+// Sweep 2 of a row in which few scores are hits: a warp's lanes store one hit each per round, for as many rounds as
+// one of them has hits among its 16 scores, reading the score again instead of going through the registers.
+template <typename T>
+__device__ __forceinline__ float score_at(const T* p) {
+  if constexpr (Elem<T>::kPerUnit == 4) return __ldg(p);
+  else return Elem<T>::from_bits16(__ldg(reinterpret_cast<const unsigned short*>(p)));
+}
+template <typename T, int NT, int CAP>
+__device__ __noinline__ void collect_row_sparse(const Chunk<T>& c, float vmin, RowList<CAP> list, RowsShared& sh) {
+  using Group = RowGroup<T, NT>;
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int u0 = c.fb; u0 < c.fe; u0 += Group::kStep) {
+    Group g;
+    g.load(c, u0);
+    const int pos0 = Group::position(c, u0);
+    uint32_t hits = 0u;
+    auto test = [&](float x, int e) {
+      if (!(x < vmin)) hits |= 1u << e;
+    };
+    if (u0 + Group::kStep <= c.fe) g.template each<true>(c, u0, test); else g.template each<false>(c, u0, test);
+    const int total = static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<uint32_t>(__popc(hits))));
+    if (total == 0) continue;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(&sh.count, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (base + total > CAP) continue;
+    for (uint32_t more = __ballot_sync(0xffffffffu, hits != 0u); more != 0u; more = __ballot_sync(0xffffffffu, hits != 0u)) {
+      if (hits != 0u) {
+        const int e = __ffs(static_cast<int>(hits)) - 1;
+        hits &= hits - 1u;
+        const int pos = pos0 + Group::distance(e);
+        list.put(base + __popc(more & ((1u << lane) - 1u)), score_at(c.abase + (pos + c.mis)), pos);
+      }
+      base += __popc(more);
+    }
+  }
+  if (c.head || c.tail) {   // (uniform)
+    float x = 0.f;
+    const int pos = partial_element(c, x);
+    if (pos >= 0 && !(x < vmin)) {
+      const int at = atomicAdd(&sh.count, 1);
+      if (at < CAP) list.put(at, x, pos);
+    }
+  }
+}
+
 template <typename T, int NT, int CAP>
 __device__ __noinline__ void collect_row_exact(const Chunk<T>& c, uint64_t floor_comp, RowList<CAP> list, RowsShared& sh) {
   collect_row<T, NT, CAP, true>(c, nullptr, prefilter_value(static_cast<uint32_t>(floor_comp >> 32)), floor_comp, list, sh);
@@ -382,8 +484,12 @@ __device__ __forceinline__ uint32_t expected_rank2(uint32_t packed, uint32_t dep
 }
 
 // PER: survivors a thread holds in the finish (the list takes PER * NT); CTAS: CTAs per SM it is compiled for.
-template <typename T, int NT, int PER, int CTAS, bool HINTS>
+// CLUSTER: a thread-block cluster per row.  Each CTA sweeps its share, its counts are added to every CTA's merged
+// histogram, all find the same cut, and their survivors meet in the first CTA, which finishes the row alone.
+// (Not with guesses: a single sweep leaves the finish, and that the clusters of ff_topk_kernel.cuh share out.)
+template <typename T, int NT, int PER, int CTAS, bool HINTS, bool CLUSTER>
 __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p) {
+  static_assert(!(HINTS && CLUSTER), "rows with guesses have one CTA");
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ RowsShared sh;
   using Group = RowGroup<T, NT>;
@@ -394,6 +500,9 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   const RowList<kCap> list = {reinterpret_cast<float*>(smem + kRowsBins * 4)};
   uint32_t* bins = reinterpret_cast<uint32_t*>(list.x);                      // 2 * kCap finish bins
   int32_t* ranked = reinterpret_cast<int32_t*>(list.x);                      // kCap positions
+  uint32_t* merged = CLUSTER ? reinterpret_cast<uint32_t*>(list.x + 2 * kCap) : hist;
+  const RowList<kCap> own_list = {CLUSTER ? reinterpret_cast<float*>(merged + kRowsBins) : list.x};
+  const uint32_t C = CLUSTER ? cluster_size() : 1u, rank = CLUSTER ? cluster_rank() : 0u;
   const int tid = threadIdx.x;
   auto clear_words = [&](uint32_t* a, int n) {
 #pragma unroll 4
@@ -401,7 +510,10 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   };
   // set-up that reads nothing of the kernels in front, behind which it may run
   clear_words(hist, kRowsBins);
+  if (CLUSTER) clear_words(merged, kRowsBins);
   if (tid == 0) {
+    sh.reserved = 0;
+    sh.gathered = 0;
     sh.t = 0;
     sh.above = 0;
     sh.total = 0;
@@ -415,7 +527,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   FF_TRACE(p, 0);
-  const int row = static_cast<int>(blockIdx.x);
+  const int row = static_cast<int>(CLUSTER ? blockIdx.x / C : blockIdx.x);
   const int k = p.k;
   const int rs = p.row_starts != nullptr ? p.row_starts[row] : 0;
   int64_t l = p.lengths[row];
@@ -461,6 +573,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     header = reinterpret_cast<uint32_t*>(p.handover + static_cast<int64_t>(row) * kHandoverRowBytes);
 
   if (len <= k) {   // nothing to select
+    if (CLUSTER && rank != 0u) return;
     if (HINTS && tid == 0) {
       if (header != nullptr) header[0] = header[1] = 0u;
       if (p.hint_out != nullptr) p.hint_out[row] = __uint_as_float(0x7fffffffu);
@@ -470,9 +583,11 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   }
 
   const T* rowp = reinterpret_cast<const T*>(p.scores) + static_cast<int64_t>(row) * p.row_stride + rs;
-  // the row in 16-byte units on absolute addresses, partial ones at its ends
+  // the row (or this CTA's share of it) in 16-byte units on absolute addresses, partial ones at the ends
   Chunk<T> chunk;
-  {
+  if (CLUSTER) {
+    chunk = make_chunk<T>(rowp, nullptr, len, static_cast<int>(C), static_cast<int>(rank), 0, 0);
+  } else {
     chunk.mis = static_cast<int>((reinterpret_cast<uintptr_t>(rowp) >> Elem<T>::kLog2Bytes) & (kPU - 1));
     chunk.abase = rowp - chunk.mis;
     chunk.len = len;
@@ -484,39 +599,77 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   }
   __syncthreads();   // set up
 
-  bool listed = false;          // the list holds survivors found with a guess
+  // Clusters: no access to a peer's shared memory before every CTA has started and set up its own.  Arrived at here,
+  // waited for behind the first sweep.
+  if (CLUSTER) cluster_arrive();
+  // After a sweep: how many survivors the row has.  Clusters: they are in the first CTA's list then (as far as
+  // they fit), and every CTA knows the number.
+  auto gather = [&]() -> int {
+    __syncthreads();
+    FF_TRACE(p, 3);
+    const int own = sh.count;
+    if constexpr (CLUSTER) {
+      if (tid == 0) sh.base = static_cast<int>(dsmem_atomic_add_u32(dsmem_addr(smem_addr(&sh.reserved), 0u), static_cast<uint32_t>(own)));
+      if (tid >= 32 && tid < 32 + static_cast<int>(C))
+        dsmem_red_add(dsmem_addr(smem_addr(&sh.gathered), static_cast<uint32_t>(tid - 32)), static_cast<uint32_t>(own));
+      __syncthreads();
+      const int base = sh.base;
+      const uint32_t to = dsmem_addr(smem_addr(list.x), 0u);
+      const uint64_t* from = reinterpret_cast<const uint64_t*>(own_list.x);
+      for (int i = tid; i < min(own, kCap - base); i += NT) dsmem_st_u64(to + 8u * static_cast<uint32_t>(base + i), from[i]);
+      cluster_barrier();
+      FF_TRACE(p, 4);
+      return sh.gathered;
+    }
+    return own;
+  };
+  auto discard = [&]() {   // the sweep did not fit: the lists are empty again
+    __syncthreads();
+    if (CLUSTER) cluster_barrier();   // everyone has read the number
+    if (tid == 0) {
+      sh.count = 0;
+      sh.reserved = 0;
+      sh.gathered = 0;
+    }
+    __syncthreads();
+    if (CLUSTER) cluster_barrier();
+  };
+
+  // Where so few scores are hits, going by hits instead of by scores is faster (1 x 128 Ki, one CTA: 23.8 -> 21.5 us; 64 x
+  // 128 Ki, k = 512, four CTAs a row: 21.4 -> 20.2), with four CTAs on an SM (256 threads) it is not.
+  const bool sparse = NT > 256 && len / k > (CLUSTER ? 128 : 48);
+  int n = 0;                    // survivors in the list
+  bool listed = false;          // ... found with a guess
   if constexpr (HINTS) {
     const float hint = p.hint_in != nullptr ? p.hint_in[row] : __uint_as_float(0x7fffffffu);
     const bool use = hint == hint;
     if (header != nullptr) {
-      const int n = static_cast<int>(__ldcg(header));
-      if (use && n >= k && n <= kCap) {
-        const unsigned long long* given = reinterpret_cast<const unsigned long long*>(header + 16);
+      const int given = static_cast<int>(__ldcg(header));
+      listed = use && given >= k && given <= kCap;
+      if (listed) {
+        const unsigned long long* from = reinterpret_cast<const unsigned long long*>(header + 16);
 #pragma unroll 4
-        for (int i = tid; i < n; i += NT) {
-          const uint64_t c = __ldcg(given + i);
+        for (int i = tid; i < given; i += NT) {
+          const uint64_t c = __ldcg(from + i);
           list.put(i, __uint_as_float(bits_of_key(comp_key(c))), comp_index(c));
         }
-        listed = true;
+        n = given;
       }
-      __syncthreads();
+      __syncthreads();   // every thread has read the count
       if (tid == 0) {
-        if (listed) sh.count = n;
-        else if (use && p.status != nullptr) atomicOr(p.status, 8);
+        if (!listed && use && p.status != nullptr) atomicOr(p.status, 8);
         header[0] = header[1] = 0u;   // empty for the producer's next launch
       }
     } else if (use) {
-      collect_row<T, NT, kCap, false>(chunk, nullptr, hint, 0ull, list, sh);
-      __syncthreads();
-      const int n = sh.count;
+      if (sparse) collect_row_sparse<T, NT, kCap>(chunk, hint, own_list, sh);
+      else collect_row<T, NT, kCap, false>(chunk, nullptr, hint, 0ull, own_list, sh);
+      n = gather();
       listed = n >= k && n <= kCap;
-      __syncthreads();
-      if (!listed && tid == 0) {
-        sh.count = 0;
-        if (p.status != nullptr) atomicOr(p.status, 8);
+      if (!listed) {
+        if (tid == 0 && p.status != nullptr) atomicOr(p.status, 8);
+        discard();
       }
     }
-    __syncthreads();
   }
 
   bool rebuild = listed;        // the packed bins do not fit the list: they are rebuilt from it
@@ -544,32 +697,37 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     }
     __syncthreads();
     FF_TRACE(p, 1);
+    if (CLUSTER) {
+      cluster_wait();
+      add_to_peers<NT>(hist, merged, kRowsBins);
+      FF_TRACE(p, 26);
+      cluster_barrier();
+      FF_TRACE(p, 27);
+    }
     // ---- threshold ----
-    pack_bins<NT>(hist, true, k, sh, sh.warp_tot[0]);
+    pack_bins<NT>(merged, true, k, sh, sh.warp_tot[0]);
     FF_TRACE(p, 2);
     // ---- sweep 2 ----
     const int above = sh.above, in_bin = sh.total - above;
     const uint32_t bin_key = static_cast<uint32_t>(sh.t) << kRowsShift;
     int keep, spread;
-    const uint32_t cut = bin_key + cut_in_digit(hist, sh.t, in_bin, k - above, kCap - above, keep, spread);
+    const uint32_t cut = bin_key + cut_in_digit(merged, sh.t, in_bin, k - above, kCap - above, keep, spread);
     bool exact = bin_key > 0xff800000u || sh.max_bin > kPackMax || keep < k - above ||
                  (sh.total > kCap && 8 * sh.max_bin > 7 * sh.total);
     if (!exact) {
-      collect_row<T, NT, kCap, false>(chunk, &first, prefilter_value(cut), 0ull, list, sh);
-      if (tid == 0) hist[rows_raw_of(sh.t)] = packed_bin(above, spread);   // (read in the finish)
-      __syncthreads();
-      const int n = sh.count;
+      if (sparse) collect_row_sparse<T, NT, kCap>(chunk, prefilter_value(cut), own_list, sh);
+      else collect_row<T, NT, kCap, false>(chunk, &first, prefilter_value(cut), 0ull, own_list, sh);
+      if (tid == 0) merged[rows_raw_of(sh.t)] = packed_bin(above, spread);   // (read in the finish)
+      n = gather();
       span = above + keep;
       if (n < k || n > kCap) {   // the interpolation was off
-        __syncthreads();
-        if (tid == 0) sh.count = 0;
-        __syncthreads();
+        discard();
         exact = n > kCap || sh.total > kCap;
         if (!exact) {
-          if (tid == 0) hist[rows_raw_of(sh.t)] = packed_bin(above, in_bin);
-          collect_row<T, NT, kCap, false>(chunk, &first, prefilter_value(bin_key), 0ull, list, sh);
+          if (tid == 0) merged[rows_raw_of(sh.t)] = packed_bin(above, in_bin);
+          collect_row<T, NT, kCap, false>(chunk, &first, prefilter_value(bin_key), 0ull, own_list, sh);
           span = sh.total;
-          __syncthreads();
+          n = gather();
         }
       }
       rebuild = 8 * sh.max_bin > 7 * sh.total;   // one digit holds nearly all: it says little about their ranks
@@ -577,13 +735,13 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     if (exact) {
       rebuild = true;
       const uint64_t floor_comp = sh.total <= kCap ? static_cast<uint64_t>(sh.t) << rows_level_shift(0)
-                                                   : deeper_digits<T, NT>(chunk, hist, k, kCap, sh, p.status);
-      collect_row_exact<T, NT, kCap>(chunk, floor_comp, list, sh);
-      __syncthreads();
+                                                   : deeper_digits<T, NT, CLUSTER>(chunk, hist, merged, k, kCap, sh, p.status);
+      collect_row_exact<T, NT, kCap>(chunk, floor_comp, own_list, sh);
+      n = gather();
     }
   }
-  FF_TRACE(p, 3);
-  const int n = min(sh.count, kCap);
+  if (CLUSTER && rank != 0u) return;   // nobody reads this CTA's shared memory any more
+  n = min(n, kCap);
   if (rebuild) span = n;
 
   // ---- finish ----
@@ -613,7 +771,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
         pos[j] = static_cast<int32_t>(entry.y);
         value_bits |= __float_as_uint(x);
         depth[j] = __float_as_uint(__fadd_rn(x, 0.0f));   // (-0.0 and NaN as in the keys)
-        if (!rebuild) where[j] = hist[depth[j] >> kRowsShift];
+        if (!rebuild) where[j] = merged[depth[j] >> kRowsShift];
       }
     });
     value_bits = __reduce_or_sync(0xffffffffu, value_bits);
@@ -625,7 +783,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   if (rebuild) {
     // digits of the survivors' own key range instead of the row's first digit
     uint32_t kmin = 0xffffffffu, kmax = 0u;
-    if (!listed) clear_words(hist, kRowsBins);
+    if (CLUSTER || !listed) clear_words(hist, kRowsBins);
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       if (pos[j] >= 0) {

@@ -51,12 +51,18 @@ def _check(oracle, s, lengths, k, rs=None, **kw):
 # 16 scores per thread and group: 4,096 with 256 threads (more rows than SMs), 16,384 with 1,024 (fewer rows)
 @pytest.mark.parametrize("B,L,k", [(20, 2049, 2048), (20, 16383, 2048), (20, 16385, 512), (20, 33000, 2048), (20, 70, 1),
                                    (160, 4095, 2048), (160, 4096, 1024), (160, 4097, 512), (160, 12289, 2048), (160, 70, 69),
-                                   (310, 9000, 2048), (300, 50001, 1024)])
+                                   (310, 9000, 2048), (300, 50001, 1024),
+                                   # clusters of four, eight and sixteen CTAs per row; rows too short for all of them to have a share
+                                   (3, 20481, 2048), (12, 40960, 2048), (12, 40961, 512), (11, 98305, 2048), (7, 131073, 1024),
+                                   (20, 33001, 2048), (30, 100003, 1), (40, 82001, 1024)])
 def test_rows_of_every_kind(oracle, B, L, k):
     g = torch.Generator().manual_seed(L + k)
     s = torch.stack([_row(i % KINDS, L, g) for i in range(B)])
     lengths = torch.full((B,), L, dtype=torch.int32)
-    lengths[KINDS:2 * KINDS] = torch.randint(1, L + 1, (KINDS,), generator=g, dtype=torch.int32)
+    some = lengths[KINDS:2 * KINDS] if B > KINDS else lengths[B - 1:]
+    some[:] = torch.randint(1, L + 1, some.shape, generator=g, dtype=torch.int32)
+    if B > 2:
+        lengths[2] = min(L, k + 3)                              # a few scores per CTA
     _check(oracle, s, lengths, k)
 
 

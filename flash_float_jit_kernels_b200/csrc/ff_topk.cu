@@ -125,6 +125,9 @@ void init_device(int device) {
   if (e == cudaSuccess) e = prepare_kernel(ff::topk_cluster_kernel<false, ff::kModePlain, __nv_bfloat16>);
   if (e == cudaSuccess) e = prepare_kernel(ff::topk_cluster_kernel<false, ff::kModeHinted, __nv_bfloat16>);
   if (e == cudaSuccess) e = prepare_kernel(ff::topk_cluster_kernel<false, ff::kModePlain, __half>);
+  if (e == cudaSuccess) e = prepare_kernel(ff::topk_cluster_kernel<false, ff::kModeHintedSplit>);
+  if (e == cudaSuccess) e = prepare_kernel(ff::topk_cluster_kernel<false, ff::kModeHintedSplit, __nv_bfloat16>);
+  if (e == cudaSuccess) e = prepare_kernel(ff::topk_cluster_kernel<false, ff::kModeHintedSplit, __half>);
   if (e == cudaSuccess) e = prepare_kernel(ff::topk_cluster_kernel<false, ff::kModeHinted, __half>);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(ff::cp_merge_sorted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -268,7 +271,12 @@ int launch(const ff::TopkParams& p, int cluster, cudaStream_t stream, int dtype 
   // ff_topk_set_self_seed(0) switch that off); the code lives in the instantiation with guesses.
   if (!HAS_MAP && groups > 1 && self_seed_enabled()) q.self_seed = 1;
   const bool hints = q.hint_in != nullptr || q.hint_out != nullptr || q.self_seed != 0;
-  if (!HAS_MAP && dtype == FF_DTYPE_BF16)
+  const bool split = groups > 1;
+  if (!HAS_MAP && dtype == FF_DTYPE_BF16 && hints && split)
+    e = cudaLaunchKernelEx(&cfg, ff::topk_cluster_kernel<false, ff::kModeHintedSplit, __nv_bfloat16>, q);
+  else if (!HAS_MAP && dtype == FF_DTYPE_F16 && hints && split)
+    e = cudaLaunchKernelEx(&cfg, ff::topk_cluster_kernel<false, ff::kModeHintedSplit, __half>, q);
+  else if (!HAS_MAP && dtype == FF_DTYPE_BF16)
     e = hints ? cudaLaunchKernelEx(&cfg, ff::topk_cluster_kernel<false, ff::kModeHinted, __nv_bfloat16>, q)
               : cudaLaunchKernelEx(&cfg, ff::topk_cluster_kernel<false, ff::kModePlain, __nv_bfloat16>, q);
   else if (!HAS_MAP && dtype == FF_DTYPE_F16)
@@ -280,6 +288,8 @@ int launch(const ff::TopkParams& p, int cluster, cudaStream_t stream, int dtype 
     e = cudaLaunchKernelEx(&cfg, ff::topk_cluster_kernel<false, ff::kModePushHinted>, q);
   else if (!HAS_MAP && q.push_world > 0)
     e = cudaLaunchKernelEx(&cfg, ff::topk_cluster_kernel<false, ff::kModePush>, q);
+  else if (!HAS_MAP && hints && split)
+    e = cudaLaunchKernelEx(&cfg, ff::topk_cluster_kernel<false, ff::kModeHintedSplit>, q);
   else if (!HAS_MAP && hints)
     e = cudaLaunchKernelEx(&cfg, ff::topk_cluster_kernel<false, ff::kModeHinted>, q);
   else

@@ -192,41 +192,66 @@ int choose_cluster(int device, int32_t B, int64_t L_width, int32_t k) {
   return c;
 }
 
-// Rows that are long and few are split over several clusters (groups) so that
-// all SMs sweep them; that needs the caller's zero-filled workspace and a
-// cooperative launch (all CTAs of a row wait for each other through global
-// memory).  Returns the number of clusters per row and may lower `cluster`.
-// Measured on B200 (B = 1, k = 2048, clusters of 8): with 15 or more clusters a split row beats one
-// cluster of 16 from 128 Ki columns up (15.9 against 16.2 us; 16.8 against 20.3 us at 512 Ki), and
-// with a threshold guess from 64 Ki up (10.1 against 12.5 us); with only 4 clusters it loses below
-// 768 Ki columns.  So shorter rows are split only if at least 8 clusters are free for each.
-constexpr int64_t kGroupMinWidth = 131072;
+// Rows that are long and few are split over several clusters (groups) so that all SMs sweep them; that needs the
+// caller's zero-filled workspace and a cooperative launch (all CTAs of a row wait for each other through
+// global memory).  Returns the number of clusters per row and may lower `cluster`.
+//
+// Clusters of two: 74 of them fit, on all 148 SMs (of eight only 15, on 120), and rows that need no histogram have no
+// use for wider ones (B = 1, 8 Mi columns 19.4 -> 18.6 us, B = 4, 1 Mi, k = 512 15.7 -> 14.7).
+//   * Rows with guesses, and rows that make their own, are swept once: split rows of 128 Ki columns take 13.1 us (B = 2),
+//     13.3 (B = 4), 13.7 (B = 8), k = 512 10.2 us, against 12.7 to 18.6 us in one cluster.  The own guess needs about 400
+//     hits in the CTAs' samples (seed_plan), so nine rows at most, and k of about 300.
+//   * From 32 Ki + 32 k columns up (2 x 98,304: 13.0 us against 12.9 to 13.8; k = 512, 2 x 65,536: 10.1 against 11.2).
+//   * Rows that have to be swept twice are split if very long, or if one row has the GPU.
+constexpr int64_t kGroupMinWidthSingle = 131072;
 constexpr int64_t kGroupMinWidthHinted = 65536;
 constexpr int64_t kGroupAlwaysWidth = 786432;
-constexpr int kGroupCluster = 8;
-int choose_groups(int device, int32_t B, int64_t L_width, size_t workspace_bytes, int* cluster, bool hinted = false) {
+// Whether a row of `len` scores makes its own guess on n_share CTAs (the kernel's seed_plan, roughly).
+bool own_guess_likely(int64_t len, int32_t k, int n_share, int per_unit) {
+  const double target = k + (k >> 2) + 64;
+  const int64_t sample = static_cast<int64_t>(n_share) * 2 * ff::kTileUnits * per_unit;
+  const double hits = sample < len ? target * static_cast<double>(sample) / static_cast<double>(len) : target;
+  return len >= 4 * target && hits >= 420.0 && 27 * n_share >= 420 && len / n_share >= 64 * per_unit;
+}
+// cp: a context-parallel rank's row, which keeps clusters of eight (its merge and the exchange of survivors are
+// laid out for at most 128 CTAs a row).
+int choose_groups(int device, int32_t B, int64_t L_width, int32_t k, size_t workspace_bytes, int* cluster, bool hinted,
+                  int per_unit = 4, bool cp = false) {
   int g = g_groups_override.load();
   if (g == 0) {
     const char* env = getenv("FF_TOPK_GROUPS");
     if (env != nullptr) g = atoi(env);
   }
   const size_t need = static_cast<size_t>(B) * ff::kWsRowWords * sizeof(uint32_t);
-  if (workspace_bytes < need || g == 1) return 1;
+  if (workspace_bytes < need || g == 1 || B < 1) return 1;
   int c = *cluster;
   const bool automatic = g == 0;
   if (automatic) {
-    if (L_width < (hinted ? kGroupMinWidthHinted : kGroupMinWidth) || g_cluster_override.load() != 0) return 1;
-    c = kGroupCluster;
-    g = 16;                                                     // more clusters than that bring nothing
-    const int64_t by_size = L_width / (static_cast<int64_t>(c) * 1024);   // at least 1 Ki columns per CTA
+    if (g_cluster_override.load() != 0) return 1;
+    c = cp ? 8 : 2;
+    const int log2c = cp ? 3 : 1;
+    g = g_active_clusters[device][log2c] / B;
+    if (cp && g > 16) g = 16;
+    const int64_t by_size = L_width / (static_cast<int64_t>(c) * (cp ? 1024 : 512));   // at least so many columns per CTA
     if (g > by_size) g = static_cast<int>(by_size);
+    bool worth = L_width >= kGroupAlwaysWidth;
+    if (cp) {
+      worth = worth || (L_width >= (hinted ? kGroupMinWidthHinted : kGroupMinWidthSingle) && g >= 8);
+    } else if (hinted) {
+      worth = worth || L_width >= 2 * kGroupMinWidthHinted ? g >= *cluster : L_width >= kGroupMinWidthHinted && B <= 4;
+    } else {
+      worth = worth || (self_seed_enabled() && L_width >= 32768 + 32 * static_cast<int64_t>(k) &&
+                        own_guess_likely(L_width, k, g * c, per_unit)) ||
+              (B == 1 && L_width >= kGroupMinWidthSingle);
+    }
+    if (!worth) return 1;
+  } else {
+    int log2c = 0;
+    while ((1 << log2c) < c) ++log2c;
+    const int room = g_active_clusters[device][log2c] / B;   // co-resident clusters per row
+    if (g > room) g = room;
+    if (g > 64) g = 64;
   }
-  int log2c = 0;
-  while ((1 << log2c) < c) ++log2c;
-  const int room = g_active_clusters[device][log2c] / (B > 0 ? B : 1);   // co-resident clusters per row
-  if (g > room) g = room;
-  if (automatic && L_width < kGroupAlwaysWidth && g < 8) return 1;
-  if (g > 64) g = 64;
   if (g < 2) return 1;
   *cluster = c;
   return g;
@@ -374,10 +399,11 @@ int launch_rows(const ff::TopkParams& p, int shape, cudaStream_t stream, int dty
 //   * more rows than SMs: four CTAs of 256 threads per SM (296 rows of 16 Ki: 14.6 us against 18.9 with one CTA of 1024),
 //     unless a second row per SM is all there is and the rows are long (296 rows of 64 Ki: 41 against 38);
 //   * one CTA of 1024 threads: 8.5 us for 4 Ki columns, 9.2 for 16 Ki, 11.4 for 32 Ki, 15.6 for 64 Ki, 23.6 for 128 Ki;
-//   * a cluster of 512-thread CTAs, four: 10.7 us for 32 Ki, 12.4 for 64 Ki, 15.3 for 128 Ki; eight: 11.2, 11.2, 12.9;
-//     sixteen: 12.5 for 128 Ki, 13.9 for 256 Ki, 16.2 for 512 Ki.  As many as the device holds with an SM for each CTA
-//     (two on an SM slow each other down: 32 rows of 64 Ki 13.8 us with four, 18.5 with eight), but four also for long
-//     rows of up to as many as fit two on an SM (64 ragged rows of 128 Ki: 20.8 us against 23.5 in clusters of two);
+//   * a cluster of 512-thread CTAs, four: 10.7 us for 32 Ki, 12.4 for 64 Ki, 15.3 for 128 Ki; eight: 11.2, 11.2, 12.9 (
+//     rows whose scores spread over many digits, as N(0, 1) does, 1 us more with eight and 6 us with sixteen, which are
+//     not used).  As many as the device holds with an SM for each CTA (two on an SM slow each other down: 32 rows of
+//     64 Ki 13.8 us with four, 18.5 with eight), but four also for long rows of up to as many as fit two on an SM
+//     (64 ragged rows of 128 Ki: 20.8 us against 23.5 in clusters of two of the other kernel);
 //   * ff_topk_kernel.cuh: 13.8 us for 64 Ki, 14.3 for 128 Ki, 15.0 for 256 Ki, 16.8 for 512 Ki (sixteen CTAs; 12.4, 12.5 and
 //     12.9 split over clusters), 24.7 for 64 rows of 128 Ki; with guesses it is the faster one from 48 Ki columns up.
 int choose_rows_shape(int device, int32_t B, int64_t L_width, bool hints, bool split) {
@@ -395,7 +421,7 @@ int choose_rows_shape(int device, int32_t B, int64_t L_width, bool hints, bool s
   if (L_width <= (B > one_per_sm[3] ? 32768 : 20480)) return 1024;
   if (L_width <= (B > one_per_sm[3] ? 131072 : 40960)) return -40512;
   if (B > one_per_sm[3]) return 0;
-  return L_width > 98304 && B <= one_per_sm[4] ? -160512 : -80512;
+  return -80512;
 }
 
 // Built-in scratch for ff_topk_launch_static: enough for FF_TOPK_STATIC_MAX_ROWS
@@ -483,7 +509,7 @@ int ff_topk_policy_launch_shape(int32_t B, int64_t L_width, int32_t k, int32_t h
   int cluster = choose_cluster(device, B, L_width, k);
   int groups = 1;
   if (has_workspace != 0)
-    groups = choose_groups(device, B, L_width, ff_topk_workspace_bytes(B, L_width, k), &cluster, hinted != 0);
+    groups = choose_groups(device, B, L_width, k, ff_topk_workspace_bytes(B, L_width, k), &cluster, hinted != 0);
   if (const int shape = choose_rows_shape(device, B, L_width, hinted != 0, groups > 1)) {
     cluster = shape_cluster(shape);
     groups = 1;
@@ -496,7 +522,7 @@ int ff_topk_policy_launch_shape(int32_t B, int64_t L_width, int32_t k, int32_t h
 size_t ff_topk_workspace_bytes(int32_t B, int64_t L_width, int32_t k) {
   (void)k;
   // Only rows split over several clusters use scratch: long rows, small batches.
-  if (B < 1 || B > 16 || (L_width < kGroupMinWidthHinted && g_groups_override.load() < 2)) return 0;
+  if (B < 1 || B > 16 || (L_width < 32768 && g_groups_override.load() < 2)) return 0;
   return static_cast<size_t>(B) * ff::kWsRowWords * sizeof(uint32_t);
 }
 
@@ -580,7 +606,7 @@ int transform_launch_impl(const void* scores_any, int dtype, int64_t row_stride,
   }
   int cluster = choose_cluster(device, B, L_width, k);
   if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
-    p.groups = choose_groups(device, B, L_width, workspace_bytes, &cluster, hint_in != nullptr);
+    p.groups = choose_groups(device, B, L_width, k, workspace_bytes, &cluster, hint_in != nullptr, dtype == FF_DTYPE_F32 ? 4 : 8);
     p.workspace = static_cast<uint32_t*>(workspace);
   }
   if (const int shape = choose_rows_shape(device, B, L_width, hint_in != nullptr || hint_out != nullptr, p.groups > 1))
@@ -673,7 +699,7 @@ int ff_topk_launch_static(const float* scores, int64_t row_stride, const int32_t
   p.epilogue = FF_EPILOGUE_INDEX;
   p.status = status;
   int cluster = choose_cluster(device, B, L_width, k);
-  p.groups = choose_groups(device, B, L_width, FF_TOPK_STATIC_MAX_ROWS * row_bytes, &cluster);
+  p.groups = choose_groups(device, B, L_width, k, FF_TOPK_STATIC_MAX_ROWS * row_bytes, &cluster, false);
   if (const int shape = choose_rows_shape(device, B, L_width, false, p.groups > 1))
     return launch_rows(p, shape, static_cast<cudaStream_t>(stream), FF_DTYPE_F32);
   p.workspace = scratch;
@@ -716,7 +742,7 @@ int ff_topk_cp_local(const float* scores, int64_t row_stride, const int32_t* len
   p.status = status;
   int cluster = choose_cluster(device, B, L_width, k);
   if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
-    p.groups = choose_groups(device, B, L_width, workspace_bytes, &cluster);
+    p.groups = choose_groups(device, B, L_width, k, workspace_bytes, &cluster, false, 4, true);
     p.workspace = static_cast<uint32_t*>(workspace);
   }
   return launch<false>(p, cluster, static_cast<cudaStream_t>(stream));
@@ -982,7 +1008,7 @@ int cp_fill_params(FfCpExchange* ex, const float* scores, int64_t row_stride, co
   p.hint_out = hint_out;
   int cluster = choose_cluster(device, ex->B, L_width, ex->k);
   if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
-    p.groups = choose_groups(device, ex->B, L_width, workspace_bytes, &cluster, hint_in != nullptr);
+    p.groups = choose_groups(device, ex->B, L_width, ex->k, workspace_bytes, &cluster, hint_in != nullptr, 4, true);
     p.workspace = static_cast<uint32_t*>(workspace);
   }
   *out = p;

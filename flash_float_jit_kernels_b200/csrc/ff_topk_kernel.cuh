@@ -980,10 +980,14 @@ __device__ __forceinline__ SeedPlan seed_plan(int len, int mis, int per_unit, in
     n0 = min(per, 2 * kTileUnits);
     rho = rho_of(n0);
   }
-  if (rho > 26.f) {
-    // more hits than the kept 32 can show: look at a part of the tile only (a multiple of the
-    // thread count, so that every thread reads the same number of units)
-    n0 = max(kThreads, (static_cast<int>(static_cast<float>(n0) * 24.f / rho) / kThreads) * kThreads);
+  if (rho > 28.f) {
+    // more hits than the kept 32 can show: look at as much of the tile as lets 27 of the threads' maxima reach the
+    // wanted score (fewer units than threads where one unit per thread would show more)
+    const float g = log1pf(-27.f / static_cast<float>(kThreads)) / log1pf(-sp.p);   // scores per thread
+    const int units = static_cast<int>(g >= static_cast<float>(per_unit)
+                                           ? g * static_cast<float>(kThreads / per_unit)
+                                           : 27.f / (1.f - __expf(static_cast<float>(per_unit) * log1pf(-sp.p))));
+    n0 = min(n0, max(units, 64));
     rho = rho_of(n0);
   }
   sp.n_use = n0;

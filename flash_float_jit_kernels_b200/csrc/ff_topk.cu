@@ -199,8 +199,8 @@ int choose_cluster(int device, int32_t B, int64_t L_width, int32_t k) {
 // Clusters of two: 74 of them fit, on all 148 SMs (of eight only 15, on 120), and rows that need no histogram have no
 // use for wider ones (B = 1, 8 Mi columns 19.4 -> 18.6 us, B = 4, 1 Mi, k = 512 15.7 -> 14.7).
 //   * Rows with guesses, and rows that make their own, are swept once: split rows of 128 Ki columns take 13.1 us (B = 2),
-//     13.3 (B = 4), 13.7 (B = 8), k = 512 10.2 us, against 12.7 to 18.6 us in one cluster.  The own guess needs about 400
-//     hits in the CTAs' samples (seed_plan), so nine rows at most, and k of about 300.
+//     13.3 (B = 4), 13.7 (B = 8), k = 512 10.2 us, against 12.7 to 18.6 us in one cluster.  The own guess needs about 200
+//     hits in the CTAs' samples (seed_plan), 27 of them from one CTA at most.
 //   * From 32 Ki + 32 k columns up (2 x 98,304: 13.0 us against 12.9 to 13.8; k = 512, 2 x 65,536: 10.1 against 11.2).
 //   * Rows that have to be swept twice are split if very long, or if one row has the GPU.
 constexpr int64_t kGroupMinWidthSingle = 131072;
@@ -211,7 +211,7 @@ bool own_guess_likely(int64_t len, int32_t k, int n_share, int per_unit) {
   const double target = k + (k >> 2) + 64;
   const int64_t sample = static_cast<int64_t>(n_share) * 2 * ff::kTileUnits * per_unit;
   const double hits = sample < len ? target * static_cast<double>(sample) / static_cast<double>(len) : target;
-  return len >= 4 * target && hits >= 420.0 && 27 * n_share >= 420 && len / n_share >= 64 * per_unit;
+  return len >= 6 * target && hits >= 210.0 && 27 * n_share >= 210 && len / n_share >= 64 * per_unit;
 }
 // cp: a context-parallel rank's row, which keeps clusters of eight (its merge and the exchange of survivors are
 // laid out for at most 128 CTAs a row).

@@ -958,8 +958,9 @@ __device__ __forceinline__ SeedPlan seed_plan(int len, int mis, int per_unit, in
   // hint_target_rank(k) for one rank.  Several ranks' guesses side by side: the list must hold k
   // entries not below the LARGEST guess, which sits a standard deviation or two above the rest, so
   // aim half-way between k and the list's capacity.
-  const int target = ranks > 1 ? min(k + (k >> 1), kSortCap - (kSortCap >> 3))
-                               : min(k + (k >> 2) + 64, kSortCap - (kSortCap >> 3));
+  // Few CTAs on the row give a noisier mean: aim a little higher, away from k.
+  const int target = min(ranks > 1 ? k + (k >> 1) : n_share < 16 ? k + (k >> 2) + (k >> 3) + 64 : k + (k >> 2) + 64,
+                         kSortCap - (kSortCap >> 3));
   if (len_for_p <= 0) len_for_p = len;
   sp.p = static_cast<float>(target) / static_cast<float>(len_for_p);
   sp.n_use = 0;
@@ -993,12 +994,13 @@ __device__ __forceinline__ SeedPlan seed_plan(int len, int mis, int per_unit, in
   sp.n_use = n0;
   // a usable order statistic inside the kept 32, and enough hits over the row for a steady mean
   // (relative noise of the row's survivor count about 1.25 / sqrt(hits): 6 % at 400 hits, against a
-  // window of -22 % .. +56 % around the target)
+  // window of -22 % .. +56 % around the target; 9 % at the 200 hits that fewer than sixteen CTAs give, against
+  // -29 % .. +42 %)
   // In a context-parallel step the `ranks` guesses are used side by side (every rank's own
   // for its own shard), so the row's count averages over all of them; a single rank's guess may be
   // noisier (it only shifts the largest guess, which the final check allows for).
   const float hits = rho * static_cast<float>(n_share);
-  sp.use = rho >= 3.f && rho <= 30.f && hits * static_cast<float>(ranks) >= 400.f && hits >= 100.f;
+  sp.use = rho >= 3.f && rho <= 30.f && hits * static_cast<float>(ranks) >= (ranks > 1 ? 400.f : 200.f) && hits >= 100.f;
   return sp;
 }
 

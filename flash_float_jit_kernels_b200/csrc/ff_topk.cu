@@ -198,10 +198,13 @@ int choose_cluster(int device, int32_t B, int64_t L_width, int32_t k) {
 //
 // Clusters of two: 74 of them fit, on all 148 SMs (of eight only 15, on 120), and rows that need no histogram have no
 // use for wider ones (B = 1, 8 Mi columns 19.4 -> 18.6 us, B = 4, 1 Mi, k = 512 15.7 -> 14.7).
-//   * Rows with guesses, and rows that make their own, are swept once: split rows of 128 Ki columns take 13.1 us (B = 2),
-//     13.3 (B = 4), 13.7 (B = 8), k = 512 10.2 us, against 12.7 to 18.6 us in one cluster.  The own guess needs about 200
-//     hits in the CTAs' samples (seed_plan), 27 of them from one CTA at most.
-//   * From 32 Ki + 32 k columns up (2 x 98,304: 13.0 us against 12.9 to 13.8; k = 512, 2 x 65,536: 10.1 against 11.2).
+//   * Rows that make their own guess are swept once: split rows of 256 Ki columns take 13.2 us (B = 2), 13.5 (B = 4), 14.1
+//     (B = 8), 16.2 (B = 16), against 15.7 to 22 in clusters of topk_rows_kernel.  The guess needs about 200 hits in the
+//     CTAs' samples (seed_plan), 27 of them from one CTA at most.
+//   * A cooperative launch that is not replayed from a graph starts on a 2.048 us beat behind the kernel in front of it
+//     (12.3, 14.3 or 16.4 us per call where a graph shows 10.2, 13.2 or 14.1), so shorter rows are not split although a
+//     graph would gain: from 128 Ki + 32 k columns up (4 x 256 Ki 16.3 against 15.8 to 17.3 us per call, 8 x 128 Ki
+//     16.4 against 13.2 to 14.2), and with guesses, which leave less to gain, only very long rows or a single row.
 //   * Rows that have to be swept twice are split if very long, or if one row has the GPU.
 constexpr int64_t kGroupMinWidthSingle = 131072;
 constexpr int64_t kGroupMinWidthHinted = 65536;
@@ -238,9 +241,9 @@ int choose_groups(int device, int32_t B, int64_t L_width, int32_t k, size_t work
     if (cp) {
       worth = worth || (L_width >= (hinted ? kGroupMinWidthHinted : kGroupMinWidthSingle) && g >= 8);
     } else if (hinted) {
-      worth = worth || L_width >= 2 * kGroupMinWidthHinted ? g >= *cluster : L_width >= kGroupMinWidthHinted && B <= 4;
+      worth = worth || (B == 1 && L_width >= kGroupMinWidthHinted) || (B > 4 && g >= *cluster && L_width >= 524288);
     } else {
-      worth = worth || (self_seed_enabled() && L_width >= 32768 + 32 * static_cast<int64_t>(k) &&
+      worth = worth || (self_seed_enabled() && L_width >= 131072 + 32 * static_cast<int64_t>(k) &&
                         own_guess_likely(L_width, k, g * c, per_unit)) ||
               (B == 1 && L_width >= kGroupMinWidthSingle);
     }
@@ -522,7 +525,7 @@ int ff_topk_policy_launch_shape(int32_t B, int64_t L_width, int32_t k, int32_t h
 size_t ff_topk_workspace_bytes(int32_t B, int64_t L_width, int32_t k) {
   (void)k;
   // Only rows split over several clusters use scratch: long rows, small batches.
-  if (B < 1 || B > 16 || (L_width < 32768 && g_groups_override.load() < 2)) return 0;
+  if (B < 1 || B > 16 || (L_width < kGroupMinWidthHinted && g_groups_override.load() < 2)) return 0;
   return static_cast<size_t>(B) * ff::kWsRowWords * sizeof(uint32_t);
 }
 

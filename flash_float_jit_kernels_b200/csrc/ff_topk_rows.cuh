@@ -157,6 +157,13 @@ __device__ __forceinline__ uint32_t packed_bin(int above, int count) {
   return (static_cast<uint32_t>(above) << (kPackShift + 1)) | static_cast<uint32_t>(2 * min(count, kPackMax));
 }
 
+// The cut is an estimate: correctly rounded roots and quotients, which every thread of the CTA would go through, cost 0.1 to
+// 0.2 us of a single row's 7.7 to 9.6 and 1 % of a batch.
+__device__ __forceinline__ float approximate_sqrt(float x) {
+  const float y = fmaxf(x, 1e-6f);
+  return y * rsqrtf(y);
+}
+
 // Where to cut inside the threshold digit so that a few more than the `wanted` largest of its `in_bin` scores are
 // kept: the density of scores is taken as linear over the digit, from its own count and the next
 // digit's (c0, c1): above a point x of the way down lie (c0 + c1) / 2 x + (c0 - c1) / 2 x^2 of them,
@@ -166,7 +173,7 @@ __device__ __forceinline__ uint32_t packed_bin(int above, int count) {
 // would have at the kept part's density, which is what the finish interpolates with.
 __device__ __forceinline__ uint32_t cut_in_digit(const uint32_t* packed, int t, int in_bin, int wanted, int room, int& keep, int& spread) {
   const float c0 = static_cast<float>(in_bin);
-  const int margin = (in_bin >> 4) + static_cast<int>(2.f * sqrtf(c0)) + 8;
+  const int margin = (in_bin >> 4) + static_cast<int>(2.f * approximate_sqrt(c0)) + 8;
   keep = min(in_bin, wanted + margin);
   if (keep > room) keep = room >= wanted + (margin >> 1) ? room : -1;
   const int up = t + 1;
@@ -174,9 +181,9 @@ __device__ __forceinline__ uint32_t cut_in_digit(const uint32_t* packed, int t, 
   if ((up & 7) == 0) c1 *= up >= kRowsBins / 2 ? 0.5f : 2.f;   // the next digit spans a step of another width
   c1 = fminf(c1, 3.f * c0);
   const float b = 0.5f * (c0 + c1), a = 0.5f * (c0 - c1), want = static_cast<float>(keep);
-  const float x = 2.f * want / (b + sqrtf(fmaxf(b * b + 4.f * a * want, 0.f)));
+  const float x = __fdividef(2.f * want, b + approximate_sqrt(b * b + 4.f * a * want));
   const bool all = keep >= in_bin || !(x < 1.f);
-  spread = all ? in_bin : static_cast<int>(fminf(want / x, static_cast<float>(kPackMax)));
+  spread = all ? in_bin : static_cast<int>(fminf(__fdividef(want, x), static_cast<float>(kPackMax)));
   return all ? 0u : static_cast<uint32_t>((1.f - x) * static_cast<float>(1 << kRowsShift));
 }
 

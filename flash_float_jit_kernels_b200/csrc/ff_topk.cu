@@ -402,9 +402,9 @@ int launch_rows(const ff::TopkParams& p, int shape, cudaStream_t stream, int dty
 //   * more rows than SMs: four CTAs of 256 threads per SM (296 rows of 16 Ki: 14.6 us against 18.9 with one CTA of 1024),
 //     unless a second row per SM is all there is and the rows are long (296 rows of 64 Ki: 41 against 38);
 //   * one CTA of 1024 threads: 8.5 us for 4 Ki columns, 9.2 for 16 Ki, 11.4 for 32 Ki, 15.6 for 64 Ki, 23.6 for 128 Ki;
-//   * a cluster of 512-thread CTAs, four: 10.7 us for 32 Ki, 12.4 for 64 Ki, 15.3 for 128 Ki; eight: 11.2, 11.2, 12.9 (
-//     rows whose scores spread over many digits, as N(0, 1) does, 1 us more with eight and 6 us with sixteen, which are
-//     not used).  As many as the device holds with an SM for each CTA (two on an SM slow each other down: 32 rows of
+//   * a cluster of 512-thread CTAs, four: 10.7 us for 32 Ki, 12.4 for 64 Ki, 15.3 for 128 Ki; eight: 11.2, 11.2, 12.9.
+//     Scores that spread over many digits, as N(0, 1) does, take 1 us more with eight and 6 us more with sixteen, which
+//     are not used.  As many as the device holds with an SM for each CTA (two on an SM slow each other down: 32 rows of
 //     64 Ki 13.8 us with four, 18.5 with eight), but four also for long rows of up to as many as fit two on an SM
 //     (64 ragged rows of 128 Ki: 20.8 us against 23.5 in clusters of two of the other kernel);
 //   * ff_topk_kernel.cuh: 13.8 us for 64 Ki, 14.3 for 128 Ki, 15.0 for 256 Ki, 16.8 for 512 Ki (sixteen CTAs; 12.4, 12.5 and

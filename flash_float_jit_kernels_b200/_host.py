@@ -55,6 +55,11 @@ def transform():
 
 
 @functools.lru_cache(maxsize=None)
+def scratch():
+    return load().scratch
+
+
+@functools.lru_cache(maxsize=None)
 def logits():
     from .indexer_logits import load as load_indexer
     module = load()

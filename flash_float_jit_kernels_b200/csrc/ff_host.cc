@@ -12,7 +12,9 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
@@ -20,7 +22,9 @@
 
 #include <limits>
 #include <map>
+#include <mutex>
 #include <utility>
+#include <vector>
 
 #include "../../include/ff_indexer_logits.h"
 #include "../../include/ff_topk.h"
@@ -53,32 +57,93 @@ inline const Tensor* vector_of(PyObject* o, int64_t n, at::ScalarType type, c10:
   return t;
 }
 
+// ---- zero-filled scratch of split rows ----
+// The kernels leave it zeroed, and no two launches that may overlap on the GPU share it:
+//   * a call in plain stream order takes the buffer of its (device, stream), grown on demand; the number of streams
+//     bounds the map, and a buffer that was replaced is reused in stream order;
+//   * a call under stream capture takes a buffer of its (capture, stream), filled at once on a stream of its own, because
+//     a fill that were only recorded would not have run for another graph or an eager call, and owned by the graph,
+//     because graphs captured one after the other on one stream may be replayed side by side on two.
+std::mutex g_returned_mutex;
+std::vector<Tensor*>& g_returned = *new std::vector<Tensor*>();   // of destroyed graphs, given back by the next call
+
+// Called by the CUDA runtime when the last graph that holds the buffer is gone (no CUDA call is allowed here).
+void CUDART_CB return_scratch(void* t) {
+  const std::lock_guard<std::mutex> lock(g_returned_mutex);
+  g_returned.push_back(static_cast<Tensor*>(t));
+}
+
+Tensor zeroed(int64_t bytes, c10::Device dev, cudaStream_t stream) {
+  Tensor t = at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(dev));
+  C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, static_cast<size_t>(bytes), stream));
+  return t;
+}
+
+// A buffer that is zero when this returns and belongs to no capture, whatever the calling thread is capturing.
+Tensor zeroed_outside_capture(int64_t bytes, c10::Device dev) {
+  const c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);
+  static auto& streams = *new std::map<int, cudaStream_t>();   // one per device; guarded by the GIL
+  cudaStream_t& side = streams[dev.index()];
+  if (side == nullptr) C10_CUDA_CHECK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+  const c10::cuda::CUDAStreamGuard guard(c10::cuda::getStreamFromExternal(side, dev.index()));
+  Tensor t = zeroed(bytes, dev, side);
+  C10_CUDA_CHECK(cudaStreamSynchronize(side));
+  return t;
+}
+
+// `dev` is the current device.
+Tensor scratch_for(c10::Device dev, cudaStream_t stream, int64_t need) {
+  {
+    std::vector<Tensor*> returned;
+    {
+      const std::lock_guard<std::mutex> lock(g_returned_mutex);
+      returned.swap(g_returned);
+    }
+    for (Tensor* t : returned) delete t;
+  }
+  const std::pair<int, cudaStream_t> key{dev.index(), stream};
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo(stream, &status, &id, &graph) != cudaSuccess) {
+    (void)cudaGetLastError();   // (the legacy stream beside a capture on a blocking one: the launch will say so)
+    status = cudaStreamCaptureStatusNone;
+  }
+  if (status == cudaStreamCaptureStatusActive) {
+    struct Captured {
+      unsigned long long id = 0;    // ids are not used twice
+      Tensor* scratch = nullptr;    // the graph's: valid while `id` is being captured
+    };
+    static auto& captured = *new std::map<std::pair<int, cudaStream_t>, Captured>();   // guarded by the GIL
+    Captured& c = captured[key];
+    if (c.scratch != nullptr && c.id == id && c.scratch->numel() >= need) return *c.scratch;
+    Tensor* owned = new Tensor(zeroed_outside_capture(need, dev));
+    cudaUserObject_t object;
+    const cudaError_t e = cudaUserObjectCreate(&object, owned, return_scratch, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) delete owned;
+    C10_CUDA_CHECK(e);
+    C10_CUDA_CHECK(cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove));
+    c = {id, owned};
+    return *owned;
+  }
+  static auto& kept = *new std::map<std::pair<int, cudaStream_t>, Tensor>();   // guarded by the GIL
+  Tensor& t = kept[key];
+  if (!t.defined() || t.numel() < need) t = zeroed(need, dev, stream);
+  return t;
+}
+
 struct Workspace {
   void* ptr = nullptr;
   size_t bytes = 0;
   Tensor keep;   // holds the memory while the launch is enqueued without the GIL
 };
 
-// Zero-filled scratch of split rows, one per (device, stream), made once at the size the largest batch
-// that uses scratch needs (about 4 MB) and never replaced: a captured graph may hold its address.
-// The number of streams a process uses bounds the map.
-bool workspace_for(c10::Device dev, cudaStream_t stream, int64_t B, int64_t L, int64_t k, Workspace& ws) {
+void workspace_for(c10::Device dev, cudaStream_t stream, int64_t B, int64_t L, int64_t k, Workspace& ws) {
   const size_t need = p_workspace_bytes(static_cast<int32_t>(B), L, static_cast<int32_t>(k));
-  if (need == 0) return true;
-  static auto& kept = *new std::map<std::pair<int, cudaStream_t>, Tensor>();   // guarded by the GIL
-  Tensor& t = kept[{dev.index(), stream}];
-  if (!t.defined() || static_cast<size_t>(t.numel()) < need) {
-    size_t bytes = need;
-    for (int b = 1; b <= 64; ++b) {
-      const size_t n = p_workspace_bytes(b, std::numeric_limits<int32_t>::max(), 1);
-      if (n > bytes) bytes = n;
-    }
-    t = at::zeros({static_cast<int64_t>(bytes)}, at::TensorOptions().dtype(at::kByte).device(dev));
-  }
-  ws.ptr = t.data_ptr();
-  ws.bytes = static_cast<size_t>(t.numel());
-  ws.keep = t;
-  return true;
+  if (need == 0) return;
+  ws.keep = scratch_for(dev, stream, static_cast<int64_t>(need));
+  ws.ptr = ws.keep.data_ptr();
+  ws.bytes = static_cast<size_t>(ws.keep.numel());
 }
 
 PyObject* report(int rc, const char* what) {
@@ -349,6 +414,23 @@ PyObject* py_logits(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
 }
 
+// scratch(device index, bytes): zero-filled scratch for a launch on the device's current stream
+PyObject* py_scratch(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  int64_t device, bytes;
+  if (n != 2 || !take_k(a[0], device) || !take_k(a[1], bytes) || device < 0 || device > 127 || bytes < 1) {
+    PyErr_SetString(PyExc_TypeError, "scratch(device index, bytes)");
+    return nullptr;
+  }
+  try {
+    const c10::Device dev(c10::kCUDA, static_cast<c10::DeviceIndex>(device));
+    const c10::cuda::OptionalCUDAGuard guard(dev);
+    return THPVariable_Wrap(scratch_for(dev, c10::cuda::getCurrentCUDAStream(dev.index()).stream(), bytes));
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
 // bind(name, address): the C ABI functions of the loaded libraries; bind("on_error", callable)
 PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 2 || !PyUnicode_Check(a[0])) {
@@ -380,6 +462,7 @@ PyObject* py_bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 PyMethodDef kMethods[] = {
     {"bind", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_bind)), METH_FASTCALL, nullptr},
+    {"scratch", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_scratch)), METH_FASTCALL, nullptr},
     {"topk", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_topk)), METH_FASTCALL, nullptr},
     {"transform", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_transform)), METH_FASTCALL, nullptr},
     {"logits", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_logits)), METH_FASTCALL, nullptr},

@@ -32,9 +32,6 @@ class TopkArgumentError(AssertionError, ValueError):
     """
 
 
-_WORKSPACES: dict = {}
-
-
 def _require(cond: bool, msg: str) -> None:
     if not cond:
         raise TopkArgumentError(msg)
@@ -48,16 +45,12 @@ def _stream_ptr(device: torch.device):
     return torch.cuda.current_stream(device).cuda_stream
 
 
-def _workspace(lib, device: torch.device, B: int, L: int, k: int, stream: Optional[int] = None):
-    """Per-(device, stream) scratch, grown on demand and zero-filled once."""
+def _workspace(lib, device: torch.device, B: int, L: int, k: int):
+    """Zero-filled scratch for a launch on the device's current stream; under stream capture the graph owns it."""
     need = int(lib.ff_topk_workspace_bytes(B, L, k))
     if need == 0:
         return None, 0
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream if stream is None else stream)
-    ws = _WORKSPACES.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(need, dtype=torch.uint8, device=device)
-        _WORKSPACES[key] = ws
+    ws = _host.scratch()(torch.cuda.current_device() if device.index is None else device.index, need)
     return ws, ws.numel()
 
 
@@ -149,7 +142,7 @@ def fast_topk_v3(
         return out
     dev = score.device
     stream = torch.cuda.current_stream(dev).cuda_stream
-    ws, ws_bytes = _workspace(lib, dev, B, L, topk, stream)
+    ws, ws_bytes = _workspace(lib, dev, B, L, topk)
     row_stride = score.stride(0) if B > 1 else max(score.stride(0), L)
     if threshold_hint is not None:
         _require(threshold_hint.shape == (B,) and threshold_hint.dtype == torch.float32

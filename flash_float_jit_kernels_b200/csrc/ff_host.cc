@@ -7,7 +7,8 @@
 //
 // Every function returns None when an argument is not of the plain, valid kind it handles; the Python
 // layer then runs the full checks, which raise the documented errors (or handle the rare kinds,
-// such as tensor subclasses).  The C ABI functions are bound by address (bind()), so that this module
+// such as tensor subclasses).  C++ exceptions leave as the Python ones torch maps them to (an allocation that does
+// not fit is torch.OutOfMemoryError).  The C ABI functions are bound by address (bind()), so that this module
 // uses the very library instance ctypes has loaded, whatever its build knobs.
 #include <Python.h>
 
@@ -18,6 +19,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <limits>
@@ -279,66 +281,60 @@ bool take_k(PyObject* o, int64_t& k) {
 PyObject* py_topk(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int64_t k;
   if (n != 9 || !take_k(a[2], k)) Py_RETURN_NONE;
-  try {
-    return select(a[0], a[1], k, a[3], a[4], a[5], a[6], a[7], a[8], "fast_topk_v3");
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  HANDLE_TH_ERRORS
+  return select(a[0], a[1], k, a[3], a[4], a[5], a[6], a[7], a[8], "fast_topk_v3");
+  END_HANDLE_TH_ERRORS
 }
 
 // transform(score, lengths, out, row_starts, table, cu_seqlens, offset): table and cu_seqlens for the
 // page-table gather, offset for the per-row offset; True when launched
 PyObject* py_transform(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 7) Py_RETURN_NONE;
-  try {
-    const Tensor* out = cuda_tensor(a[2]);
-    if (out == nullptr || out->dim() != 2 || !out->is_contiguous() || out->scalar_type() != at::kInt) Py_RETURN_NONE;
-    const int64_t k = out->size(1);
-    Scores s;
-    if (!take_scores(a[0], a[1], a[3], k, s) || s.score->scalar_type() != at::kFloat || out->size(0) != s.B) Py_RETURN_NONE;
-    const c10::Device dev = s.score->device();
-    if (out->device() != dev) Py_RETURN_NONE;
-    const bool pages = !is_none(a[4]);
-    const int32_t *table = nullptr, *cu = nullptr, *offsets = nullptr;
-    int64_t table_stride = 0, requests = 0;
-    if (pages) {
-      const Tensor* t = cuda_tensor(a[4]);
-      const Tensor* c = cuda_tensor(a[5]);
-      if (t == nullptr || c == nullptr || t->dim() != 2 || t->scalar_type() != at::kInt || t->stride(1) != 1 ||
-          t->device() != dev || c->dim() != 1)
-        Py_RETURN_NONE;
-      requests = c->size(0) - 1;
-      if (vector_of(a[5], requests + 1, at::kInt, dev) == nullptr || t->size(0) != requests || requests > s.B || requests < 1)
-        Py_RETURN_NONE;
-      table = static_cast<const int32_t*>(t->data_ptr());
-      table_stride = t->stride(0);
-      if (!(s.row_starts == nullptr && requests == s.B)) cu = static_cast<const int32_t*>(c->data_ptr());
-    } else {
-      const Tensor* o = vector_of(a[6], s.B, at::kInt, dev);
-      if (o == nullptr) Py_RETURN_NONE;
-      offsets = static_cast<const int32_t*>(o->data_ptr());
-    }
-    const c10::cuda::OptionalCUDAGuard guard(dev);
-    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    Workspace ws;
-    workspace_for(dev, stream, s.B, s.L, k, ws);
-    const float* scores = static_cast<const float*>(s.score->data_ptr());
-    const int32_t* lengths = static_cast<const int32_t*>(s.lengths->data_ptr());
-    const int32_t* row_starts = s.row_starts == nullptr ? nullptr : static_cast<const int32_t*>(s.row_starts->data_ptr());
-    int32_t* out_ptr = static_cast<int32_t*>(out->data_ptr());
-    const int rc = without_gil([&] {
-      return p_transform(scores, s.row_stride, lengths, row_starts, out_ptr, static_cast<int32_t>(s.B), s.L,
-                         static_cast<int32_t>(k), pages ? FF_EPILOGUE_PAGE_TABLE : FF_EPILOGUE_ADD_OFFSET, table,
-                         table_stride, cu, static_cast<int32_t>(pages ? requests : 0), offsets, ws.ptr, ws.bytes, nullptr,
-                         stream);
-    });
-    if (rc != 0) return report(rc, pages ? "fast_topk_transform_fused" : "fast_topk_transform_ragged_fused");
-    Py_RETURN_TRUE;
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
+  HANDLE_TH_ERRORS
+  const Tensor* out = cuda_tensor(a[2]);
+  if (out == nullptr || out->dim() != 2 || !out->is_contiguous() || out->scalar_type() != at::kInt) Py_RETURN_NONE;
+  const int64_t k = out->size(1);
+  Scores s;
+  if (!take_scores(a[0], a[1], a[3], k, s) || s.score->scalar_type() != at::kFloat || out->size(0) != s.B) Py_RETURN_NONE;
+  const c10::Device dev = s.score->device();
+  if (out->device() != dev) Py_RETURN_NONE;
+  const bool pages = !is_none(a[4]);
+  const int32_t *table = nullptr, *cu = nullptr, *offsets = nullptr;
+  int64_t table_stride = 0, requests = 0;
+  if (pages) {
+    const Tensor* t = cuda_tensor(a[4]);
+    const Tensor* c = cuda_tensor(a[5]);
+    if (t == nullptr || c == nullptr || t->dim() != 2 || t->scalar_type() != at::kInt || t->stride(1) != 1 ||
+        t->device() != dev || c->dim() != 1)
+      Py_RETURN_NONE;
+    requests = c->size(0) - 1;
+    if (vector_of(a[5], requests + 1, at::kInt, dev) == nullptr || t->size(0) != requests || requests > s.B || requests < 1)
+      Py_RETURN_NONE;
+    table = static_cast<const int32_t*>(t->data_ptr());
+    table_stride = t->stride(0);
+    if (!(s.row_starts == nullptr && requests == s.B)) cu = static_cast<const int32_t*>(c->data_ptr());
+  } else {
+    const Tensor* o = vector_of(a[6], s.B, at::kInt, dev);
+    if (o == nullptr) Py_RETURN_NONE;
+    offsets = static_cast<const int32_t*>(o->data_ptr());
   }
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  Workspace ws;
+  workspace_for(dev, stream, s.B, s.L, k, ws);
+  const float* scores = static_cast<const float*>(s.score->data_ptr());
+  const int32_t* lengths = static_cast<const int32_t*>(s.lengths->data_ptr());
+  const int32_t* row_starts = s.row_starts == nullptr ? nullptr : static_cast<const int32_t*>(s.row_starts->data_ptr());
+  int32_t* out_ptr = static_cast<int32_t*>(out->data_ptr());
+  const int rc = without_gil([&] {
+    return p_transform(scores, s.row_stride, lengths, row_starts, out_ptr, static_cast<int32_t>(s.B), s.L,
+                       static_cast<int32_t>(k), pages ? FF_EPILOGUE_PAGE_TABLE : FF_EPILOGUE_ADD_OFFSET, table,
+                       table_stride, cu, static_cast<int32_t>(pages ? requests : 0), offsets, ws.ptr, ws.bytes, nullptr,
+                       stream);
+  });
+  if (rc != 0) return report(rc, pages ? "fast_topk_transform_fused" : "fast_topk_transform_ragged_fused");
+  Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
 }
 
 // The logits launch; returns a new reference like select().
@@ -406,12 +402,9 @@ PyObject* logits(PyObject* py_q, PyObject* py_k, PyObject* py_w, PyObject* py_le
 PyObject* py_logits(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int64_t ctas;
   if (n != 9 || !take_k(a[6], ctas) || ctas > 65535 || ctas < -65535) Py_RETURN_NONE;
-  try {
-    return logits(a[0], a[1], a[2], a[3], a[4], a[5], ctas, a[7], a[8]);
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  HANDLE_TH_ERRORS
+  return logits(a[0], a[1], a[2], a[3], a[4], a[5], ctas, a[7], a[8]);
+  END_HANDLE_TH_ERRORS
 }
 
 // scratch(device index, bytes): zero-filled scratch for a launch on the device's current stream
@@ -421,14 +414,11 @@ PyObject* py_scratch(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyErr_SetString(PyExc_TypeError, "scratch(device index, bytes)");
     return nullptr;
   }
-  try {
-    const c10::Device dev(c10::kCUDA, static_cast<c10::DeviceIndex>(device));
-    const c10::cuda::OptionalCUDAGuard guard(dev);
-    return THPVariable_Wrap(scratch_for(dev, c10::cuda::getCurrentCUDAStream(dev.index()).stream(), bytes));
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-    return nullptr;
-  }
+  HANDLE_TH_ERRORS
+  const c10::Device dev(c10::kCUDA, static_cast<c10::DeviceIndex>(device));
+  const c10::cuda::OptionalCUDAGuard guard(dev);
+  return THPVariable_Wrap(scratch_for(dev, c10::cuda::getCurrentCUDAStream(dev.index()).stream(), bytes));
+  END_HANDLE_TH_ERRORS
 }
 
 // bind(name, address): the C ABI functions of the loaded libraries; bind("on_error", callable)

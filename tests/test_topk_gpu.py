@@ -396,3 +396,21 @@ def test_threshold_hint_edge_shapes(oracle, k):
         torch.cuda.synchronize()
         exp = oracle.topk_c(s.numpy(), lengths.numpy(), k, starts.numpy())
         assert np.array_equal(out.cpu().numpy(), exp), step
+
+
+@pytest.mark.gpu
+def test_a_result_that_does_not_fit_is_an_out_of_memory_error():
+    """The allocation inside the operator fails as torch's own do, so that callers that free caches and retry on
+    ``torch.OutOfMemoryError`` still can."""
+    import flash_float_jit_kernels_b200 as pkg
+    dev = torch.device("cuda:0")
+    s = torch.randn((200_000, 8), device=dev)
+    lengths = torch.full((200_000,), 8, dtype=torch.int32, device=dev)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    try:
+        torch.cuda.set_per_process_memory_fraction(0.01)     # 1.8 GB; the result would take 3.3 GB
+        with pytest.raises(torch.OutOfMemoryError):
+            pkg.fast_topk_v3(s, lengths, 2048, index_dtype=torch.int64)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)

@@ -166,16 +166,23 @@ int ensure_init(int* device_out) {
 }
 
 
+// Launch shapes forced by a call or, where no call did, by the environment; 0: chosen here.
+int forced_shape(const std::atomic<int>& override_, const char* variable) {
+  const int n = override_.load();
+  if (n != 0) return n;
+  const char* env = getenv(variable);
+  return env != nullptr ? atoi(env) : 0;
+}
+int forced_cluster() { return forced_shape(g_cluster_override, "FF_TOPK_CLUSTER"); }
+int forced_groups() { return forced_shape(g_groups_override, "FF_TOPK_GROUPS"); }
+
+
 // Cluster size per row.  One CTA sweeps about 16 Ki scores; the cluster grows
 // with the row up to the largest size the device can schedule, but not beyond
 // what lets every row of the batch run at the same time.
 int choose_cluster(int device, int32_t B, int64_t L_width, int32_t k) {
   (void)k;
-  int c = g_cluster_override.load();
-  if (c == 0) {
-    const char* env = getenv("FF_TOPK_CLUSTER");
-    if (env != nullptr) c = atoi(env);
-  }
+  int c = forced_cluster();
   if (c == 0) {
     // Measured on B200: the widest cluster is fastest at every row length down
     // to 4 Ki (the finish is shared out over the cluster), so take the largest
@@ -220,11 +227,7 @@ bool own_guess_likely(int64_t len, int32_t k, int n_share, int per_unit) {
 // laid out for at most 128 CTAs a row).
 int choose_groups(int device, int32_t B, int64_t L_width, int32_t k, size_t workspace_bytes, int* cluster, bool hinted,
                   int per_unit = 4, bool cp = false) {
-  int g = g_groups_override.load();
-  if (g == 0) {
-    const char* env = getenv("FF_TOPK_GROUPS");
-    if (env != nullptr) g = atoi(env);
-  }
+  int g = forced_groups();
   const size_t need = static_cast<size_t>(B) * ff::kWsRowWords * sizeof(uint32_t);
   if (workspace_bytes < need || g == 1 || B < 1) return 1;
   int c = *cluster;
@@ -410,7 +413,7 @@ int launch_rows(const ff::TopkParams& p, int shape, cudaStream_t stream, int dty
 //   * ff_topk_kernel.cuh: 13.8 us for 64 Ki, 14.3 for 128 Ki, 15.0 for 256 Ki, 16.8 for 512 Ki (sixteen CTAs; 12.4, 12.5 and
 //     12.9 split over clusters), 24.7 for 64 rows of 128 Ki; with guesses it is the faster one from 48 Ki columns up.
 int choose_rows_shape(int device, int32_t B, int64_t L_width, bool hints, bool split) {
-  if (g_cluster_override.load() != 0 || g_groups_override.load() != 0) return 0;
+  if (forced_cluster() != 0 || forced_groups() != 0) return 0;
   const int sms = g_sm_count[device];
   if (B > sms) return B <= 2 * sms && L_width > 49152 ? 1024 : 256;
   const int* one_per_sm = g_active_clusters[device];   // of 1, 2, 4, 8, 16 CTAs

@@ -414,3 +414,19 @@ def test_a_result_that_does_not_fit_is_an_out_of_memory_error():
             pkg.fast_topk_v3(s, lengths, 2048, index_dtype=torch.int64)
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("variable,value,shape", [("FF_TOPK_CLUSTER", "2", (2, 1)), ("FF_TOPK_GROUPS", "1", (16, 1))])
+def test_launch_shape_forced_by_the_environment(ff, oracle, monkeypatch, variable, value, shape):
+    """The environment forces the shape of short rows as it does that of long ones."""
+    import ctypes
+    _, lib = ff
+    B, L, k = 4, 16384, 512
+    monkeypatch.setenv(variable, value)
+    lib.ff_topk_set_cluster_override(0)
+    got = (ctypes.c_int32 * 2)()
+    assert lib.ff_topk_policy_launch_shape(B, L, k, 1, 0, got) == 0
+    assert tuple(got) == shape
+    s = torch.randn((B, L), generator=torch.Generator().manual_seed(3))
+    run_case(ff, oracle, s, torch.full((B,), L, dtype=torch.int32), k)

@@ -193,6 +193,9 @@ __device__ __forceinline__ uint32_t cut_in_digit(const uint32_t* packed, int t, 
 template <int NT>
 __device__ __forceinline__ void pack_bins(uint32_t* hist, bool raw, int limit, RowsShared& sh, int* warp_tot) {
   constexpr int per = kRowsBins / NT;
+  // whole 16-byte quads per thread, their rotation a mask, and a divisor of the 32 banks: 4,096 bins over 192 threads are
+  // 21 each, at 4-byte addresses
+  static_assert((NT & (NT - 1)) == 0 && per % 4 == 0 && 32 % per == 0, "bins per thread: 4, 8, 16 or 32");
   const int tid = threadIdx.x;
   const int m0 = tid * per;
   const bool up = !raw || m0 >= kRowsBins / 2;   // the thread's bins lie in ascending order

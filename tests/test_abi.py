@@ -1,6 +1,7 @@
 """The C-ABI library loads, exports every declared symbol, and rejects bad arguments before touching a GPU."""
 import ctypes
 import re
+import subprocess
 from pathlib import Path
 
 import pytest
@@ -64,3 +65,16 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.undo()
     _lib.load.cache_clear()
     _lib.load()
+
+
+@pytest.mark.parametrize("threads,compiles", [(256, True), (192, False)])
+def test_thread_counts_the_bin_scan_cannot_serve_do_not_compile(tmp_path, threads, compiles):
+    """192 threads would read their 21 bins each with misaligned 16-byte loads: refused when it is built."""
+    from flash_float_jit_kernels_b200 import build
+    src = tmp_path / "scan.cu"
+    src.write_text(f'#include "{build.CSRC}/ff_topk_rows.cuh"\n'
+                   f"template __device__ void ff::pack_bins<{threads}>(uint32_t*, bool, int, ff::RowsShared&, int*);\n")
+    res = subprocess.run([build._nvcc(), "-arch=compute_100a", "-std=c++17", "-ptx", "-o", str(tmp_path / "scan.ptx"), str(src)],
+                         capture_output=True, text=True, timeout=600)
+    assert (res.returncode == 0) == compiles, res.stderr[-2000:]
+    assert compiles or "bins per thread" in res.stderr

@@ -562,9 +562,16 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     }
     const int32_t* table = p.epilogue == 1 ? p.table + static_cast<int64_t>(table_row) * p.table_stride : nullptr;
     const int32_t offset = p.epilogue == 2 ? p.offsets[row] : 0;
+    // Nothing is addressed by a position outside the row: scores that are overwritten between the two sweeps (a missing
+    // wait between streams) and handed-over lists of a longer row give wrong results, not wrong accesses.
+    auto inside = [&](int32_t o) {
+      const bool in = static_cast<uint32_t>(o) < static_cast<uint32_t>(len);
+      if (!in && o >= 0) (void)FF_IN_RANGE(p, o, len, 19);
+      return in;
+    };
     auto result = [&](int j) -> int32_t {
       const int32_t o = index_of(j);
-      return o < 0 ? -1 : table != nullptr ? __ldg(table + o) : o + offset;
+      return !inside(o) ? -1 : table != nullptr ? __ldg(table + o) : o + offset;
     };
     const int64_t at = static_cast<int64_t>(row) * k;
     if (p.out_idx64 != nullptr) {
@@ -573,7 +580,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
       for (int j = tid; j < k; j += NT) out[j] = result(j);
     } else if (p.epilogue != 1 && ((k & 3) | (static_cast<int>(reinterpret_cast<uintptr_t>(p.out_idx)) & 15)) == 0) {
       int4* out = reinterpret_cast<int4*>(p.out_idx + at);
-      auto placed = [&](int32_t o) { return o < 0 ? -1 : o + offset; };
+      auto placed = [&](int32_t o) { return inside(o) ? o + offset : -1; };
 #pragma unroll 2
       for (int j = tid; j < (k >> 2); j += NT) {
         const int4 o = quad_of(j);
@@ -827,7 +834,8 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       const uint32_t d = (key_bits(depth[j]) - base) >> shift;
-      if (pos[j] >= 0 && FF_IN_RANGE(p, d, kRowsBins, 15)) atomicAdd(&hist[d], 1u);
+      if (pos[j] >= 0 && !FF_IN_RANGE(p, d, kRowsBins, 15)) pos[j] = -1;   // (a place that trips drops its survivor)
+      if (pos[j] >= 0) atomicAdd(&hist[d], 1u);
     }
     __syncthreads();
     pack_bins<NT>(hist, false, n, sh, sh.warp_tot[2]);
@@ -855,7 +863,8 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   }
   __syncthreads();   // the bins are clear
   mine([&](int j) {
-    if (pos[j] >= 0 && FF_IN_RANGE(p, where[j], 2 * kCap, 12)) where[j] |= atomicAdd(&bins[where[j]], 1u) << 16;
+    if (pos[j] >= 0 && !FF_IN_RANGE(p, where[j], 2 * kCap, 12)) pos[j] = -1;
+    if (pos[j] >= 0) where[j] |= atomicAdd(&bins[where[j]], 1u) << 16;
   });
   __syncthreads();
   FF_TRACE(p, 22);
@@ -896,7 +905,8 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
       }
     });
     mine([&](int j) {
-      if (pos[j] >= 0 && FF_IN_RANGE(p, at[j], kCap, 13)) bucketed[at[j]] = depth[j];
+      if (pos[j] >= 0 && !FF_IN_RANGE(p, at[j], kCap, 13)) pos[j] = -1;
+      if (pos[j] >= 0) bucketed[at[j]] = depth[j];
     });
   }
   __syncthreads();
@@ -925,7 +935,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
         tied |= more;
       }
       where[j] = rank;
-      if (FF_IN_RANGE(p, rank, kCap, 18)) ranked[rank] = pos[j];
+      if (FF_IN_RANGE(p, rank, kCap, 18)) ranked[rank] = pos[j]; else pos[j] = -1;
     }
   });
   if (__syncthreads_or(tied ? 1 : 0)) {
@@ -974,11 +984,15 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
       const int want = hint_target_rank(k);
       const int rank_a = min(n, want) - 1, rank_m = n >> 1;
       if (tid == 0) {
-        const float va = Elem<T>::to_float(rowp[ranked[rank_a]]), vm = Elem<T>::to_float(rowp[ranked[rank_m]]);
-        float guess = va;
-        if (n < want && rank_a > rank_m) {
-          const float lower = va - (vm - va) * (static_cast<float>(want - 1 - rank_a) / static_cast<float>(rank_a - rank_m));
-          if (lower == lower && fabsf(lower) <= 3.0e38f) guess = lower;
+        const int32_t at_a = rank_a >= 0 ? ranked[rank_a] : -1, at_m = ranked[rank_m];
+        float guess = __uint_as_float(0x7fffffffu);
+        if (static_cast<uint32_t>(at_a) < static_cast<uint32_t>(len) && static_cast<uint32_t>(at_m) < static_cast<uint32_t>(len)) {
+          const float va = Elem<T>::to_float(rowp[at_a]), vm = Elem<T>::to_float(rowp[at_m]);
+          guess = va;
+          if (n < want && rank_a > rank_m) {
+            const float lower = va - (vm - va) * (static_cast<float>(want - 1 - rank_a) / static_cast<float>(rank_a - rank_m));
+            if (lower == lower && fabsf(lower) <= 3.0e38f) guess = lower;
+          }
         }
         p.hint_out[row] = guess;
       }

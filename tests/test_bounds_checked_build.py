@@ -80,3 +80,37 @@ def test_full_work_arrays_through_the_checked_build(oracle, shape):
         out, status = _launch(lib, sd, ld, k, hint=hint)
         assert status & _lib.FF_STATUS_BOUNDS == 0, f"status {status:#x}"
         assert np.array_equal(out.cpu().numpy(), exp)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("checked", [False, True])
+def test_a_position_beyond_the_row_addresses_nothing(checked):
+    """A handed-over list with a position behind the row's end (but inside the score buffer): no score is read and no table
+    gathered with it in either build, and the checked one names the place."""
+    from flash_float_jit_kernels_b200 import _lib
+    lib = _lib.load_checked() if checked else _lib.load()
+    dev = torch.device("cuda:0")
+    L, n, k, given = 20000, 15000, 512, 600
+    s = torch.randn((1, L), generator=torch.Generator().manual_seed(2)).abs() + 0.5
+    order = torch.argsort(s[0, :n], descending=True)[:given]
+    guess = float(s[0, order[-1]])
+    pos = order.numpy().astype(np.uint32)
+    pos[10] = n + 1000
+    keys = s[0, order].numpy().view(np.uint32) | np.uint32(0x80000000)
+    entries = (keys.astype(np.uint64) << np.uint64(32)) | (~pos).astype(np.uint64)
+    buf = np.zeros(_lib.FF_TOPK_HANDOVER_ROW_BYTES, dtype=np.uint8)
+    buf[:4] = np.array([given], dtype=np.uint32).view(np.uint8)
+    buf[64:64 + 8 * given] = entries.view(np.uint8)
+    handover = torch.from_numpy(buf).to(dev)
+    sd, ld = s.to(dev), torch.tensor([n], dtype=torch.int32, device=dev)
+    hint = torch.tensor([guess], dtype=torch.float32, device=dev)
+    out = torch.full((1, k), -7, dtype=torch.int32, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    rc = lib.ff_topk_launch_handover(sd.data_ptr(), L, ld.data_ptr(), None, out.data_ptr(), 1, L, k, hint.data_ptr(),
+                                     hint.data_ptr(), handover.data_ptr(), None, 0, status.data_ptr(),
+                                     torch.cuda.current_stream().cuda_stream)
+    assert rc == 0, lib.ff_last_error_string()
+    torch.cuda.synchronize()
+    assert bool(int(status.item()) & _lib.FF_STATUS_BOUNDS) == checked
+    got, exp = out.cpu().numpy()[0], order[:k].numpy()
+    assert got[10] == -1 and np.array_equal(np.delete(got, 10), np.delete(exp, 10))

@@ -390,8 +390,10 @@ __global__ void __launch_bounds__(kThreads, 2) indexer_logits_kernel(const Param
 // The tiles of all rows are numbered row by row (a prefix sum over the rows' tile counts, computed by every CTA from
 // the device-side lengths) and CTA c of the G takes tiles [c T / G, (c + 1) T / G): one wave, the same number of
 // tiles for everyone whatever the lengths, and at most a row change or two per CTA on the way.
-//   * one thread asks for the K tiles with cp.async.bulk.tensor (128-byte swizzle done by the copy; keys
-//     past the tensor's end arrive as zero) and, at a row change, for the new row's q into the other q buffer;
+//   * one thread asks for the K tiles with cp.async.bulk.tensor (128-byte swizzle done by the copy) and, at a row
+//     change, for the new row's q into the other q buffer.  A row's last tile is moved up so that it ends with the
+//     row's last key: nothing at or behind a row's length is read (a row shorter than a tile starts in front of
+//     its first key, where the copy fills in zeros);
 //   * one thread issues the tensor-core instructions;
 //   * four epilogue warps as above; in front of their first tile they also write the -inf of a fresh result.
 // Bound by the K bytes: 64 full rows of 131,072 keys 179.7 us (6.16 TB/s, 94 % of the measured copy peak), lengths
@@ -414,6 +416,7 @@ struct RunShared {
   uint32_t tmem_base;
   int timed_out;
   int prefix[kRunMaxRows + 1];           // tiles in front of row b
+  uint8_t last[kRunMaxRows];             // keys in the last tile of row b (1 to 128)
   float w[2][kHeads];
   unsigned long long handover[kEpilogueWarps][2][kHandoverWarpBuf];
 };
@@ -443,6 +446,8 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
 struct RunCursor {
   int row, tile, n_tiles;  // tile of the row, tiles of the row
   int rows_done;           // rows of this CTA before this one (drives the q buffers)
+  // How far the current tile is moved up (0 but for a row's last one).
+  __device__ __forceinline__ int moved_up(const uint8_t* last) const { return tile == n_tiles - 1 ? kTileKeys - last[row] : 0; }
   __device__ __forceinline__ void start(const int* prefix, int B, int first) {
     int lo = 0, hi = B;    // last row with prefix[row] <= first (empty rows share a prefix with the next)
     while (hi - lo > 1) {
@@ -507,7 +512,9 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
     int running = 0;
     for (int b0 = 0; b0 < B; b0 += 32) {
       const int b = b0 + lane;
-      int incl = b < B ? (clamp_len(p, b) + kTileKeys - 1) / kTileKeys : 0;
+      const int len = b < B ? clamp_len(p, b) : 0;
+      if (b < B) sh.last[b] = static_cast<uint8_t>(((len - 1) & (kTileKeys - 1)) + 1);
+      int incl = (len + kTileKeys - 1) / kTileKeys;
 #pragma unroll
       for (int off = 1; off < 32; off <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, incl, off);
@@ -543,7 +550,7 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
         if (i >= kRunStages)
           (void)mbar_wait(smem_u32(&sh.empty[stage]), static_cast<uint32_t>((i / kRunStages - 1) & 1), &sh.timed_out);
         mbar_expect(smem_u32(&sh.full[stage]), kTileBytes);
-        tma_load_3d(k_s + stage * kTileBytes, &k_map, 0, c.tile * kTileKeys, c.row, smem_u32(&sh.full[stage]));
+        tma_load_3d(k_s + stage * kTileBytes, &k_map, 0, c.tile * kTileKeys - c.moved_up(sh.last), c.row, smem_u32(&sh.full[stage]));
         new_row = c.next(sh.prefix, B);
       }
     }
@@ -616,11 +623,7 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
       __syncwarp();
       n_cur = n_pending = 0;
     };
-    int len = 0;
-    if (n_mine > 0) {
-      len = clamp_len(p, c.row);
-      enter_row();
-    }
+    if (n_mine > 0) enter_row();
     for (int i = 0; i < n_mine; ++i) {
       const int buf = i & 1, wb = c.rows_done & 1;
       (void)mbar_wait(smem_u32(&sh.tfull[buf]), static_cast<uint32_t>((i / 2) & 1), &sh.timed_out);
@@ -629,15 +632,18 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
       const float s = score_of_lane(taddr, sh.w[wb]);
       tc_fence_before();
       mbar_arrive(smem_u32(&sh.tempty[buf]));
-      const int key = c.tile * kTileKeys + key_in_tile;
+      // the first lanes of a tile that is moved up hold keys of the tile before it, and write the -inf behind the row's end instead
+      const int up = c.moved_up(sh.last);
+      const bool own = key_in_tile >= up;
+      const int key = c.tile * kTileKeys + key_in_tile - up + (own ? 0 : kTileKeys);
       if (key < p.L_width)
-        p.scores[static_cast<int64_t>(c.row) * p.score_stride + key] = key < len ? s : __uint_as_float(0xff800000u);
+        p.scores[static_cast<int64_t>(c.row) * p.score_stride + key] = own ? s : __uint_as_float(0xff800000u);
       if (hint == hint) {
         if (n_pending > 0) {   // last tile's reservation has long arrived
           store_handover(row_base, sh.handover[warp][cur ^ 1], n_pending, __shfl_sync(0xffffffffu, pending_base, 0), lane);
           n_pending = 0;
         }
-        const bool hit = key < len && !(s < hint);
+        const bool hit = own && !(s < hint);
         const uint32_t votes = __ballot_sync(0xffffffffu, hit);
         if (votes != 0u) {
           if (hit)
@@ -658,7 +664,6 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
         leave_row();
         if (i + 1 < n_mine) {
           load_w(c.row, c.rows_done & 1);
-          len = clamp_len(p, c.row);
           enter_row();
           asm volatile("bar.sync 1, 128;" ::: "memory");
         }

@@ -32,7 +32,8 @@ extern "C" {
 #define FF_INDEXER_HEAD_DIM 128
 
 /* q_e4m3: [B, 64, 128] bytes, contiguous, 16-byte aligned.
- * k_e4m3: key j of row b at k_e4m3 + b * k_row_stride_bytes + j * 128 (16-byte aligned stride).
+ * k_e4m3: key j of row b at k_e4m3 + b * k_row_stride_bytes + j * 128 (16-byte aligned stride); keys at or
+ * behind lengths[b] are not read and need not exist.
  * w: [B, 64] float32.  lengths: [B] int32.  scores: [B, score_stride] float32, score_stride >= L_width.
  * ctas_per_row: 0 = automatic (shares of about 32 tiles of 128 keys per CTA, sized from each row's
  * length on the device); > 0 = that many CTAs for a full row; < 0 = the persistent variant (two CTAs

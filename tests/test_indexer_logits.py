@@ -95,6 +95,38 @@ def test_runs_of_tiles_over_many_rows(oracle, B, L):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 64, 127, 128, 129, 255, 1000])
+def test_keys_behind_a_rows_length_need_not_exist(oracle, n):
+    """The last row's K ends with its last key, far in front of the width: scores and hand-over list of the keys that are
+    there, -inf up to the tile's end, nothing behind it."""
+    from flash_float_jit_kernels_b200.indexer_logits import load, new_handover
+    dev, L = torch.device("cuda:0"), 4096
+    q, k, w = _make(2, L, n, dev)
+    keys = torch.cat([k[0].reshape(-1), k[1, :n].reshape(-1)]).to(dev)
+    qd, wd, lengths = q.to(dev), w.to(dev), torch.tensor([L, n], dtype=torch.int32, device=dev)
+    scores = torch.full((2, L), 7.0, device=dev)
+    hint = torch.tensor([float("nan"), 0.0], device=dev)       # every score of row 1 is listed
+    handover = new_handover(2, dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    rc = load().ff_indexer_logits_launch_handover(
+        qd.data_ptr(), keys.data_ptr(), L * 128, wd.data_ptr(), lengths.data_ptr(), scores.data_ptr(), L, 2, L, 0,
+        hint.data_ptr(), handover.data_ptr(), status.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    got = scores.cpu().numpy()
+    for b, m in ((0, L), (1, n)):
+        exp, _ = oracle.indexer_logits(q[b].float().numpy(), k[b, :m].float().numpy(), w[b].numpy())
+        assert np.array_equal(got[b, :m].view(np.uint32), exp.view(np.uint32)), b
+    end = (n + 127) // 128 * 128
+    assert np.all(np.isneginf(got[1, n:end])) and np.all(got[1, end:] == 7.0)
+    row = handover[handover.numel() // 2:].cpu().numpy()
+    assert int(row[:4].view(np.uint32)[0]) == n
+    listed = ~row[64:64 + 8 * n].view(np.uint64).astype(np.uint32)
+    assert sorted(listed.tolist()) == list(range(n))
+
+
+@pytest.mark.gpu
 def test_logits_feed_the_indexer(oracle):
     """Producer and selector back to back: the top-k of the produced scores is the oracle's
     top-k of the oracle's scores."""

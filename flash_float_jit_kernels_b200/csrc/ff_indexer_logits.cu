@@ -500,11 +500,13 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
     sh.prefix[0] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // Not in front of the wait: a kernel in front that let this one in before it had its own tensor memory would wait for
+  // the columns held here, and this one for its end.  And not behind the signal, for the same reason the other way round.
   if (warp == kMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh.tmem_base)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   // tiles per row -> exclusive prefix (one warp sums 32 rows at a time)
@@ -533,6 +535,7 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
   const int n_mine = static_cast<int>(total * (blockIdx.x + 1) / gridDim.x) - first;
   RunCursor c;
   if (n_mine > 0) c.start(sh.prefix, B, first);
+  int asked = 0, asked_q = 0;   // tiles that this thread asked for (copies, or products), and rows of q
 
   if (warp == kRunProducerWarp) {
     // ---------------- copies (one thread) ----------------
@@ -541,14 +544,18 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
       for (int i = 0; i < n_mine; ++i) {
         if (new_row) {
           const int qb = c.rows_done & 1;
-          if (c.rows_done >= 2)   // the buffer's previous row must be multiplied
-            (void)mbar_wait(smem_u32(&sh.qempty[qb]), static_cast<uint32_t>((c.rows_done / 2 - 1) & 1), &sh.timed_out);
+          if (c.rows_done >= 2 &&   // the buffer's previous row must be multiplied
+              !mbar_wait(smem_u32(&sh.qempty[qb]), static_cast<uint32_t>((c.rows_done / 2 - 1) & 1), &sh.timed_out))
+            break;
+          ++asked_q;
           mbar_expect(smem_u32(&sh.qfull[qb]), kQBytes);
           tma_load_3d(q_s + qb * kQBytes, &q_map, 0, 0, c.row, smem_u32(&sh.qfull[qb]));
         }
         const int stage = i % kRunStages;
-        if (i >= kRunStages)
-          (void)mbar_wait(smem_u32(&sh.empty[stage]), static_cast<uint32_t>((i / kRunStages - 1) & 1), &sh.timed_out);
+        if (i >= kRunStages &&
+            !mbar_wait(smem_u32(&sh.empty[stage]), static_cast<uint32_t>((i / kRunStages - 1) & 1), &sh.timed_out))
+          break;
+        asked = i + 1;
         mbar_expect(smem_u32(&sh.full[stage]), kTileBytes);
         tma_load_3d(k_s + stage * kTileBytes, &k_map, 0, c.tile * kTileKeys - c.moved_up(sh.last), c.row, smem_u32(&sh.full[stage]));
         new_row = c.next(sh.prefix, B);
@@ -560,9 +567,9 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
       bool new_row = true;
       for (int i = 0; i < n_mine; ++i) {
         const int stage = i % kRunStages, buf = i & 1, qb = c.rows_done & 1;
-        if (new_row) (void)mbar_wait(smem_u32(&sh.qfull[qb]), static_cast<uint32_t>((c.rows_done / 2) & 1), &sh.timed_out);
-        if (i >= 2) (void)mbar_wait(smem_u32(&sh.tempty[buf]), static_cast<uint32_t>((i / 2 - 1) & 1), &sh.timed_out);
-        (void)mbar_wait(smem_u32(&sh.full[stage]), static_cast<uint32_t>((i / kRunStages) & 1), &sh.timed_out);
+        if (new_row && !mbar_wait(smem_u32(&sh.qfull[qb]), static_cast<uint32_t>((c.rows_done / 2) & 1), &sh.timed_out)) break;
+        if (i >= 2 && !mbar_wait(smem_u32(&sh.tempty[buf]), static_cast<uint32_t>((i / 2 - 1) & 1), &sh.timed_out)) break;
+        if (!mbar_wait(smem_u32(&sh.full[stage]), static_cast<uint32_t>((i / kRunStages) & 1), &sh.timed_out)) break;
         tc_fence_after();
         const uint32_t a_addr = k_s + stage * kTileBytes, b_addr = q_s + qb * kQBytes;
 #pragma unroll
@@ -570,8 +577,9 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
           mma_f8(tmem + buf * kHeads, smem_desc(a_addr + ks * 32), smem_desc(b_addr + ks * 32), ks > 0 ? 1u : 0u);
         mma_commit(smem_u32(&sh.empty[stage]));
         mma_commit(smem_u32(&sh.tfull[buf]));
+        asked = i + 1;
         new_row = c.next(sh.prefix, B);
-        if (new_row) mma_commit(smem_u32(&sh.qempty[qb]));
+        if (new_row && i + 1 < n_mine) mma_commit(smem_u32(&sh.qempty[qb]));   // (nobody waits for the last row's)
       }
     }
   } else {
@@ -673,6 +681,21 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
   }
   tc_fence_before();
   __syncthreads();
+  if (sh.timed_out) {
+    // After a wait that ran out nobody may have waited for the last copies and products: they have to be done before the
+    // tensor memory goes back and the CTA leaves.  (These waits have limits of their own.)
+    int late = 0;
+    if (warp == kRunProducerWarp) {
+      for (int j = max(asked - kRunStages, 0); j < asked; ++j)
+        (void)mbar_wait(smem_u32(&sh.full[j % kRunStages]), static_cast<uint32_t>((j / kRunStages) & 1), &late);
+      for (int j = max(asked_q - 2, 0); j < asked_q; ++j)
+        (void)mbar_wait(smem_u32(&sh.qfull[j & 1]), static_cast<uint32_t>((j / 2) & 1), &late);
+    } else if (warp == kMmaWarp) {
+      for (int j = max(asked - 2, 0); j < asked; ++j)
+        (void)mbar_wait(smem_u32(&sh.tfull[j & 1]), static_cast<uint32_t>((j / 2) & 1), &late);
+    }
+    __syncthreads();
+  }
   if (warp == kMmaWarp) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");

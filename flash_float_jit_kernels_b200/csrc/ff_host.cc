@@ -371,7 +371,7 @@ PyObject* logits(PyObject* py_q, PyObject* py_k, PyObject* py_w, PyObject* py_le
   if (is_none(py_out)) {
     // the kernel writes the -inf behind the rows' ends itself where it can (a fill kernel of its own: 5 us for 64 x 128 Ki)
     const auto options = at::TensorOptions().dtype(at::kFloat).device(dev);
-    fill = ctas_per_row == 0 && B <= FF_INDEXER_MAX_FILL_ROWS && keys->stride(0) < (int64_t{1} << 40);
+    fill = ctas_per_row == 0 && B <= FF_INDEXER_MAX_FILL_ROWS && (B == 1 || keys->stride(0) < (int64_t{1} << 40));
     fresh = fill ? at::empty({B, L}, options) : at::full({B, L}, -std::numeric_limits<float>::infinity(), options);
     out = &fresh;
   } else {

@@ -776,9 +776,12 @@ int ff_indexer_logits_launch_fresh(const void* q_e4m3, const void* k_e4m3, int64
   if (B < 0 || L_width < 0) return fail(-2, "negative B or L_width");
   if ((hint == nullptr) != (handover == nullptr)) return fail(-3, "hint and handover go together");
   if (handover != nullptr && ((reinterpret_cast<uintptr_t>(handover) & 63u) != 0 || ctas_per_row < 0))
-    return fail(-2, "the hand-over list must be 64-byte aligned and needs the default kernel (ctas_per_row >= 0)");
-  if (fill != 0 && (ctas_per_row != 0 || B > ffl::kRunMaxRows))
-    return fail(-2, "fill needs ctas_per_row == 0 and at most FF_INDEXER_MAX_FILL_ROWS rows");
+    return fail(-2, "the hand-over list must be 64-byte aligned and needs ctas_per_row >= 0");
+  // A tensor map holds row strides below 2^40 bytes; a single row has none.
+  const bool mapped = B <= 1 || k_row_stride_bytes < (1ll << 40);
+  if (fill != 0 && (ctas_per_row != 0 || B > ffl::kRunMaxRows || !mapped))
+    return fail(-2, "fill needs ctas_per_row == 0, at most FF_INDEXER_MAX_FILL_ROWS rows and a K row stride below 2^40 bytes");
+  if (ctas_per_row < 0 && B > ffl::kRunMaxRows) return fail(-6, "ctas_per_row < 0 takes at most 1024 rows");
   if (B == 0 || L_width == 0) return 0;
   if (q_e4m3 == nullptr || k_e4m3 == nullptr || w == nullptr || lengths == nullptr || scores == nullptr)
     return fail(-3, "q, k, w, lengths and scores must not be NULL");
@@ -808,13 +811,12 @@ int ff_indexer_logits_launch_fresh(const void* q_e4m3, const void* k_e4m3, int64
   p.status = status;
   p.hint = hint;
   p.handover = static_cast<unsigned char*>(handover);
-  // A K row stride that a tensor map cannot hold (2^40 bytes) goes to the other kernel too.
-  if (ctas_per_row <= 0 && B <= ffl::kRunMaxRows && k_row_stride_bytes < (1ll << 40)) {
+  if (ctas_per_row <= 0 && B <= ffl::kRunMaxRows && mapped) {
     // Two CTAs per SM, or one per tile where there are fewer tiles.
     const int64_t most = static_cast<int64_t>(B) * tiles;
     const ffl::RunParams a = {p, B, fill};
     CUtensorMap k_map, q_map;
-    if (!encode_map(&k_map, k_e4m3, L_width, B, k_row_stride_bytes, ffl::kTileKeys) ||
+    if (!encode_map(&k_map, k_e4m3, L_width, B, B > 1 ? k_row_stride_bytes : static_cast<int64_t>(L_width) * ffl::kDim, ffl::kTileKeys) ||
         !encode_map(&q_map, q_e4m3, ffl::kHeads, B, ffl::kQBytes, ffl::kHeads))
       return fail(-2, "cuTensorMapEncodeTiled rejected q or K");
     cudaLaunchConfig_t cfg = {};
@@ -832,11 +834,10 @@ int ff_indexer_logits_launch_fresh(const void* q_e4m3, const void* k_e4m3, int64
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return 0;
   }
-  if (ctas_per_row < 0) return fail(-6, "the persistent kernel takes at most 1024 rows");
-  // More rows than the persistent kernel numbers: every row is cut into shares of about 32 tiles (512 KiB of K), but
+  // More rows than the persistent kernel numbers (or a K row stride it cannot map): every row is cut into shares of about 32 tiles (512 KiB of K), but
   // into at least so many that the batch has about four CTAs per SM when every row is full, so that
   // small batches still fill the device.  ctas_per_row > 0 fixes the number of CTAs of a full row.
-  int per_row = ctas_per_row;
+  int per_row = ctas_per_row > 0 ? ctas_per_row : 0;
   int tiles_per_cta = 32;
   if (per_row <= 0) {
     const int want_ctas = (4 * g_sms[device] + B - 1) / B;             // per row

@@ -35,9 +35,9 @@ extern "C" {
  * k_e4m3: key j of row b at k_e4m3 + b * k_row_stride_bytes + j * 128 (16-byte aligned stride); keys at or
  * behind lengths[b] are not read and need not exist.
  * w: [B, 64] float32.  lengths: [B] int32.  scores: [B, score_stride] float32, score_stride >= L_width.
- * ctas_per_row: 0 = automatic (shares of about 32 tiles of 128 keys per CTA, sized from each row's
- * length on the device); > 0 = that many CTAs for a full row; < 0 = the persistent variant (two CTAs
- * per SM walk units of 8 tiles round robin; at most 1024 rows). */
+ * ctas_per_row: 0 = automatic: up to 1024 rows, a persistent grid of two CTAs per SM that deals the batch's tiles of 128
+ * keys out evenly, from the lengths on the device; more rows (or a K row stride of 2^40 bytes and more), shares of about 32
+ * tiles per CTA.  > 0 = that many CTAs for a full row.  < 0 = as 0, but more than 1024 rows and hand-over lists are refused. */
 int ff_indexer_logits_launch(const void* q_e4m3, const void* k_e4m3, int64_t k_row_stride_bytes,
                              const float* w, const int32_t* lengths, float* scores,
                              int64_t score_stride, int32_t B, int32_t L_width, int32_t ctas_per_row,
@@ -52,7 +52,7 @@ int ff_indexer_logits_launch(const void* q_e4m3, const void* k_e4m3, int64_t k_r
  * The counts must be zero when the launch starts (the buffer is zero-filled once by the caller;
  * ff_topk_launch_handover leaves every count it has read at zero again).  With the list the select
  * reads no score at all when the guess fits; when it does not, it falls back to the scores.
- * Only the default kernel (ctas_per_row >= 0) takes a hand-over. */
+ * ctas_per_row < 0 takes no hand-over. */
 #define FF_HANDOVER_ROW_BYTES (64 + 4096 * 8)
 int ff_indexer_logits_launch_handover(const void* q_e4m3, const void* k_e4m3, int64_t k_row_stride_bytes,
                                       const float* w, const int32_t* lengths, float* scores,
@@ -61,7 +61,8 @@ int ff_indexer_logits_launch_handover(const void* q_e4m3, const void* k_e4m3, in
 
 /* The same for a `scores` buffer that holds nothing yet: with fill = 1 every position behind a row's last key is
  * written as -inf, not only those inside a processed 128-key tile, so that the caller need not fill the
- * buffer first.  fill needs ctas_per_row == 0 and B <= FF_INDEXER_MAX_FILL_ROWS; hint and handover may be NULL. */
+ * buffer first.  fill needs ctas_per_row == 0, B <= FF_INDEXER_MAX_FILL_ROWS and a K
+ * row stride below 2^40 bytes; hint and handover may be NULL. */
 #define FF_INDEXER_MAX_FILL_ROWS 1024
 int ff_indexer_logits_launch_fresh(const void* q_e4m3, const void* k_e4m3, int64_t k_row_stride_bytes, const float* w,
                                    const int32_t* lengths, float* scores, int64_t score_stride, int32_t B,

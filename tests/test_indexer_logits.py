@@ -32,6 +32,22 @@ def test_library_loads_and_exports_every_declared_symbol():
     assert lib.ff_indexer_logits_launch(None, None, 0, None, None, None, 0, 0, 8, 0, None, None) == 0
 
 
+def test_what_the_persistent_grid_cannot_take_is_refused_by_its_name():
+    """Neither a fill that would be left out nor a message that names the wrong limit."""
+    from flash_float_jit_kernels_b200 import build, indexer_logits
+    build.build_indexer_library()
+    lib = indexer_logits.load()
+    fresh = lib.ff_indexer_logits_launch_fresh
+    far = 1 << 40
+    assert fresh(None, None, far, None, None, None, 8, 2, 8, 0, 1, None, None, None, None) == -2
+    assert b"row stride" in lib.ff_indexer_last_error_string()
+    assert lib.ff_indexer_logits_launch(None, None, 1024, None, None, None, 8, 1025, 8, -1, None, None) == -6
+    assert b"1024 rows" in lib.ff_indexer_last_error_string()
+    # (not refused for its rows; the missing pointers stop it)
+    assert lib.ff_indexer_logits_launch(None, None, far, None, None, None, 8, 2, 8, -1, None, None) == -3
+    assert fresh(None, None, far, None, None, None, 8, 1, 8, 0, 1, None, None, None, None) == -3
+
+
 def test_oracle_logits_agree_with_a_plain_matmul(oracle):
     g = torch.Generator().manual_seed(0)
     q = (torch.randn((64, 128), generator=g) / 4).to(torch.float8_e4m3fn).float()

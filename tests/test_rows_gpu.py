@@ -80,3 +80,35 @@ def test_windows_types_guesses_and_wide_indices(oracle, B, dtype):
     hint = new_threshold_hint(B, "cuda")
     for _ in range(3):
         _check(oracle, s, lengths, k, rs, threshold_hint=hint)
+
+
+def _us_per_call(call, n=20):
+    call()
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    times = []
+    for _ in range(3):
+        start.record()
+        for _ in range(n):
+            call()
+        end.record()
+        end.synchronize()
+        times.append(start.elapsed_time(end) * 1e3 / n)
+    return min(times)
+
+
+@pytest.mark.parametrize("B,L", [(4, 65536), (30, 65536), (64, 131072), (200, 16384)])
+def test_equal_neighbours_are_exact_and_cost_little(oracle, B, L):
+    """Rows of blocks of 32 equal scores with full mantissas, whose survivors share depths by the dozen: exact, and within a
+    few times the call without ties (one list of all of them that each survivor walked took 16 to 30 times)."""
+    from flash_float_jit_kernels_b200 import fast_topk_v3
+    k, dev = 2048, torch.device("cuda:0")
+    g = torch.Generator().manual_seed(B)
+    x = torch.randn((B, L), generator=g)
+    blocks = x[:, : L // 32].repeat_interleave(32, dim=1).contiguous()
+    lengths = torch.full((B,), L, dtype=torch.int32)
+    _check(oracle, blocks, lengths, k)
+    xd, bd, ld = x.to(dev), blocks.to(dev), lengths.to(dev)
+    out = torch.empty((B, k), dtype=torch.int32, device=dev)
+    plain = _us_per_call(lambda: fast_topk_v3(xd, ld, k, out=out))
+    tied = _us_per_call(lambda: fast_topk_v3(bd, ld, k, out=out))
+    assert tied < 4 * max(plain, 15.0), f"{tied:.1f} us against {plain:.1f} us"

@@ -112,3 +112,22 @@ def test_equal_neighbours_are_exact_and_cost_little(oracle, B, L):
     plain = _us_per_call(lambda: fast_topk_v3(xd, ld, k, out=out))
     tied = _us_per_call(lambda: fast_topk_v3(bd, ld, k, out=out))
     assert tied < 4 * max(plain, 15.0), f"{tied:.1f} us against {plain:.1f} us"
+
+
+@pytest.mark.parametrize("B,L", [(4, 65536), (30, 65536), (200, 16384)])
+@pytest.mark.parametrize("rest", [float("-inf"), 0.0])
+def test_masked_rows_are_exact_and_cost_little(oracle, B, L, rest):
+    """About a thousand scores and one value everywhere else, the row's first few hundred of which are among the top k: exact,
+    and within a few times the call without ties (all of those in one bucket took ten to thirty times)."""
+    from flash_float_jit_kernels_b200 import fast_topk_v3
+    k, dev = 2048, torch.device("cuda:0")
+    g = torch.Generator().manual_seed(B)
+    x = torch.randn((B, L), generator=g).abs() + 0.1
+    masked = torch.where(torch.rand((B, L), generator=g) < 1000.0 / L, x, torch.full_like(x, rest))
+    lengths = torch.full((B,), L, dtype=torch.int32)
+    _check(oracle, masked, lengths, k)
+    xd, md, ld = x.to(dev), masked.to(dev), lengths.to(dev)
+    out = torch.empty((B, k), dtype=torch.int32, device=dev)
+    plain = _us_per_call(lambda: fast_topk_v3(xd, ld, k, out=out))
+    tied = _us_per_call(lambda: fast_topk_v3(md, ld, k, out=out))
+    assert tied < 5 * max(plain, 15.0), f"{tied:.1f} us against {plain:.1f} us"

@@ -85,8 +85,9 @@ def test_graphs_of_one_stream_replayed_on_two(oracle):
     del graphs, graph
 
 
-def test_scratch_of_a_capture_goes_back_with_the_graph():
-    from flash_float_jit_kernels_b200 import _host, fast_topk_v3
+def test_scratch_of_many_captures_is_bounded_and_goes_back():
+    """The first captures keep their buffers, up to a bound; those of later ones go back with their graphs."""
+    from flash_float_jit_kernels_b200 import _host, _lib, fast_topk_v3
     dev = torch.device("cuda:0")
     s, lengths = _rows(5)
     d, ld, out = s.to(dev), lengths.to(dev), torch.empty((B, K), dtype=torch.int32, device=dev)
@@ -96,18 +97,24 @@ def test_scratch_of_a_capture_goes_back_with_the_graph():
     gc.collect()
 
     def settled():
-        for _ in range(50):                                  # the runtime gives the buffer back on a thread of its own
+        for _ in range(50):                                  # the runtime gives a buffer back on a thread of its own
             torch.cuda.synchronize()
             _host.scratch()(0, 256)
             time.sleep(0.01)
         return torch.cuda.memory_allocated()
 
+    bound, need = 64 << 20, int(_lib.load().ff_topk_workspace_bytes(B, L, K))
     before = settled()
+    for _ in range(bound // need + 1):
+        _capture(side, d, ld, out)
+    gc.collect()
+    kept = settled()
+    assert kept - before <= bound + (2 << 20)
     graphs = [_capture(side, d, ld, out) for _ in range(8)]
-    assert torch.cuda.memory_allocated() > before
+    assert torch.cuda.memory_allocated() - kept >= 8 * need
     for g in graphs:
         g.replay()
     torch.cuda.synchronize()
     del graphs, g
     gc.collect()
-    assert settled() == before
+    assert settled() == kept

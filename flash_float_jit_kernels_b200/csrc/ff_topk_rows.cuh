@@ -5,14 +5,14 @@
 //   threshold one suffix scan; every bin at or above the threshold digit keeps (elements above it, elements in it)
 //   sweep 2   scores not below a cut inside the threshold digit -> survivor list.  The cut is interpolated from
 //             the digit's count with a margin, so that little more than k survive; a cut that turns
-//             out too high is replaced by the digit's lower edge
+//             out too high or too low is moved by what was found
 //   finish    counting sort of the survivors in one pass of bins: a survivor's bin is its EXPECTED rank
 //             (elements above its digit + its position inside the digit, interpolated), at two bins
 //             per survivor, so that buckets hold one or two entries whatever the scores' distribution;
 //             exact rank inside the bucket by counting; indices leave through shared memory
 //
 // What bounds it: batches of many rows keep issue slots and the shared-memory pipe 62 % busy each (4,096 rows of 5,461
-// scores, k = 2048: 107 us, 20,000 warp instructions and 5,000 shared-memory wavefronts per row; the kernel of
+// scores, k = 2048: 103.5 us, 20,000 warp instructions and 4,800 shared-memory wavefronts per row; the kernel of
 // ff_topk_kernel.cuh, one row per SM, took 455 us); a single row is a chain of eight phases, 9.3 us for 16 Ki scores
 // (12.5 us in a cluster of sixteen CTAs of the other kernel).  Hence 64 registers and 36 KiB per row, four rows on an SM.
 #pragma once
@@ -166,27 +166,46 @@ __device__ __forceinline__ float approximate_sqrt(float x) {
   return y * rsqrtf(y);
 }
 
-// Where to cut inside the threshold digit so that a few more than the `wanted` largest of its `in_bin` scores are
-// kept: the density of scores is taken as linear over the digit, from its own count and the next
-// digit's (c0, c1): above a point x of the way down lie (c0 + c1) / 2 x + (c0 - c1) / 2 x^2 of them,
-// solved for the wanted count plus a margin (the steps of scores rounded to bf16,
-// sixteen to a digit, and four standard deviations).  Returns key bits above the digit's lower edge;
-// keep: how many are expected (less than wanted: they do not fit in `room`); spread: the count that the whole digit
-// would have at the kept part's density, which is what the finish interpolates with.
-__device__ __forceinline__ uint32_t cut_in_digit(const uint32_t* packed, int t, int in_bin, int wanted, int room, int& keep, int& spread) {
-  const float c0 = static_cast<float>(in_bin);
-  const int margin = (in_bin >> 4) + static_cast<int>(2.f * approximate_sqrt(c0)) + 8;
-  keep = min(in_bin, wanted + margin);
-  if (keep > room) keep = room >= wanted + (margin >> 1) ? room : -1;
-  const int up = t + 1;
-  float c1 = static_cast<float>((packed[rows_raw_of(up)] & ((1u << kPackShift) - 1u)) >> 1);
-  if ((up & 7) == 0) c1 *= up >= kRowsBins / 2 ? 0.5f : 2.f;   // the next digit spans a step of another width
-  c1 = fminf(c1, 3.f * c0);
-  const float b = 0.5f * (c0 + c1), a = 0.5f * (c0 - c1), want = static_cast<float>(keep);
-  const float x = __fdividef(2.f * want, b + approximate_sqrt(b * b + 4.f * a * want));
+// Where to cut inside the threshold digit so that a few more than the wanted largest of its scores are kept: the density
+// of scores is taken as linear over the digit, from its own count and the next digit's (c0, c1): above a point x of
+// the way down lie b x + a x^2 of them, b = (c0 + c1) / 2 and a = (c0 - c1) / 2.
+struct DigitDensity {
+  float a, b;
+  __device__ __forceinline__ DigitDensity(const uint32_t* packed, int t, int in_bin) {
+    const float c0 = static_cast<float>(in_bin);
+    const int up = t + 1;
+    float c1 = static_cast<float>((packed[rows_raw_of(up)] & ((1u << kPackShift) - 1u)) >> 1);
+    if ((up & 7) == 0) c1 *= up >= kRowsBins / 2 ? 0.5f : 2.f;   // the next digit spans a step of another width
+    c1 = fminf(c1, 3.f * c0);
+    a = 0.5f * (c0 - c1);
+    b = 0.5f * (c0 + c1);
+  }
+  __device__ __forceinline__ float depth_of_count(float n) const { return __fdividef(2.f * n, b + approximate_sqrt(b * b + 4.f * a * n)); }
+  __device__ __forceinline__ float count_above(float x) const { return (b + a * x) * x; }
+};
+// 16-bit scores come in steps of the key (bf16 sixteen to a digit, fp16 128): a cut is put on a step, at or below the
+// point it was meant for, since between two steps it keeps nothing of the lower one (one row in four of 64 to 256 Ki bf16
+// logits found too few).
+template <typename T> constexpr uint32_t kKeyStep = 1u;
+template <> constexpr uint32_t kKeyStep<__nv_bfloat16> = 1u << 16;
+template <> constexpr uint32_t kKeyStep<__half> = 1u << 13;
+template <typename T> constexpr bool kCoarseSteps = kKeyStep<T> >= (1u << 16);
+// How many of the digit's scores to keep for the `wanted` largest of them: a margin of four standard deviations and
+// a sixteenth of the digit (the step of fp32 scores that were rounded to bf16; half of it where the cut is put on
+// such a step anyway); less than wanted: they do not fit in `room`.
+template <typename T>
+__device__ __forceinline__ int kept_in_digit(int in_bin, int wanted, int room) {
+  const int margin = (in_bin >> (kCoarseSteps<T> ? 5 : 4)) + static_cast<int>(2.f * approximate_sqrt(static_cast<float>(in_bin))) + 8;
+  const int keep = min(in_bin, wanted + margin);
+  return keep <= room ? keep : room >= wanted + (margin >> 1) ? room : -1;
+}
+// A point x of the way down the digit as key bits above its lower edge.  spread: the count that the whole digit would have
+// at the density of the `keep` above x, which is what the finish interpolates with.
+template <typename T>
+__device__ __forceinline__ uint32_t cut_at(float x, int keep, int in_bin, int& spread) {
   const bool all = keep >= in_bin || !(x < 1.f);
-  spread = all ? in_bin : static_cast<int>(fminf(__fdividef(want, x), static_cast<float>(kPackMax)));
-  return all ? 0u : static_cast<uint32_t>((1.f - x) * static_cast<float>(1 << kRowsShift));
+  spread = all ? in_bin : static_cast<int>(fminf(__fdividef(static_cast<float>(keep), x), static_cast<float>(kPackMax)));
+  return all ? 0u : static_cast<uint32_t>((1.f - x) * static_cast<float>(1 << kRowsShift)) & ~(kKeyStep<T> - 1u);
 }
 
 // Suffix scan of the bins in monotone order (raw: the array is in rows_raw_digit() order).  Every non-empty bin
@@ -463,6 +482,10 @@ __device__ __noinline__ void collect_row_sparse(const Chunk<T>& c, float vmin, R
   }
 }
 
+template <typename T, int NT, int CAP>
+__device__ __noinline__ void collect_row_again(const Chunk<T>& c, float vmin, RowList<CAP> list, RowsShared& sh) {
+  collect_row<T, NT, CAP, false>(c, nullptr, vmin, 0ull, list, sh);
+}
 template <typename T, int NT, int CAP>
 __device__ __noinline__ void collect_row_exact(const Chunk<T>& c, uint64_t floor_comp, RowList<CAP> list, RowsShared& sh) {
   collect_row<T, NT, CAP, true>(c, nullptr, prefilter_value(static_cast<uint32_t>(floor_comp >> 32)), floor_comp, list, sh);
@@ -744,29 +767,40 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     // ---- sweep 2 ----
     const int above = sh.above, in_bin = sh.total - above;
     const uint32_t bin_key = static_cast<uint32_t>(sh.t) << kRowsShift;
-    int keep, spread;
-    const uint32_t cut = bin_key + cut_in_digit(merged, sh.t, in_bin, k - above, kCap - above, keep, spread);
+    const int keep = kept_in_digit<T>(in_bin, k - above, kCap - above);
     bool exact = bin_key > 0xff800000u || sh.max_bin > kPackMax || keep < k - above ||
                  (sh.total > kCap && 8 * sh.max_bin > 7 * sh.total);
     if (!exact) {
+      int spread;
+      const uint32_t cut =
+          bin_key + cut_at<T>(DigitDensity(merged, sh.t, in_bin).depth_of_count(static_cast<float>(keep)), keep, in_bin, spread);
       if (sparse) collect_row_sparse<T, NT, kCap>(chunk, prefilter_value(cut), own_list, sh);
       else collect_row<T, NT, kCap, false>(chunk, &first, prefilter_value(cut), 0ull, own_list, sh);
       if (tid == 0) merged[rows_raw_of(sh.t)] = packed_bin(above, spread);   // (read in the finish)
       n = gather();
       span = above + keep;
-      if (n < k || n > kCap) {   // the interpolation was off
-        discard();
-        exact = n > kCap || sh.total > kCap;
-        if (!exact) {
-          if (tid == 0) merged[rows_raw_of(sh.t)] = packed_bin(above, in_bin);
-          collect_row<T, NT, kCap, false>(chunk, &first, prefilter_value(bin_key), 0ull, own_list, sh);
-          span = sh.total;
+      if (__builtin_expect(n < k || n > kCap, 0)) {   // the interpolation was off
+        // The whole digit if that fits and the cut was too high; else to a place between k and what fits (nearer to k where
+        // the cut goes down to a step), by the same density scaled to what was found.  Another time or two where that
+        // is off again (blocks of equal scores): a sweep each, further digits take four.
+        const DigitDensity density(merged, sh.t, in_bin);
+        float x = density.depth_of_count(static_cast<float>(keep));
+#pragma unroll 1
+        for (int attempt = 0; attempt < 3 && (n < k || n > kCap); ++attempt) {
+          discard();
+          const int more = n < k && sh.total <= kCap ? in_bin : k - above + ((kCap - k) >> (kCoarseSteps<T> ? 2 : 1));
+          x = density.depth_of_count(static_cast<float>(more) * __fdividef(density.count_above(x), static_cast<float>(max(n - above, 1))));
+          collect_row_again<T, NT, kCap>(chunk, prefilter_value(bin_key + cut_at<T>(x, more, in_bin, spread)), own_list, sh);
+          if (tid == 0) merged[rows_raw_of(sh.t)] = packed_bin(above, spread);
           n = gather();
+          span = above + more;
         }
+        exact = n < k || n > kCap;
+        if (exact) discard();
       }
       rebuild = 8 * sh.max_bin > 7 * sh.total;   // one digit holds nearly all: it says little about their ranks
     }
-    if (exact) {
+    if (__builtin_expect(exact, 0)) {
       rebuild = true;
       const uint64_t floor_comp = sh.total <= kCap ? static_cast<uint64_t>(sh.t) << rows_level_shift(0)
                                                    : deeper_digits<T, NT, CLUSTER>(chunk, hist, merged, k, kCap, sh, p.status);
@@ -866,6 +900,13 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
       if (pos[j] >= 0) where[j] = hist[(key_bits(depth[j]) - base) >> shift];
   } else {
     __syncthreads();   // the list has been read
+  }
+  if (!rebuild && (sh.value_bits & 0x1fffu) == 0u) {
+    // Scores in steps (fp16, bf16, or rounded to them) go on below the cut for up to a sixteenth of the threshold digit, and
+    // those, all given the last rank, would share one bucket (64 ragged rows of 128 Ki bf16 logits: 31.7 us).
+    const uint32_t digit = merged[rows_raw_of(sh.t)];
+    const int above = static_cast<int>(digit >> (kPackShift + 1)), spread = static_cast<int>(digit & ((1u << kPackShift) - 1u)) >> 1;
+    span = min(above + min(span - above + (spread >> 4) + 1, spread), kCap);
   }
   clear_words(bins, 2 * span);
   const DepthMap map = depth_map(shift, sh.value_bits, len);

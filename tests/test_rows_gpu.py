@@ -52,7 +52,9 @@ def _check(oracle, s, lengths, k, rs=None, **kw):
 @pytest.mark.parametrize("B,L,k", [(20, 2049, 2048), (20, 16383, 2048), (20, 16385, 512), (20, 33000, 2048), (20, 70, 1),
                                    (160, 4095, 2048), (160, 4096, 1024), (160, 4097, 512), (160, 12289, 2048), (160, 70, 69),
                                    (310, 9000, 2048), (300, 50001, 1024),
-                                   # clusters of four, eight and sixteen CTAs per row; rows too short for all of them to have a share
+                                   # more scores in one digit than its packed count can hold
+                                   (75, 300001, 2048), (40, 300001, 1024),
+                                   # clusters of four and eight CTAs per row; rows too short for all of them to have a share
                                    (3, 20481, 2048), (12, 40960, 2048), (12, 40961, 512), (11, 98305, 2048), (7, 131073, 1024),
                                    (20, 33001, 2048), (30, 100003, 1), (40, 82001, 1024)])
 def test_rows_of_every_kind(oracle, B, L, k):
@@ -131,3 +133,21 @@ def test_masked_rows_are_exact_and_cost_little(oracle, B, L, rest):
     plain = _us_per_call(lambda: fast_topk_v3(xd, ld, k, out=out))
     tied = _us_per_call(lambda: fast_topk_v3(md, ld, k, out=out))
     assert tied < 5 * max(plain, 15.0), f"{tied:.1f} us against {plain:.1f} us"
+
+
+@pytest.mark.parametrize("B,L", [(64, 131072), (200, 65536)])
+def test_logits_in_steps_are_exact_and_cost_no_more(oracle, B, L):
+    """Logits rounded to bf16 come in sixteen steps to a digit: a cut between two of them has to keep the whole lower step, and
+    the finish bins for all of it (where they did not, the batch took 1.4 times as long as in fp32)."""
+    from flash_float_jit_kernels_b200 import fast_topk_v3
+    k, dev = 2048, torch.device("cuda:0")
+    g = torch.Generator().manual_seed(B)
+    x = (torch.randn((B, L), generator=g) * 1.8 + 9.0).clamp_(min=0.0)
+    lengths = torch.randint(4096, L + 1, (B,), generator=g, dtype=torch.int32)
+    ld, out = lengths.to(dev), torch.empty((B, k), dtype=torch.int32, device=dev)
+    us = {}
+    for name, s in (("f32", x), ("bf16", x.to(torch.bfloat16)), ("f32 in steps", x.to(torch.bfloat16).float())):
+        _check(oracle, s, lengths, k)
+        sd = s.to(dev)
+        us[name] = _us_per_call(lambda: fast_topk_v3(sd, ld, k, out=out))
+    assert us["bf16"] < 1.2 * us["f32"] and us["f32 in steps"] < 1.3 * us["f32"], us

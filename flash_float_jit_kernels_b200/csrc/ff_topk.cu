@@ -205,17 +205,27 @@ int choose_cluster(int device, int32_t B, int64_t L_width, int32_t k) {
 //
 // Clusters of two: 74 of them fit, on all 148 SMs (of eight only 15, on 120), and rows that need no histogram have no
 // use for wider ones (B = 1, 8 Mi columns 19.4 -> 18.6 us, B = 4, 1 Mi, k = 512 15.7 -> 14.7).
-//   * Rows that make their own guess are swept once: split rows of 256 Ki columns take 13.2 us (B = 2), 13.5 (B = 4), 14.1
-//     (B = 8), 16.2 (B = 16), against 15.7 to 22 in clusters of topk_rows_kernel.  The guess needs about 200 hits in the
-//     CTAs' samples (seed_plan), 27 of them from one CTA at most.
-//   * A cooperative launch that is not replayed from a graph starts on a 2.048 us beat behind the kernel in front of it
-//     (12.3, 14.3 or 16.4 us per call where a graph shows 10.2, 13.2 or 14.1), so shorter rows are not split although a
-//     graph would gain: from 128 Ki + 32 k columns up (4 x 256 Ki 16.3 against 15.8 to 17.3 us per call, 8 x 128 Ki
-//     16.4 against 13.2 to 14.2), and with guesses, which leave less to gain, only very long rows or a single row.
+//   * Rows that make their own guess are swept once: split rows of 256 Ki columns take 13.2 us (B = 2), 13.4 (B = 4), 14.8
+//     (B = 8), 17.5 (B = 16) in a graph, against 14.4, 14.5, 17.1 and 23.3 in one cluster each.  The guess needs about 200 hits
+//     in the CTAs' samples (seed_plan), 27 of them from one CTA at most.
+//   * A cooperative launch that is not replayed from a graph starts on a 2.048 us beat behind the kernel in front of it, and
+//     short rows of a ragged batch make no guess (12 ragged rows of 192 Ki bf16 columns 22.7 us split, 15.1 in clusters).
+//     So eager calls and 16-bit scores are split from 256 Ki + 64 k columns up (B = 4, eager, split : clusters, 256 Ki
+//     16.4 : 15.0 us full and 17.1 : 14.9 ragged, 384 Ki 16.6 : 16.8 and 17.4 : 17.2, 512 Ki 16.6 : 18.2 and 16.7 : 17.3),
+//     captured fp32 calls from 128 Ki + 32 k (192 Ki 13.3 : 14.1 full, 14.5 : 14.1 ragged), and so are batches whose clusters
+//     have fewer than eight CTAs (B = 16, 192 Ki, eager 18.8 : 21.2 and 20.4 : 19.6).  With guesses, which leave less to gain,
+//     only very long rows or a single row.
 //   * Rows that have to be swept twice are split if very long, or if one row has the GPU.
 constexpr int64_t kGroupMinWidthSingle = 131072;
 constexpr int64_t kGroupMinWidthHinted = 65536;
 constexpr int64_t kGroupAlwaysWidth = 786432;
+// Whether what is launched on `stream` goes into a graph.
+bool is_captured(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) == cudaSuccess) return status == cudaStreamCaptureStatusActive;
+  (void)cudaGetLastError();   // (the legacy stream beside a capture: the launch will say so)
+  return false;
+}
 // Whether a row of `len` scores makes its own guess on n_share CTAs (the kernel's seed_plan, roughly).
 bool own_guess_likely(int64_t len, int32_t k, int n_share, int per_unit) {
   const double target = k + (k >> 2) + 64;
@@ -225,8 +235,9 @@ bool own_guess_likely(int64_t len, int32_t k, int n_share, int per_unit) {
 }
 // cp: a context-parallel rank's row, which keeps clusters of eight (its merge and the exchange of survivors are
 // laid out for at most 128 CTAs a row).
+// captured: the launch goes into a graph.
 int choose_groups(int device, int32_t B, int64_t L_width, int32_t k, size_t workspace_bytes, int* cluster, bool hinted,
-                  int per_unit = 4, bool cp = false) {
+                  int per_unit, bool cp, bool captured) {
   int g = forced_groups();
   const size_t need = static_cast<size_t>(B) * ff::kWsRowWords * sizeof(uint32_t);
   if (workspace_bytes < need || g == 1 || B < 1) return 1;
@@ -246,8 +257,9 @@ int choose_groups(int device, int32_t B, int64_t L_width, int32_t k, size_t work
     } else if (hinted) {
       worth = worth || (B == 1 && L_width >= kGroupMinWidthHinted) || (B > 4 && g >= *cluster && L_width >= 524288);
     } else {
-      worth = worth || (self_seed_enabled() && L_width >= 131072 + 32 * static_cast<int64_t>(k) &&
-                        own_guess_likely(L_width, k, g * c, per_unit)) ||
+      const int64_t least = (captured && per_unit == 4) || *cluster < 8 ? 131072 + 32 * static_cast<int64_t>(k)
+                                                                         : 262144 + 64 * static_cast<int64_t>(k);
+      worth = worth || (self_seed_enabled() && L_width >= least && own_guess_likely(L_width, k, g * c, per_unit)) ||
               (B == 1 && L_width >= kGroupMinWidthSingle);
     }
     if (!worth) return 1;
@@ -401,33 +413,52 @@ int launch_rows(const ff::TopkParams& p, int shape, cudaStream_t stream, int dty
 }
 
 // Shape of topk_rows_kernel for this batch, or 0: the kernel of ff_topk_kernel.cuh (also whenever a launch shape is
-// forced; `split`: that one would split the row over several clusters).  Measured on B200, k = 2048:
-//   * more rows than SMs: four CTAs of 256 threads per SM (296 rows of 16 Ki: 14.6 us against 18.9 with one CTA of 1024),
-//     unless a second row per SM is all there is and the rows are long (296 rows of 64 Ki: 41 against 38);
-//   * one CTA of 1024 threads: 8.5 us for 4 Ki columns, 9.2 for 16 Ki, 11.4 for 32 Ki, 15.6 for 64 Ki, 23.6 for 128 Ki;
+// forced; `split`: that one would split the row over several clusters; `half`: 16-bit scores).  Measured on B200, k = 2048, us in
+// a graph, full rows N(0, 1) / ragged rows of logits (lengths from 4 Ki up):
+//   * more rows than SMs: four CTAs of 256 threads per SM (296 rows of 16 Ki: 14.6 against 18.9 with one CTA of 1024), unless
+//     the rows are long: at four to an SM they do not stay in L2 for the second sweep (297 rows of 128 Ki 100.8 / 71.0 against
+//     79.5 / 48.1, of 256 Ki 188 / 137 against 150 / 74; 900 rows of 128 Ki bf16 152.6 / 99.0 against 159.1 / 108.0, of 160 Ki
+//     192.9 / 120.7 against 185.0 / 120.1), and a second row per SM is all there is up to 296 rows (64 Ki: 41 against 38);
+//   * one CTA of 1024 threads: 8.5 us for 4 Ki columns, 9.2 for 16 Ki, 11.4 for 32 Ki, 15.6 for 64 Ki, 23.6 for 128 Ki; beyond
+//     half as many rows as SMs at any width (75 rows of 64 Ki 18.0 / 16.8 against 26.7 / 26.6, of 1 Mi 163 / 136 against 184 / 237);
 //   * a cluster of 512-thread CTAs, four: 10.7 us for 32 Ki, 12.4 for 64 Ki, 15.3 for 128 Ki; eight: 11.2, 11.2, 12.9.
 //     Scores that spread over many digits, as N(0, 1) does, take 1 us more with eight and 6 us more with sixteen, which
 //     are not used.  As many as the device holds with an SM for each CTA (two on an SM slow each other down: 32 rows of
-//     64 Ki 13.8 us with four, 18.5 with eight), but four also for long rows of up to as many as fit two on an SM
-//     (64 ragged rows of 128 Ki: 20.8 us against 23.5 in clusters of two of the other kernel);
+//     64 Ki 13.8 us with four, 18.5 with eight), eight up to 160 Ki (4 rows of 160 Ki 15.3 / 13.4 against 14.1 / 14.2, of
+//     256 Ki 17.2 / 15.3 against 14.5 / 14.5), but four also for long rows of up to as many as fit two on an SM (against
+//     clusters of two of the other kernel: 64 rows of 128 Ki 24.5 / 21.6 : 25.3 / 24.3, of 256 Ki 36.2 / 30.1 : 36.9 / 33.2, 37
+//     of 512 Ki 50.6 / 40.7 : 56.4 / 57.8, 64 of 512 Ki 60.4 / 43.2 : 58.6 / 72.7; bf16 of 192 Ki 27.3 / 24.6 : 26.8 / 25.1, of 256
+//     Ki 31.6 / 29.6 : 30.1 / 28.1, of 384 Ki 38.1 / 37.7 : 38.2 / 49.1);
 //   * ff_topk_kernel.cuh: 13.8 us for 64 Ki, 14.3 for 128 Ki, 15.0 for 256 Ki, 16.8 for 512 Ki (sixteen CTAs; 12.4, 12.5 and
-//     12.9 split over clusters), 24.7 for 64 rows of 128 Ki; with guesses it is the faster one from 48 Ki columns up.
-int choose_rows_shape(int device, int32_t B, int64_t L_width, bool hints, bool split) {
+//     12.9 split over clusters);
+//   * with guesses, one CTA against that kernel: 4 rows of 32 Ki 9.6 : 9.7, of 40,000 10.5 : 9.8, of 24 Ki bf16 10.5 : 9.9;
+//     16 of 48 Ki 10.7 : 11.0, bf16 of 40,000 11.7 : 11.4; 32 of 48 Ki 11.1 : 11.2, of 64 Ki 13.4 : 12.2, bf16 of 48 Ki 12.0 : 11.6;
+//     64 of 96 Ki 16.7 : 17.3, bf16 17.4 : 16.8; 75 of 256 Ki 31.8 : 34.9, bf16 of 192 Ki 26.4 : 25.6, of 256 Ki 31.1 : 28.8;
+//     297 of 256 Ki 95.7 (256 threads 104.4) : 99.5, bf16 87.3 (96.3) : 79.6, of 192 Ki 46.0 : 48.1 ragged.
+int choose_rows_shape(int device, int32_t B, int64_t L_width, bool hints, bool split, bool half) {
   if (forced_cluster() != 0 || forced_groups() != 0) return 0;
   const int sms = g_sm_count[device];
-  if (B > sms) return B <= 2 * sms && L_width > 49152 ? 1024 : 256;
+  if (hints && half && 2 * B > sms && L_width > (B > 2 * sms ? 229376 : 180224)) return 0;
+  if (B > 2 * sms) return L_width > (hints ? 229376 : B <= 4 * sms ? 114688 : 163840) ? 1024 : 256;
+  if (B > sms) return L_width > 49152 ? 1024 : 256;
   const int* one_per_sm = g_active_clusters[device];   // of 1, 2, 4, 8, 16 CTAs
   if (2 * B > sms) return 1024;
-  if (hints) return L_width <= (B <= 8 ? 40960 : B <= 18 ? 49152 : B <= 37 ? 65536 : 98304) ? 1024 : 0;
+  if (hints) {
+    if (B <= 8) return L_width <= (half ? 20480 : 36864) ? 1024 : 0;
+    if (B <= 18) return L_width <= (half ? 36864 : 49152) ? 1024 : 0;
+    if (B <= one_per_sm[2]) return L_width <= (half ? 40960 : 53248) ? 1024 : 0;
+    return L_width <= (half ? 81920 : 98304) ? 1024 : 0;
+  }
   if (split || L_width > 524288) return 0;
   if (B > one_per_sm[2]) {
     if (L_width <= 81920) return 1024;
-    return L_width <= 131072 && B <= g_rows_clusters_of_4[device] ? -40512 : 0;
+    if (B > g_rows_clusters_of_4[device]) return 0;
+    if (half) return L_width <= 196608 || L_width > 327680 ? -40512 : 0;
+    return L_width <= (B <= 56 ? 524288 : 393216) ? -40512 : 0;
   }
   if (L_width <= (B > one_per_sm[3] ? 32768 : 20480)) return 1024;
   if (L_width <= (B > one_per_sm[3] ? 131072 : 40960)) return -40512;
-  if (B > one_per_sm[3]) return 0;
-  return -80512;
+  return B <= one_per_sm[3] && L_width <= 163840 ? -80512 : 0;
 }
 
 // Built-in scratch for ff_topk_launch_static: enough for FF_TOPK_STATIC_MAX_ROWS
@@ -515,8 +546,8 @@ int ff_topk_policy_launch_shape(int32_t B, int64_t L_width, int32_t k, int32_t h
   int cluster = choose_cluster(device, B, L_width, k);
   int groups = 1;
   if (has_workspace != 0)
-    groups = choose_groups(device, B, L_width, k, ff_topk_workspace_bytes(B, L_width, k), &cluster, hinted != 0);
-  if (const int shape = choose_rows_shape(device, B, L_width, hinted != 0, groups > 1)) {
+    groups = choose_groups(device, B, L_width, k, ff_topk_workspace_bytes(B, L_width, k), &cluster, hinted != 0, 4, false, false);
+  if (const int shape = choose_rows_shape(device, B, L_width, hinted != 0, groups > 1, false)) {
     cluster = shape_cluster(shape);
     groups = 1;
   }
@@ -612,10 +643,12 @@ int transform_launch_impl(const void* scores_any, int dtype, int64_t row_stride,
   }
   int cluster = choose_cluster(device, B, L_width, k);
   if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
-    p.groups = choose_groups(device, B, L_width, k, workspace_bytes, &cluster, hint_in != nullptr, dtype == FF_DTYPE_F32 ? 4 : 8);
+    p.groups = choose_groups(device, B, L_width, k, workspace_bytes, &cluster, hint_in != nullptr, dtype == FF_DTYPE_F32 ? 4 : 8, false,
+                             is_captured(static_cast<cudaStream_t>(stream)));
     p.workspace = static_cast<uint32_t*>(workspace);
   }
-  if (const int shape = choose_rows_shape(device, B, L_width, hint_in != nullptr || hint_out != nullptr, p.groups > 1))
+  if (const int shape = choose_rows_shape(device, B, L_width, hint_in != nullptr || hint_out != nullptr, p.groups > 1,
+                                          dtype != FF_DTYPE_F32))
     return launch_rows(p, shape, static_cast<cudaStream_t>(stream), dtype);
   return launch<false>(p, cluster, static_cast<cudaStream_t>(stream), dtype);
 }
@@ -705,8 +738,9 @@ int ff_topk_launch_static(const float* scores, int64_t row_stride, const int32_t
   p.epilogue = FF_EPILOGUE_INDEX;
   p.status = status;
   int cluster = choose_cluster(device, B, L_width, k);
-  p.groups = choose_groups(device, B, L_width, k, FF_TOPK_STATIC_MAX_ROWS * row_bytes, &cluster, false);
-  if (const int shape = choose_rows_shape(device, B, L_width, false, p.groups > 1))
+  p.groups = choose_groups(device, B, L_width, k, FF_TOPK_STATIC_MAX_ROWS * row_bytes, &cluster, false, 4, false,
+                           is_captured(static_cast<cudaStream_t>(stream)));
+  if (const int shape = choose_rows_shape(device, B, L_width, false, p.groups > 1, false))
     return launch_rows(p, shape, static_cast<cudaStream_t>(stream), FF_DTYPE_F32);
   p.workspace = scratch;
   if (p.groups > 1) {
@@ -748,7 +782,7 @@ int ff_topk_cp_local(const float* scores, int64_t row_stride, const int32_t* len
   p.status = status;
   int cluster = choose_cluster(device, B, L_width, k);
   if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
-    p.groups = choose_groups(device, B, L_width, k, workspace_bytes, &cluster, false, 4, true);
+    p.groups = choose_groups(device, B, L_width, k, workspace_bytes, &cluster, false, 4, true, false);
     p.workspace = static_cast<uint32_t*>(workspace);
   }
   return launch<false>(p, cluster, static_cast<cudaStream_t>(stream));
@@ -1014,7 +1048,7 @@ int cp_fill_params(FfCpExchange* ex, const float* scores, int64_t row_stride, co
   p.hint_out = hint_out;
   int cluster = choose_cluster(device, ex->B, L_width, ex->k);
   if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0) {
-    p.groups = choose_groups(device, ex->B, L_width, ex->k, workspace_bytes, &cluster, hint_in != nullptr, 4, true);
+    p.groups = choose_groups(device, ex->B, L_width, ex->k, workspace_bytes, &cluster, hint_in != nullptr, 4, true, false);
     p.workspace = static_cast<uint32_t*>(workspace);
   }
   *out = p;

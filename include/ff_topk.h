@@ -321,7 +321,9 @@ int32_t ff_topk_policy_cluster_size(int32_t B, int64_t L_width, int32_t k);
  * (hinted != 0) uses for (B, L_width, k) on the current device: out2[0] = CTAs
  * per cluster, out2[1] = clusters per row (more than one only with workspace of
  * ff_topk_workspace_bytes; pass has_workspace = 0 for a call without).  The
- * grid is B * out2[0] * out2[1] CTAs.  Plays the role of reading the reference's
+ * grid is B * out2[0] * out2[1] CTAs.  A captured launch of fp32 scores may split rows of
+ * small batches where this one does not (from 128 Ki + 32 k instead of 256 Ki + 64 k columns: a
+ * cooperative launch outside a graph starts late).  Plays the role of reading the reference's
  * split policy off its launcher (topk_indexer_radix.cu:1309-1321). */
 int ff_topk_policy_launch_shape(int32_t B, int64_t L_width, int32_t k, int32_t has_workspace, int32_t hinted,
                                 int32_t* out2);

@@ -430,3 +430,46 @@ def test_launch_shape_forced_by_the_environment(ff, oracle, monkeypatch, variabl
     assert tuple(got) == shape
     s = torch.randn((B, L), generator=torch.Generator().manual_seed(3))
     run_case(ff, oracle, s, torch.full((B,), L, dtype=torch.int32), k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rows_of_small_batches_are_split_where_the_call_gains(ff, oracle, dtype):
+    """4 x 256 Ki: in one cluster per row call by call (a split launch would start on a 2 us beat) and with 16-bit scores
+    (whose ragged batches lose), split when it is captured; the grid is counted by the CTAs that stamp their start."""
+    import ctypes
+    from flash_float_jit_kernels_b200 import _lib
+    pkg, lib = ff
+    lib.ff_topk_set_cluster_override(0)
+    B, L, k, dev = 4, 262144, 2048, torch.device("cuda:0")
+    shape = (ctypes.c_int32 * 2)()
+    assert lib.ff_topk_policy_launch_shape(B, L, k, 1, 0, shape) == 0
+    assert shape[0] >= 8 and shape[1] == 1
+    s = torch.randn((B, L), generator=torch.Generator().manual_seed(1)).to(dtype)
+    lengths = torch.full((B,), L, dtype=torch.int32)
+    exp = oracle.topk_c(s.float().numpy(), lengths.numpy(), k)
+    sd, ld = s.to(dev), lengths.to(dev)
+    out = torch.empty((B, k), dtype=torch.int32, device=dev)
+    pkg.fast_topk_v3(sd, ld, k, out=out)
+    stamps = torch.zeros((B * 1024, _lib.TRACE_SLOTS), dtype=torch.int64, device=dev)
+    torch.cuda.synchronize()
+    grids = []
+    try:
+        lib.ff_topk_set_trace_buffer(stamps.data_ptr())
+        pkg.fast_topk_v3(sd, ld, k, out=out)
+        torch.cuda.synchronize()
+        grids.append(int((stamps[:, 0] != 0).sum()))
+        stamps.zero_()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            pkg.fast_topk_v3(sd, ld, k, out=out)
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        grids.append(int((stamps[:, 0] != 0).sum()))
+    finally:
+        lib.ff_topk_set_trace_buffer(None)
+    assert np.array_equal(out.cpu().numpy(), exp)
+    one_cluster = B * shape[0]
+    assert grids[0] == one_cluster
+    assert grids[1] == one_cluster if dtype == torch.bfloat16 else grids[1] > one_cluster

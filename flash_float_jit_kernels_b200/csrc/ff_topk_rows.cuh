@@ -9,12 +9,14 @@
 //   finish    counting sort of the survivors in one pass of bins: a survivor's bin is its EXPECTED rank
 //             (elements above its digit + its position inside the digit, interpolated), at two bins
 //             per survivor, so that buckets hold one or two entries whatever the scores' distribution;
-//             exact rank inside the bucket by counting; indices leave through shared memory
+//             laid out bucket by bucket they are in order but for neighbours, and every slot is moved by the pairs
+//             of neighbours that are not; indices leave through shared memory
 //
-// What bounds it: batches of many rows keep issue slots and the shared-memory pipe 62 % busy each (4,096 rows of 5,461
-// scores, k = 2048: 103.5 us, 20,000 warp instructions and 4,800 shared-memory wavefronts per row; the kernel of
-// ff_topk_kernel.cuh, one row per SM, took 455 us); a single row is a chain of eight phases, 9.3 us for 16 Ki scores
-// (12.5 us in a cluster of sixteen CTAs of the other kernel).  Hence 64 registers and 36 KiB per row, four rows on an SM.
+// What bounds it: batches of many rows keep issue slots and the shared-memory pipe about 60 % busy each (4,096 rows of 5,461
+// scores, k = 2048: 88.2 us; 104.3 with survivors ranked by a walk of each one's bucket, sixteen scores to a group of the sweeps and
+// the cut worked out by every thread; the kernel of ff_topk_kernel.cuh, one row per SM, took 455); a single row is a chain of
+// eight phases, 8.7 us for 16 Ki scores (9.1; 12.5 in a cluster of sixteen CTAs of the other kernel).  Hence 64 registers and
+// 40 KiB per row, four rows on an SM.
 #pragma once
 
 #include "ff_topk_kernel.cuh"
@@ -48,13 +50,16 @@ constexpr int kRowsBins = 1 << kRowsBits;
 constexpr int kRowsShift = 32 - kRowsBits;
 
 // Shared memory of a CTA whose list holds `cap` survivors, in two regions:
-//   histogram, then the bucketed survivors (32 bits each)
+//   histogram, then the survivors bucket by bucket (64 bits each)
 //   list (64 bits each), then two finish bins per survivor (32 bits each), then the ranked positions
 // and in a cluster the row's histogram and this CTA's own list behind them.
-__host__ __device__ constexpr int rows_smem_bytes(int cap, bool cluster) {
-  return (kRowsBins * 4 + cap * 8) * (cluster ? 2 : 1);
+constexpr int kRankPad = 8;                       // slots in front of and behind the sorted survivors
+__host__ __device__ constexpr int rows_table_bytes(int cap) {
+  return kRowsBins * 4 > (cap + 2 * kRankPad) * 8 ? kRowsBins * 4 : (cap + 2 * kRankPad) * 8;
 }
-static_assert(kRowsBins >= kSortCap, "the bucketed survivors take the histogram's place");
+__host__ __device__ constexpr int rows_smem_bytes(int cap, bool cluster) {
+  return rows_table_bytes(cap) + cap * 8 + (cluster ? kRowsBins * 4 + cap * 8 : 0);
+}
 
 // ---- a row shared by the CTAs of a cluster ----
 __device__ __forceinline__ uint32_t cluster_size() {
@@ -99,14 +104,17 @@ struct RowsShared {
   int warp_tot[3][32];
   int t, above, total;     // threshold digit, elements above it, elements at or above it
   int max_bin;             // largest bin at or above the threshold
+  uint32_t cut;            // key of the cut inside the threshold digit,
+  int keep;                // and how many of the digit's scores are meant to be kept
   int count;               // survivors listed
   int base;                // clusters: this CTA's first slot in the row's list
   int reserved;            // clusters, first CTA: slots of the row's list given out
   int gathered;            // clusters: survivors of all CTAs
-  uint32_t value_bits;     // OR of the survivors' score bits
+  uint32_t value_bits[2];  // OR of the survivors' score bits: of every thread's first one (16-bit scores: all), of the others
   uint32_t kmin, kmax;     // bounds of the survivors' keys (rebuilt bins only)
   int last_pos;            // a crowded lowest bin of those: last position,
   uint32_t low_bits;       // and OR of the keys' distances from the smallest
+  uint32_t max_bucket;     // survivors in the largest finish bin
 };
 
 // Sum of v over all threads of higher index; `total`: over all threads.  One barrier; calls that
@@ -171,10 +179,10 @@ __device__ __forceinline__ float approximate_sqrt(float x) {
 // the way down lie b x + a x^2 of them, b = (c0 + c1) / 2 and a = (c0 - c1) / 2.
 struct DigitDensity {
   float a, b;
-  __device__ __forceinline__ DigitDensity(const uint32_t* packed, int t, int in_bin) {
+  __device__ __forceinline__ DigitDensity(int t, int in_bin, int in_next) {
     const float c0 = static_cast<float>(in_bin);
     const int up = t + 1;
-    float c1 = static_cast<float>((packed[rows_raw_of(up)] & ((1u << kPackShift) - 1u)) >> 1);
+    float c1 = static_cast<float>(in_next);
     if ((up & 7) == 0) c1 *= up >= kRowsBins / 2 ? 0.5f : 2.f;   // the next digit spans a step of another width
     c1 = fminf(c1, 3.f * c0);
     a = 0.5f * (c0 - c1);
@@ -208,11 +216,14 @@ __device__ __forceinline__ uint32_t cut_at(float x, int keep, int in_bin, int& s
   return all ? 0u : static_cast<uint32_t>((1.f - x) * static_cast<float>(1 << kRowsShift)) & ~(kKeyStep<T> - 1u);
 }
 
-// Suffix scan of the bins in monotone order (raw: the array is in rows_raw_digit() order).  Every non-empty bin
+// Suffix scan of the bins in monotone order (CUT: the array is in rows_raw_digit() order).  Every non-empty bin
 // with fewer than `limit` elements above it is packed in place, and the bin that reaches the limit
 // is published as sh.t with its counts.
-template <int NT>
-__device__ __forceinline__ void pack_bins(uint32_t* hist, bool raw, int limit, RowsShared& sh, int* warp_tot) {
+// CUT: by the thread that finds it, which calls `crossing(t, above, in_bin, in_next)` with the count of the next digit up; it returns
+// the count that the bin is packed with.  (Without: nothing is published.)
+template <int NT, bool CUT, typename F>
+__device__ __forceinline__ void pack_bins(uint32_t* hist, int limit, RowsShared& sh, int* warp_tot, F&& crossing) {
+  constexpr bool raw = CUT;
   constexpr int per = kRowsBins / NT;
   // whole 16-byte quads per thread, their rotation a mask, and a divisor of the 32 banks: 4,096 bins over 192 threads are
   // 21 each, at 4-byte addresses
@@ -221,6 +232,8 @@ __device__ __forceinline__ void pack_bins(uint32_t* hist, bool raw, int limit, R
   const int m0 = tid * per;
   const bool up = !raw || m0 >= kRowsBins / 2;   // the thread's bins lie in ascending order
   const int base = !raw ? m0 : up ? m0 - kRowsBins / 2 : kRowsBins - per - m0;
+  int next = 0;                                  // what the digit above the thread's holds, while nothing is packed
+  if (raw && tid < NT - 1) next = static_cast<int>(hist[rows_raw_of(m0 + per)]);
   int local = 0;
 #pragma unroll
   for (int j = 0; j < per / 4; ++j) {            // rotated so that eight threads read eight different bank groups
@@ -240,7 +253,7 @@ __device__ __forceinline__ void pack_bins(uint32_t* hist, bool raw, int limit, R
       c[4 * q + 2] = v.z;
       c[4 * q + 3] = v.w;
     }
-    int largest = 0;
+    int largest = 0, t = -1, above = 0, in_bin = 0, in_next = 0;
 #pragma unroll
     for (int i = 0; i < per; ++i) {              // from the thread's largest digit down
       const int n = static_cast<int>(up ? c[per - 1 - i] : c[i]);
@@ -248,24 +261,38 @@ __device__ __forceinline__ void pack_bins(uint32_t* hist, bool raw, int limit, R
         hist[base + (up ? per - 1 - i : i)] = packed_bin(running, n);
         largest = max(largest, n);
         if (running + n >= limit) {
-          sh.t = m0 + per - 1 - i;
-          sh.above = running;
-          sh.total = running + n;
+          t = m0 + per - 1 - i;
+          above = running;
+          in_bin = n;
+          in_next = next;
         }
         running += n;
       }
+      next = n;
     }
-    atomicMax(&sh.max_bin, largest);
+    if (CUT) atomicMax(&sh.max_bin, largest);
+    if (CUT && t >= 0) {
+      sh.t = t;
+      sh.above = above;
+      sh.total = above + in_bin;
+      hist[rows_raw_of(t)] = packed_bin(above, crossing(t, above, in_bin, in_next));
+    }
   }
   __syncthreads();
 }
 
-// A row's scores in groups of 16 per thread (four units of 4 or two units of 8), NT threads apart.
+// Scores of a group: the more, the less a score's share of the second sweep's slots is (prefill batches of 5.5 and 16 Ki scores:
+// sixteen 95.1 and 37.7 us, 24 89.9 and 35.8, 32 92.0 and 40.0 with spilled registers; 32 rows of 20,000, k = 1024, one CTA
+// each: 9.4 and 8.9).  A cluster's CTAs have few scores each (8 x 64 Ki 11.9 with sixteen, 12.3 with 24), and the kernel with
+// guesses has no registers for more.
+__host__ __device__ constexpr int rows_group(bool cluster, bool hints) { return cluster || hints ? 16 : 24; }
+
+// A row's scores in groups of S per thread (units of 4 or 8), NT threads apart.
 // FULL: every unit of the group is inside the row.
-template <typename T, int NT>
+template <typename T, int NT, int S>
 struct RowGroup {
   static constexpr int kPU = Elem<T>::kPerUnit;
-  static constexpr int kUnits = 16 / kPU;
+  static constexpr int kUnits = S / kPU;
   static constexpr int kStep = NT * kUnits;
   uint4 w[kUnits];
   template <bool FULL>
@@ -303,7 +330,7 @@ struct RowGroup {
 // goes to the finish.
 __host__ __device__ constexpr int rows_level_bits(int l) { return l <= 2 ? 10 : l == 5 ? 10 : 11; }
 __host__ __device__ constexpr int rows_level_shift(int l) { return l == 0 ? 52 : l == 1 ? 42 : l == 2 ? 32 : l == 3 ? 21 : l == 4 ? 10 : 0; }
-template <typename T, int NT, bool CLUSTER>
+template <typename T, int NT, int S, bool CLUSTER>
 __device__ __noinline__ uint64_t deeper_digits(const Chunk<T>& c, uint32_t* hist, uint32_t* merged, int k, int cap,
                                                RowsShared& sh, int32_t* status) {
   const int tid = threadIdx.x;
@@ -326,12 +353,12 @@ __device__ __noinline__ uint64_t deeper_digits(const Chunk<T>& c, uint32_t* hist
       if ((comp >> above_shift) == prefix) atomicAdd(&hist[static_cast<uint32_t>(comp >> shift) & mask], 1u);
     };
 #pragma unroll 1
-    for (int u0 = c.fb; u0 < c.fe; u0 += RowGroup<T, NT>::kStep) {
-      RowGroup<T, NT> g;
+    for (int u0 = c.fb; u0 < c.fe; u0 += RowGroup<T, NT, S>::kStep) {
+      RowGroup<T, NT, S> g;
       g.load(c, u0);
-      const int first = RowGroup<T, NT>::position(c, u0);
+      const int first = RowGroup<T, NT, S>::position(c, u0);
       g.template each<false>(c, u0, [&](float x, int e) {
-        if (!(x < vmin)) count_one(x, first + RowGroup<T, NT>::distance(e));
+        if (!(x < vmin)) count_one(x, first + RowGroup<T, NT, S>::distance(e));
       });
     }
     float x = 0.f;
@@ -373,34 +400,39 @@ __device__ __noinline__ uint64_t deeper_digits(const Chunk<T>& c, uint32_t* hist
   }
 }
 
+// Inclusive sum over the warp's lanes of lower index, two instructions a step.
+__device__ __forceinline__ int warp_inclusive(int v) {
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1)
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .s32 t;\n\tshfl.sync.up.b32 t|p, %0, %1, 0, 0xffffffff;\n\t@p add.s32 %0, %0, t;\n\t}" : "+r"(v) : "r"(off));
+  return v;
+}
+
 // Sweep 2: every score not below vmin (EXACT: whose composite is not below floor_comp) goes to the list.
-// `first` is the row's first group, still in registers.  A warp takes 512 scores at a time: a scan over the lanes' hit
+// `g` is the row's first group, still in registers.  A warp takes a group of its lanes' at a time: a scan over the lanes' hit
 // counts, one shared atomic for the warp's slots, and predicated stores (no hit mask: testing a score
 // again is one instruction, picking its bit out of a mask three).
-template <typename T, int NT, int CAP, bool EXACT>
-__device__ __forceinline__ void collect_row(const Chunk<T>& c, const RowGroup<T, NT>* first, float vmin, uint64_t floor_comp,
+template <typename T, int NT, int S, int CAP, bool EXACT>
+__device__ __forceinline__ void collect_row(const Chunk<T>& c, RowGroup<T, NT, S>& g, float vmin, uint64_t floor_comp,
                                             RowList<CAP> list, RowsShared& sh) {
-  using Group = RowGroup<T, NT>;
+  using Group = RowGroup<T, NT, S>;
   const int lane = threadIdx.x & 31;
   const uint32_t list_at = smem_addr(list.x);
-  auto is_hit = [&](float x, int pos) { return !(x < vmin) && (!EXACT || make_comp(fast_key(x), pos) >= floor_comp); };
-  auto take = [&](const Group& g, int u0, auto full) {
+  auto is_hit = [&](float x, int pos) { return !(x < vmin) && make_comp(fast_key(x), pos) >= floor_comp; };   // (EXACT)
+  auto take = [&](int u0, auto full) {
     constexpr bool FULL = decltype(full)::value;
     const int pos0 = Group::position(c, u0);
     int n = 0;
-    g.template each<FULL>(c, u0, [&](float x, int e) { n += is_hit(x, pos0 + Group::distance(e)) ? 1 : 0; });
-    int incl = n;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += v;
-    }
-    const int total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total == 0) return;
+    g.template each<FULL>(c, u0, [&](float x, int e) {
+      if constexpr (EXACT) n += is_hit(x, pos0 + Group::distance(e)) ? 1 : 0;
+      else asm("{\n\t.reg .pred p;\n\tsetp.geu.f32 p, %1, %2;\n\t@p add.s32 %0, %0, 1;\n\t}" : "+r"(n) : "f"(x), "f"(vmin));
+    });
+    const int incl = warp_inclusive(n);
     int base = 0;
-    if (lane == 0) base = atomicAdd(&sh.count, total);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base + total > CAP) return;
+    if (lane == 31 && incl != 0) base = atomicAdd(&sh.count, incl);
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (total == 0 || base + total > CAP) return;
     uint32_t at = list_at + 8u * static_cast<uint32_t>(base + incl - n);
     g.template each<FULL>(c, u0, [&](float x, int e) {
       const int pos = pos0 + Group::distance(e);
@@ -418,15 +450,16 @@ __device__ __forceinline__ void collect_row(const Chunk<T>& c, const RowGroup<T,
     });
   };
 #pragma unroll 1
-  for (int u0 = c.fb; u0 < c.fe; u0 += Group::kStep) {
-    Group g;
-    if (first != nullptr && u0 == c.fb) g = *first; else g.load(c, u0);
-    if (u0 + Group::kStep <= c.fe) take(g, u0, std::true_type{}); else take(g, u0, std::false_type{});
+  for (int u0 = c.fb;;) {
+    if (u0 + Group::kStep <= c.fe) take(u0, std::true_type{}); else take(u0, std::false_type{});
+    u0 += Group::kStep;
+    if (u0 >= c.fe) break;
+    g.load(c, u0);
   }
   if (c.head || c.tail) {   // (uniform)
     float x = 0.f;
     const int pos = partial_element(c, x);
-    if (pos >= 0 && is_hit(x, pos)) {
+    if (pos >= 0 && !(x < vmin) && (!EXACT || is_hit(x, pos))) {
       const int at = atomicAdd(&sh.count, 1);
       if (at < CAP) {
         list.put(at, x, pos);
@@ -442,9 +475,9 @@ __device__ __forceinline__ float score_at(const T* p) {
   if constexpr (Elem<T>::kPerUnit == 4) return __ldg(p);
   else return Elem<T>::from_bits16(__ldg(reinterpret_cast<const unsigned short*>(p)));
 }
-template <typename T, int NT, int CAP>
+template <typename T, int NT, int S, int CAP>
 __device__ __noinline__ void collect_row_sparse(const Chunk<T>& c, float vmin, RowList<CAP> list, RowsShared& sh) {
-  using Group = RowGroup<T, NT>;
+  using Group = RowGroup<T, NT, S>;
   const int lane = threadIdx.x & 31;
 #pragma unroll 1
   for (int u0 = c.fb; u0 < c.fe; u0 += Group::kStep) {
@@ -482,13 +515,17 @@ __device__ __noinline__ void collect_row_sparse(const Chunk<T>& c, float vmin, R
   }
 }
 
-template <typename T, int NT, int CAP>
+template <typename T, int NT, int S, int CAP>
 __device__ __noinline__ void collect_row_again(const Chunk<T>& c, float vmin, RowList<CAP> list, RowsShared& sh) {
-  collect_row<T, NT, CAP, false>(c, nullptr, vmin, 0ull, list, sh);
+  RowGroup<T, NT, S> g;
+  g.load(c, c.fb);
+  collect_row<T, NT, S, CAP, false>(c, g, vmin, 0ull, list, sh);
 }
-template <typename T, int NT, int CAP>
+template <typename T, int NT, int S, int CAP>
 __device__ __noinline__ void collect_row_exact(const Chunk<T>& c, uint64_t floor_comp, RowList<CAP> list, RowsShared& sh) {
-  collect_row<T, NT, CAP, true>(c, nullptr, prefilter_value(static_cast<uint32_t>(floor_comp >> 32)), floor_comp, list, sh);
+  RowGroup<T, NT, S> g;
+  g.load(c, c.fb);
+  collect_row<T, NT, S, CAP, true>(c, g, prefilter_value(static_cast<uint32_t>(floor_comp >> 32)), floor_comp, list, sh);
 }
 
 // How a survivor becomes an expected rank: its digit picks a packed bin (elements above, elements in it), and
@@ -520,6 +557,77 @@ __device__ __forceinline__ uint32_t expected_rank2(uint32_t packed, uint32_t dep
   return (packed >> kPackShift) + __umulhi(depth, packed & ((1u << kPackShift) - 1u));
 }
 
+// Consecutive slots that a thread ranks at a time.  Odd, so that 64-bit loads at that distance do not meet in a bank; five where
+// batches of many rows keep the SM busy (4,096 prefill rows 89.7 us, three 90.2, one 94.8), three where one row's latency counts
+// (8 x 64 Ki 11.7 us, five 11.9, one 12.1).
+__host__ __device__ constexpr int rows_block_slots(int per) { return per >= 8 ? 5 : 3; }
+
+// Ranks n survivors that lie in order but for neighbours at most W slots apart: a thread takes BLOCK consecutive slots and the
+// W on either side, compares every pair that is that close, and moves a survivor's slot by the pairs that are not in order.
+// No loop over buckets, no look-up of their ends, and every load consecutive.  (W slots in front of and behind the n hold
+// the smallest and the largest word.)
+template <int NT, int BLOCK, int W>
+__device__ __forceinline__ void rank_blocks(const uint64_t* sorted, int n, int32_t* ranked) {
+  static_assert(BLOCK % 2 == 1 && W <= kRankPad, "conflict-free loads, inside the padding");
+#pragma unroll 1
+  for (int s0 = static_cast<int>(threadIdx.x) * BLOCK; s0 < n; s0 += NT * BLOCK) {
+    uint64_t e[BLOCK + 2 * W];
+#pragma unroll
+    for (int i = 0; i < BLOCK + 2 * W; ++i) e[i] = sorted[s0 - W + i];
+    int rank[BLOCK];
+#pragma unroll
+    for (int i = 0; i < BLOCK; ++i) rank[i] = s0 + i;
+#pragma unroll
+    for (int i = 0; i < BLOCK + W; ++i) {
+#pragma unroll
+      for (int j = i + 1; j <= i + W; ++j) {
+        if (j >= W && j < BLOCK + 2 * W && (i >= W || j < BLOCK + W)) {
+          const bool swapped = e[j] < e[i];
+          if (i >= W && i < BLOCK + W) rank[i - W] += swapped ? 1 : 0;
+          if (j < BLOCK + W) rank[j - W] -= swapped ? 1 : 0;
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < BLOCK; ++i)
+      if (s0 + i < n) ranked[rank[i]] = static_cast<int32_t>(static_cast<uint32_t>(e[W + i]));
+  }
+}
+
+// The same where buckets are larger (blocks of equal neighbours): every slot looks its bucket up and counts in it.  (The bins hold
+// the ends of their buckets; the ranked positions take their place.)
+template <int NT, int PER>
+__device__ __noinline__ void rank_crowded(const uint64_t* sorted, const uint32_t* bins, int n_bins, int n, int32_t* ranked, int32_t* status) {
+  struct { int32_t* status; } p = {status};   // (for the bounds checks)
+  uint32_t rank[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const uint32_t slot = threadIdx.x + static_cast<uint32_t>(j * NT);
+    if (slot < static_cast<uint32_t>(n)) {
+      int b = 0, b_last = n_bins - 1;   // the first bin that ends behind the slot
+#pragma unroll 1
+      while (b < b_last) {
+        const int mid = (b + b_last) >> 1;
+        if (bins[mid] > slot) b_last = mid; else b = mid + 1;
+      }
+      const uint64_t own = sorted[slot];
+      const uint32_t first = b == 0 ? 0u : bins[b - 1], end = bins[b];
+      rank[j] = first;
+      if (FF_IN_RANGE(p, static_cast<int>(end) - 1, PER * NT, 17)) {
+#pragma unroll 1
+        for (uint32_t q = first; q < end; ++q) rank[j] += sorted[q] < own ? 1u : 0u;
+      }
+    }
+  }
+  __syncthreads();   // the bins have been read
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int slot = static_cast<int>(threadIdx.x) + j * NT;
+    if (slot < n && FF_IN_RANGE(p, rank[j], PER * NT, 18)) ranked[rank[j]] = static_cast<int32_t>(static_cast<uint32_t>(sorted[slot]));
+  }
+  (void)p;
+}
+
 // PER: survivors a thread holds in the finish (the list takes PER * NT); CTAS: CTAs per SM it is compiled for.
 // CLUSTER: a thread-block cluster per row.  Each CTA sweeps its share, its counts are added to every CTA's merged
 // histogram, all find the same cut, and their survivors meet in the first CTA, which finishes the row alone.
@@ -529,12 +637,13 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   static_assert(!(HINTS && CLUSTER), "rows with guesses have one CTA");
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ RowsShared sh;
-  using Group = RowGroup<T, NT>;
+  constexpr int kGroup = rows_group(CLUSTER, HINTS);
+  using Group = RowGroup<T, NT, kGroup>;
   constexpr int kPU = Elem<T>::kPerUnit;
   constexpr int kCap = PER * NT;
   uint32_t* hist = reinterpret_cast<uint32_t*>(smem);
-  uint32_t* bucketed = hist;                                                 // depths, bucket by bucket
-  const RowList<kCap> list = {reinterpret_cast<float*>(smem + kRowsBins * 4)};
+  uint64_t* sorted = reinterpret_cast<uint64_t*>(smem) + kRankPad;           // kCap survivors, bucket by bucket
+  const RowList<kCap> list = {reinterpret_cast<float*>(smem + rows_table_bytes(kCap))};
   uint32_t* bins = reinterpret_cast<uint32_t*>(list.x);                      // 2 * kCap finish bins
   int32_t* ranked = reinterpret_cast<int32_t*>(list.x);                      // kCap positions
   uint32_t* merged = CLUSTER ? reinterpret_cast<uint32_t*>(list.x + 2 * kCap) : hist;
@@ -556,11 +665,12 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     sh.total = 0;
     sh.max_bin = 0;
     sh.count = 0;
-    sh.value_bits = 0u;
+    sh.value_bits[0] = sh.value_bits[1] = 0u;
     sh.kmin = 0xffffffffu;
     sh.kmax = 0u;
     sh.last_pos = 0;
     sh.low_bits = 0u;
+    sh.max_bucket = 0u;
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -718,8 +828,12 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
         header[0] = header[1] = 0u;   // empty for the producer's next launch
       }
     } else if (use) {
-      if (sparse) collect_row_sparse<T, NT, kCap>(chunk, hint, own_list, sh);
-      else collect_row<T, NT, kCap, false>(chunk, nullptr, hint, 0ull, own_list, sh);
+      if (sparse) collect_row_sparse<T, NT, kGroup, kCap>(chunk, hint, own_list, sh);
+      else {
+        Group g;
+        g.load(chunk, chunk.fb);
+        collect_row<T, NT, kGroup, kCap, false>(chunk, g, hint, 0ull, own_list, sh);
+      }
       n = gather();
       listed = n >= k && n <= kCap;
       if (!listed) {
@@ -731,22 +845,22 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
 
   bool rebuild = listed;        // the packed bins do not fit the list: they are rebuilt from it
   int span = 0;                 // expected ranks are below this
-  if (!listed) {
+  if (__builtin_expect(!listed, !HINTS)) {
     // ---- sweep 1 ----
     auto count_one = [&](float x, int) {
       const uint32_t d = rows_raw_digit(x);
       if (FF_IN_RANGE(p, d, kRowsBins, 11)) atomicAdd(&hist[d], 1u);
     };
-    Group first;
+    Group first;                // stays in registers for the second sweep
     first.load(chunk, chunk.fb);
-    Group g = first;
+    if (chunk.fb + Group::kStep <= chunk.fe) first.template each<true>(chunk, chunk.fb, count_one);
+    else first.template each<false>(chunk, chunk.fb, count_one);
 #pragma unroll 1
-    for (int u0 = chunk.fb;;) {
+    for (int u0 = chunk.fb + Group::kStep; u0 < chunk.fe; u0 += Group::kStep) {
+      Group g;
+      g.load(chunk, u0);
       if (u0 + Group::kStep <= chunk.fe) g.template each<true>(chunk, u0, count_one);
       else g.template each<false>(chunk, u0, count_one);
-      u0 += Group::kStep;
-      if (u0 >= chunk.fe) break;
-      g.load(chunk, u0);
     }
     if (chunk.head || chunk.tail) {   // (uniform)
       float x = 0.f;
@@ -762,35 +876,41 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
       FF_TRACE(p, 27);
     }
     // ---- threshold ----
-    pack_bins<NT>(merged, true, k, sh, sh.warp_tot[0]);
+    // (The thread that finds the threshold digit works the cut out too: by all threads it took 120 instructions of every warp.)
+    pack_bins<NT, true>(merged, k, sh, sh.warp_tot[0], [&](int t, int above, int in_bin, int in_next) {
+      const int keep = kept_in_digit<T>(in_bin, k - above, kCap - above);
+      int spread;
+      sh.cut = (static_cast<uint32_t>(t) << kRowsShift) +
+               cut_at<T>(DigitDensity(t, in_bin, in_next).depth_of_count(static_cast<float>(keep)), keep, in_bin, spread);
+      sh.keep = keep;
+      return spread;
+    });
     FF_TRACE(p, 2);
     // ---- sweep 2 ----
-    const int above = sh.above, in_bin = sh.total - above;
+    const int above = sh.above, keep = sh.keep;
     const uint32_t bin_key = static_cast<uint32_t>(sh.t) << kRowsShift;
-    const int keep = kept_in_digit<T>(in_bin, k - above, kCap - above);
     bool exact = bin_key > 0xff800000u || sh.max_bin > kPackMax || keep < k - above ||
                  (sh.total > kCap && 8 * sh.max_bin > 7 * sh.total);
     if (!exact) {
-      int spread;
-      const uint32_t cut =
-          bin_key + cut_at<T>(DigitDensity(merged, sh.t, in_bin).depth_of_count(static_cast<float>(keep)), keep, in_bin, spread);
-      if (sparse) collect_row_sparse<T, NT, kCap>(chunk, prefilter_value(cut), own_list, sh);
-      else collect_row<T, NT, kCap, false>(chunk, &first, prefilter_value(cut), 0ull, own_list, sh);
-      if (tid == 0) merged[rows_raw_of(sh.t)] = packed_bin(above, spread);   // (read in the finish)
+      if (sparse) collect_row_sparse<T, NT, kGroup, kCap>(chunk, prefilter_value(sh.cut), own_list, sh);
+      else if (HINTS) collect_row_again<T, NT, kGroup, kCap>(chunk, prefilter_value(sh.cut), own_list, sh);   // (rare: out of the way)
+      else collect_row<T, NT, kGroup, kCap, false>(chunk, first, prefilter_value(sh.cut), 0ull, own_list, sh);
       n = gather();
       span = above + keep;
       if (__builtin_expect(n < k || n > kCap, 0)) {   // the interpolation was off
         // The whole digit if that fits and the cut was too high; else to a place between k and what fits (nearer to k where
         // the cut goes down to a step), by the same density scaled to what was found.  Another time or two where that
         // is off again (blocks of equal scores): a sweep each, further digits take four.
-        const DigitDensity density(merged, sh.t, in_bin);
+        const int in_bin = sh.total - above;
+        int spread;
+        const DigitDensity density(sh.t, in_bin, static_cast<int>((merged[rows_raw_of(sh.t + 1)] & ((1u << kPackShift) - 1u)) >> 1));
         float x = density.depth_of_count(static_cast<float>(keep));
 #pragma unroll 1
         for (int attempt = 0; attempt < 3 && (n < k || n > kCap); ++attempt) {
           discard();
           const int more = n < k && sh.total <= kCap ? in_bin : k - above + ((kCap - k) >> (kCoarseSteps<T> ? 2 : 1));
           x = density.depth_of_count(static_cast<float>(more) * __fdividef(density.count_above(x), static_cast<float>(max(n - above, 1))));
-          collect_row_again<T, NT, kCap>(chunk, prefilter_value(bin_key + cut_at<T>(x, more, in_bin, spread)), own_list, sh);
+          collect_row_again<T, NT, kGroup, kCap>(chunk, prefilter_value(bin_key + cut_at<T>(x, more, in_bin, spread)), own_list, sh);
           if (tid == 0) merged[rows_raw_of(sh.t)] = packed_bin(above, spread);
           n = gather();
           span = above + more;
@@ -803,8 +923,8 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     if (__builtin_expect(exact, 0)) {
       rebuild = true;
       const uint64_t floor_comp = sh.total <= kCap ? static_cast<uint64_t>(sh.t) << rows_level_shift(0)
-                                                   : deeper_digits<T, NT, CLUSTER>(chunk, hist, merged, k, kCap, sh, p.status);
-      collect_row_exact<T, NT, kCap>(chunk, floor_comp, own_list, sh);
+                                                   : deeper_digits<T, NT, kGroup, CLUSTER>(chunk, hist, merged, k, kCap, sh, p.status);
+      collect_row_exact<T, NT, kGroup, kCap>(chunk, floor_comp, own_list, sh);
       n = gather();
     }
   }
@@ -813,12 +933,11 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   if (rebuild) span = n;
 
   // ---- finish ----
-  // A thread keeps its survivors in registers; where[] is in turn a survivor's packed bin, finish bin and
-  // arrival in it, bucket (first slot << 16 | size), and rank.  Loads and stores are kept in loops of their
-  // own, so that a phase's loads are in flight together.  The second half of the places is skipped
-  // by the whole CTA when n leaves it empty.
+  // A thread keeps its survivors in registers; where[] is in turn a survivor's packed bin and its finish bin.  Loads and
+  // stores are kept in loops of their own, so that a phase's loads are in flight together.  The second half of the
+  // places is skipped by the whole CTA when n leaves it empty.
   constexpr int kHalf = (PER + 1) / 2;
-  uint32_t depth[PER], where[PER];
+  uint32_t bits[PER], where[PER];        // score bits (-0.0 and NaN as in the keys)
   int32_t pos[PER];                      // window position, or -1: no survivor
   auto mine = [&](auto&& f) {
 #pragma unroll
@@ -829,34 +948,39 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     }
   };
 #pragma unroll
-  for (int j = 0; j < PER; ++j) pos[j] = -1;
-  {
-    uint32_t value_bits = 0u;
-    mine([&](int j) {
-      if (tid + j * NT < n) {
-        const uint2 entry = reinterpret_cast<const uint2*>(list.x)[tid + j * NT];
-        const float x = __uint_as_float(entry.x);
-        pos[j] = static_cast<int32_t>(entry.y);
-        value_bits |= __float_as_uint(x);
-        depth[j] = __float_as_uint(__fadd_rn(x, 0.0f));   // (-0.0 and NaN as in the keys)
-        if (!rebuild) where[j] = merged[depth[j] >> kRowsShift];
-      }
-    });
-    value_bits = __reduce_or_sync(0xffffffffu, value_bits);
-    if ((tid & 31) == 0) atomicOr(&sh.value_bits, value_bits);
-  }
+  for (int j = kHalf; j < PER; ++j) pos[j] = -1;
+  mine([&](int j) {   // (behind the n survivors the list holds anything)
+    const uint2 entry = reinterpret_cast<const uint2*>(list.x)[tid + j * NT];
+    pos[j] = tid + j * NT < n ? static_cast<int32_t>(entry.y) : -1;
+    bits[j] = __float_as_uint(__fadd_rn(__uint_as_float(entry.x), 0.0f));
+    if (!rebuild) where[j] = merged[bits[j] >> kRowsShift];
+  });
+  // The low bits that are zero in all survivors' scores.  One with a low bit set tells that there are none, so the first of every
+  // thread's are looked at first.
+  auto add_value_bits = [&](int to, int j0, int j1) {
+    uint32_t v = 0u;
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (j >= j0 && j < j1) v |= pos[j] >= 0 ? bits[j] : 0u;
+    v = __reduce_or_sync(0xffffffffu, v);
+    if ((tid & 31) == 0) atomicOr(&sh.value_bits[to], v);
+  };
+  constexpr uint32_t kLowBits = 0x1ffu;
+  constexpr bool kHalfScores = Elem<T>::kPerUnit != 4;
+  // (Rebuilt bins leave out low key bits in which no two survivors differ, whatever they are.)
+  if (kHalfScores || rebuild) add_value_bits(0, 0, PER); else add_value_bits(0, 0, 1);
   auto key_bits = [](uint32_t u) { return u ^ (static_cast<uint32_t>(static_cast<int32_t>(u) >> 31) | 0x80000000u); };
   uint32_t base = 0u;
   int shift = kRowsShift;
-  if (rebuild) {
+  if (__builtin_expect(rebuild, HINTS)) {
     // digits of the survivors' own key range instead of the row's first digit
     uint32_t kmin = 0xffffffffu, kmax = 0u;
     if (CLUSTER || !listed) clear_words(hist, kRowsBins);
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       if (pos[j] >= 0) {
-        kmin = min(kmin, key_bits(depth[j]));
-        kmax = max(kmax, key_bits(depth[j]));
+        kmin = min(kmin, key_bits(bits[j]));
+        kmax = max(kmax, key_bits(bits[j]));
       }
     }
     kmin = __reduce_min_sync(0xffffffffu, kmin);
@@ -871,7 +995,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     shift = range >= static_cast<uint32_t>(kRowsBins) ? 32 - __clz(static_cast<int>(range)) - kRowsBits : 0;
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
-      const uint32_t d = (key_bits(depth[j]) - base) >> shift;
+      const uint32_t d = (key_bits(bits[j]) - base) >> shift;
       if (pos[j] >= 0 && !FF_IN_RANGE(p, d, kRowsBins, 15)) pos[j] = -1;   // (a place that trips drops its survivor)
       if (pos[j] >= 0) atomicAdd(&hist[d], 1u);
     }
@@ -881,7 +1005,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
       uint32_t low_bits = 0u;
 #pragma unroll
       for (int j = 0; j < PER; ++j) {
-        const uint32_t k0 = key_bits(depth[j]) - base;
+        const uint32_t k0 = key_bits(bits[j]) - base;
         if (pos[j] >= 0 && (k0 >> shift) == 0u) {
           last_pos = max(last_pos, pos[j]);
           low_bits |= k0;
@@ -894,14 +1018,20 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
         atomicOr(&sh.low_bits, low_bits);
       }
     }
-    pack_bins<NT>(hist, false, n, sh, sh.warp_tot[2]);
+    pack_bins<NT, false>(hist, n, sh, sh.warp_tot[2], [](int, int, int in_bin, int) { return in_bin; });
 #pragma unroll
     for (int j = 0; j < PER; ++j)
-      if (pos[j] >= 0) where[j] = hist[(key_bits(depth[j]) - base) >> shift];
+      if (pos[j] >= 0) where[j] = hist[(key_bits(bits[j]) - base) >> shift];
   } else {
     __syncthreads();   // the list has been read
   }
-  if (!rebuild && (sh.value_bits & 0x1fffu) == 0u) {
+  const bool steps = kHalfScores || (sh.value_bits[0] & kLowBits) == 0u;
+  if (__builtin_expect(!kHalfScores && !rebuild && steps, 0)) {
+    add_value_bits(1, 1, PER);
+    __syncthreads();
+  }
+  const uint32_t value_bits = sh.value_bits[0] | sh.value_bits[1];
+  if (!rebuild && (value_bits & 0x1fffu) == 0u) {
     // Scores in steps (fp16, bf16, or rounded to them) go on below the cut for up to a sixteenth of the threshold digit, and
     // those, all given the last rank, would share one bucket (64 ragged rows of 128 Ki bf16 logits: 31.7 us).
     const uint32_t digit = merged[rows_raw_of(sh.t)];
@@ -909,7 +1039,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     span = min(above + min(span - above + (spread >> 4) + 1, spread), kCap);
   }
   clear_words(bins, 2 * span);
-  const DepthMap map = depth_map(shift, sh.value_bits, len);
+  const DepthMap map = depth_map(shift, value_bits, len);
   const uint32_t last_bin = 2u * static_cast<uint32_t>(span) - 1u;
   // The lowest of the rebuilt bins of a row of -inf (or zeros) with a thousand other scores holds the first of those equal
   // ones, a thousand too: if it is crowded it spreads over the key bits and positions that it has itself.  (Over the digit's and
@@ -919,166 +1049,119 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     constexpr bool EVEN = decltype(even)::value;
     const bool crowded = !EVEN && sh.last_pos != 0;
     const int low_shift = crowded ? 32 - __clz(static_cast<int>(sh.low_bits)) : shift;
-    const DepthMap lowest = crowded ? depth_map(low_shift, sh.value_bits, sh.last_pos + 1) : map;
+    const DepthMap lowest = crowded ? depth_map(low_shift, value_bits, sh.last_pos + 1) : map;
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
-      const uint32_t k0 = key_bits(depth[j]) - base;
+      const uint32_t k0 = key_bits(bits[j]) - base;
       const bool low = !EVEN && (k0 >> shift) == 0u;
       const int width = low ? low_shift : shift;
-      depth[j] = depth_of(low ? lowest : map, width == 0 ? 0u : k0 << (32 - width), pos[j]);
-      where[j] = min(expected_rank2(where[j], depth[j]), last_bin);
+      where[j] = min(expected_rank2(where[j], depth_of(low ? lowest : map, width == 0 ? 0u : k0 << (32 - width), pos[j])), last_bin);
     }
   };
   if (HINTS && rebuild && sh.last_pos == 0) {
     spread_rebuilt(std::true_type{});
-  } else if (rebuild) {
+  } else if (__builtin_expect(rebuild, 0)) {
     spread_rebuilt(std::false_type{});
+  } else if (__builtin_expect(!steps, !kHalfScores)) {
+    // (in equal keys the index would change nothing but the last bits of the depth)
+    mine([&](int j) {
+      const uint32_t below = (bits[j] ^ static_cast<uint32_t>(static_cast<int32_t>(bits[j]) >> 31)) << kRowsBits;
+      where[j] = min(expected_rank2(where[j], ~below), last_bin);
+    });
   } else {
     mine([&](int j) {
-      depth[j] = depth_of(map, (depth[j] ^ static_cast<uint32_t>(static_cast<int32_t>(depth[j]) >> 31)) << kRowsBits, pos[j]);
-      where[j] = min(expected_rank2(where[j], depth[j]), last_bin);
+      const uint32_t below = (bits[j] ^ static_cast<uint32_t>(static_cast<int32_t>(bits[j]) >> 31)) << kRowsBits;
+      where[j] = min(expected_rank2(where[j], depth_of(map, below, pos[j])), last_bin);
     });
   }
   __syncthreads();   // the bins are clear
   mine([&](int j) {
     if (pos[j] >= 0 && !FF_IN_RANGE(p, where[j], 2 * kCap, 12)) pos[j] = -1;
-    if (pos[j] >= 0) where[j] |= atomicAdd(&bins[where[j]], 1u) << 16;
+    if (pos[j] >= 0) atomicAdd(&bins[where[j]], 1u);
   });
   __syncthreads();
   FF_TRACE(p, 22);
   {
-    // counts -> (first slot << 16 | size)
+    // counts -> first slot
     constexpr int per = 2 * PER;
     constexpr int kQuads = (per + 3) / 4;
     uint4* quads = reinterpret_cast<uint4*>(bins);
     const int q0 = tid * kQuads;
     const int q_end = (2 * span + 3) >> 2;
     uint4 v[kQuads];
-    uint32_t local = 0u;
+    uint32_t local = 0u, largest = 0u;
 #pragma unroll
     for (int q = 0; q < kQuads; ++q) {
       v[q] = q0 + q < q_end ? quads[q0 + q] : make_uint4(0u, 0u, 0u, 0u);
       local += (v[q].x + v[q].y) + (v[q].z + v[q].w);
+      largest = max(max(max(v[q].x, v[q].y), max(v[q].z, v[q].w)), largest);
     }
+    largest = __reduce_max_sync(0xffffffffu, largest);
+    if ((tid & 31) == 0) atomicMax(&sh.max_bucket, largest);
     int total;
     const int after = suffix_exclusive<NT>(static_cast<int>(local), sh.warp_tot[1], total);
     uint32_t start = static_cast<uint32_t>(total - after) - local;
 #pragma unroll
     for (int q = 0; q < kQuads; ++q) {
       const uint32_t s1 = start + v[q].x, s2 = s1 + v[q].y, s3 = s2 + v[q].z;
-      if (q0 + q < q_end)
-        quads[q0 + q] = make_uint4((start << 16) | v[q].x, (s1 << 16) | v[q].y, (s2 << 16) | v[q].z, (s3 << 16) | v[q].w);
+      if (q0 + q < q_end) quads[q0 + q] = make_uint4(start, s1, s2, s3);
       start = s3 + v[q].w;
     }
   }
   __syncthreads();
   FF_TRACE(p, 23);
-  {
-    uint32_t at[PER];
-    mine([&](int j) {
-      if (pos[j] >= 0) {
-        const uint32_t w = bins[where[j] & 0xffffu];
-        at[j] = (w >> 16) + (where[j] >> 16);
-        where[j] = w;
-      }
-    });
-    mine([&](int j) {
-      if (pos[j] >= 0 && !FF_IN_RANGE(p, at[j], kCap, 13)) pos[j] = -1;
-      if (pos[j] >= 0) bucketed[at[j]] = depth[j];
-    });
+  // Into the buckets, as (inverted key, position) words that ascend with the rank; behind, a bin's word is its bucket's end.  (With
+  // the arrival in the bin from the first atomic, and none here: 91.1 instead of 89.7 us for 4,096 prefill rows.)
+  mine([&](int j) {
+    if (pos[j] >= 0) {
+      const uint32_t at = atomicAdd(&bins[where[j]], 1u);
+      if (FF_IN_RANGE(p, at, kCap, 13))
+        sorted[at] = (static_cast<uint64_t>(~key_bits(bits[j])) << 32) | static_cast<uint32_t>(pos[j]);
+    }
+  });
+  if (tid < kRankPad) {   // what a block at either end compares with
+    sorted[-1 - tid] = 0ull;
+    sorted[n + tid] = ~0ull;
   }
   __syncthreads();
   FF_TRACE(p, 24);
-  // Rank inside the bucket by counting.  (The bins have been read: the ranked positions may take their place.)
-  bool tied = false;
-  mine([&](int j) {
-    if (pos[j] >= 0) {
-      const uint32_t size = where[j] & 0xffffu, d = depth[j];
-      uint32_t rank = where[j] >> 16;
-      const uint32_t* bucket = bucketed + rank;
-      if (FF_IN_RANGE(p, static_cast<int>(rank + size) - 1, kCap, 17)) {
-        // up to three entries without a loop; what is not there compares as the largest depth (a wrong "tied" does no harm)
-        const uint32_t b0 = bucket[0], b1 = size > 1u ? bucket[1] : 0xffffffffu, b2 = size > 2u ? bucket[2] : 0xffffffffu;
-        rank += (b0 < d ? 1u : 0u) + (b1 < d ? 1u : 0u) + (b2 < d ? 1u : 0u);
-        bool more = (b0 == d && b1 == d) || (b1 == d && b2 == d) || (b0 == d && b2 == d);
-        if (size > 3u) {
-          uint32_t same = (b0 == d ? 1u : 0u) + (b1 == d ? 1u : 0u) + (b2 == d ? 1u : 0u);
-#pragma unroll 1
-          for (uint32_t q = 3; q < size; ++q) {
-            rank += bucket[q] < d ? 1u : 0u;
-            same += bucket[q] == d ? 1u : 0u;
-          }
-          more = same > 1u;
-        }
-        tied |= more;
-      }
-      where[j] = rank;
-      if (FF_IN_RANGE(p, rank, kCap, 18)) ranked[rank] = pos[j]; else pos[j] = -1;
-    }
-  });
-  if (__builtin_expect(__syncthreads_or(tied ? 1 : 0), 0)) {
-    // Survivors of one depth (equal keys, neighbouring indices) have counted the same ones below them: they share the first
-    // of the ranks that are theirs, and one of them stands there.  Nobody else takes those ranks, so the others line up behind
-    // it in any order, and then each counts the positions below its own in its group.  (With a list of all others that
-    // every survivor walked, a row of equal neighbours took 30 times the time of one without: 4 x 64 Ki, blocks of 32, 441
-    // instead of 20 us.)
-    uint32_t* behind = reinterpret_cast<uint32_t*>(ranked + kCap);   // by first rank: how many line up behind it
-    clear_words(behind, kCap);
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      if (pos[j] >= 0 && ranked[where[j]] != pos[j]) {
-        // (neighbours in the row are neighbours in the list: one atomic for all of a group in the warp)
-        const unsigned group = __match_any_sync(__activemask(), where[j]);
-        const int first = __ffs(static_cast<int>(group)) - 1;
-        uint32_t at = 0u;
-        if ((tid & 31) == first) at = atomicAdd(&behind[where[j]], static_cast<uint32_t>(__popc(group)));
-        at = where[j] + 1u + __shfl_sync(group, at, first) + static_cast<uint32_t>(__popc(group & ((1u << (tid & 31)) - 1u)));
-        if (FF_IN_RANGE(p, at, kCap, 21)) ranked[at] = pos[j];
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      if (pos[j] >= 0) {
-        const int32_t* group = ranked + where[j];
-        const uint32_t more = behind[where[j]];
-        if (more != 0u && FF_IN_RANGE(p, where[j] + more, kCap, 21)) {
-          uint32_t below = 0u;
-#pragma unroll 4
-          for (uint32_t q = 0; q <= more; ++q) below += group[q] < pos[j] ? 1u : 0u;
-          where[j] += below;
-        }
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < PER; ++j)
-      if (pos[j] >= 0) ranked[where[j]] = pos[j];
-    __syncthreads();
+  // Buckets are in order, so a survivor's rank is its slot, moved by the neighbours that are not in order with it; they are no
+  // further away than the largest bucket reaches.
+  const uint32_t max_bucket = sh.max_bucket;
+  if (max_bucket <= 5u) {
+    rank_blocks<NT, rows_block_slots(PER), 4>(sorted, n, ranked);
+  } else if (max_bucket <= 7u) {
+    rank_blocks<NT, rows_block_slots(PER), 6>(sorted, n, ranked);
+  } else {
+    rank_crowded<NT, PER>(sorted, bins, 2 * span, n, ranked, p.status);
   }
+  __syncthreads();
   FF_TRACE(p, 31);
   write_all([&](int j) { return ranked[j]; }, [&](int j) { return reinterpret_cast<const int4*>(ranked)[j]; });
   FF_TRACE(p, 25);
   if constexpr (HINTS) {
-    if (p.hint_out != nullptr) {
+    if (p.hint_out != nullptr && tid == 0) {
       // Next call's guess: the score of rank hint_target_rank(k), or, with fewer survivors, a linear
-      // extrapolation below the smallest one from the ranks n / 2 and n.
+      // extrapolation below the smallest one from the ranks n / 2 and n.  A slot's score is its rank's, give or take the few
+      // ranks of a bucket (a read of the row less at the end); of crowded buckets the ranked position tells it.
       const int want = hint_target_rank(k);
       const int rank_a = min(n, want) - 1, rank_m = n >> 1;
-      if (tid == 0) {
-        const int32_t at_a = rank_a >= 0 ? ranked[rank_a] : -1, at_m = ranked[rank_m];
-        float guess = __uint_as_float(0x7fffffffu);
-        if (static_cast<uint32_t>(at_a) < static_cast<uint32_t>(len) && static_cast<uint32_t>(at_m) < static_cast<uint32_t>(len)) {
-          const float va = Elem<T>::to_float(rowp[at_a]), vm = Elem<T>::to_float(rowp[at_m]);
-          guess = va;
-          if (n < want && rank_a > rank_m) {
-            const float lower = va - (vm - va) * (static_cast<float>(want - 1 - rank_a) / static_cast<float>(rank_a - rank_m));
-            if (lower == lower && fabsf(lower) <= 3.0e38f) guess = lower;
-          }
+      auto score_of_rank = [&](int rank) {
+        if (max_bucket <= 7u) return __uint_as_float(bits_of_key(~static_cast<uint32_t>(sorted[rank] >> 32)));
+        const int32_t at = ranked[rank];
+        return static_cast<uint32_t>(at) < static_cast<uint32_t>(len) ? Elem<T>::to_float(rowp[at]) : __uint_as_float(0x7fffffffu);
+      };
+      float guess = __uint_as_float(0x7fffffffu);
+      if (rank_a >= 0) {   // (no survivors: scores that changed between the sweeps)
+        const float va = score_of_rank(rank_a);
+        guess = va;
+        if (n < want && rank_a > rank_m) {
+          const float vm = score_of_rank(rank_m);
+          const float lower = va - (vm - va) * (static_cast<float>(want - 1 - rank_a) / static_cast<float>(rank_a - rank_m));
+          if (lower == lower && fabsf(lower) <= 3.0e38f) guess = lower;
         }
-        p.hint_out[row] = guess;
       }
+      p.hint_out[row] = guess;
     }
   }
 }

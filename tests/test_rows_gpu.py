@@ -151,3 +151,47 @@ def test_logits_in_steps_are_exact_and_cost_no_more(oracle, B, L):
         sd = s.to(dev)
         us[name] = _us_per_call(lambda: fast_topk_v3(sd, ld, k, out=out))
     assert us["bf16"] < 1.2 * us["f32"] and us["f32 in steps"] < 1.3 * us["f32"], us
+
+
+# groups of 24 scores per thread: 6,144 with 256 threads, 24,576 with 1,024
+@pytest.mark.parametrize("B,L,k", [(160, 6143, 2048), (150, 6145, 512), (150, 12288, 1024), (20, 24575, 2048), (20, 24577, 1024),
+                                   (80, 49153, 2048)])
+def test_rows_that_end_at_a_group(oracle, B, L, k):
+    g = torch.Generator().manual_seed(L)
+    s = torch.stack([_row(i % KINDS, L, g) for i in range(B)])
+    _check(oracle, s, torch.full((B,), L, dtype=torch.int32) - torch.arange(B, dtype=torch.int32) % 3, k)
+
+
+@pytest.mark.parametrize("B,L,k", [(18, 16384, 2048), (160, 5461, 2048), (18, 40960, 1024), (160, 4000, 300)])
+@pytest.mark.parametrize("guess", [False, True])
+def test_buckets_of_two_to_ten(oracle, B, L, k, guess):
+    """Every score occurs r times, far apart and with a full mantissa, so that the largest bucket holds r and a few more: ranks
+    from the neighbours up to four and up to six slots away, and from a bucket that is looked up."""
+    from flash_float_jit_kernels_b200 import new_threshold_hint
+    g = torch.Generator().manual_seed(B + L)
+    s = torch.stack([torch.randn((L // (1 + i % 9) + 1,), generator=g).repeat(10)[:L] for i in range(B)])
+    lengths = torch.full((B,), L, dtype=torch.int32)
+    hint = new_threshold_hint(B, "cuda") if guess else None
+    for _ in range(2 if guess else 1):
+        _check(oracle, s, lengths, k, threshold_hint=hint)
+
+
+@pytest.mark.parametrize("B,L", [(40, 9000), (160, 9000), (30, 40960)])
+@pytest.mark.parametrize("zeros", [8, 9, 13])
+@pytest.mark.parametrize("guess", [False, True])
+def test_low_bits_that_two_scores_have(oracle, B, L, zeros, guess):
+    """Scores without their last `zeros` bits but for two among the winners, whose order those bits decide against their
+    positions."""
+    from flash_float_jit_kernels_b200 import new_threshold_hint
+    g = torch.Generator().manual_seed(B + zeros)
+    k = 2048
+    bits = torch.randn((B, L), generator=g).view(torch.int32) & ~((1 << zeros) - 1) | (1 << zeros)
+    rows = torch.arange(B)
+    top = bits.view(torch.float32).topk(1500, dim=1).indices[rows, 20 + 30 * (rows % 40)]   # one of the winners
+    low, high = torch.minimum(top, (top + L // 2) % L), torch.maximum(top, (top + L // 2) % L)
+    value = bits[rows, top]
+    bits[rows, low], bits[rows, high] = value + 1, value + 2
+    lengths = torch.full((B,), L, dtype=torch.int32)
+    hint = new_threshold_hint(B, "cuda") if guess else None
+    for _ in range(2 if guess else 1):
+        _check(oracle, bits.view(torch.float32), lengths, k, threshold_hint=hint)

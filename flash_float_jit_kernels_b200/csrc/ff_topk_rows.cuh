@@ -216,14 +216,17 @@ __device__ __forceinline__ uint32_t cut_at(float x, int keep, int in_bin, int& s
   return all ? 0u : static_cast<uint32_t>((1.f - x) * static_cast<float>(1 << kRowsShift)) & ~(kKeyStep<T> - 1u);
 }
 
-// Suffix scan of the bins in monotone order (CUT: the array is in rows_raw_digit() order).  Every non-empty bin
+// Suffix scan of the bins in monotone order (raw: the array is in rows_raw_digit() order).  Every non-empty bin
 // with fewer than `limit` elements above it is packed in place, and the bin that reaches the limit
 // is published as sh.t with its counts.
-// CUT: by the thread that finds it, which calls `crossing(t, above, in_bin, in_next)` with the count of the next digit up; it returns
-// the count that the bin is packed with.  (Without: nothing is published.)
-template <int NT, bool CUT, typename F>
-__device__ __forceinline__ void pack_bins(uint32_t* hist, int limit, RowsShared& sh, int* warp_tot, F&& crossing) {
-  constexpr bool raw = CUT;
+// By the thread that finds it, which calls `crossing(t, above, in_bin, in_next)` with the count of the next digit up; it returns
+// the count that the bin is packed with.  (NoCut: nothing is published.)
+struct NoCut {
+  __device__ __forceinline__ int operator()(int, int, int in_bin, int) const { return in_bin; }
+};
+template <int NT, typename F>
+__device__ __forceinline__ void pack_bins_and_cut(uint32_t* hist, bool raw, int limit, RowsShared& sh, int* warp_tot, F&& crossing) {
+  constexpr bool CUT = !std::is_same<std::decay_t<F>, NoCut>::value;
   constexpr int per = kRowsBins / NT;
   // whole 16-byte quads per thread, their rotation a mask, and a divisor of the 32 banks: 4,096 bins over 192 threads are
   // 21 each, at 4-byte addresses
@@ -233,7 +236,7 @@ __device__ __forceinline__ void pack_bins(uint32_t* hist, int limit, RowsShared&
   const bool up = !raw || m0 >= kRowsBins / 2;   // the thread's bins lie in ascending order
   const int base = !raw ? m0 : up ? m0 - kRowsBins / 2 : kRowsBins - per - m0;
   int next = 0;                                  // what the digit above the thread's holds, while nothing is packed
-  if (raw && tid < NT - 1) next = static_cast<int>(hist[rows_raw_of(m0 + per)]);
+  if (CUT && tid < NT - 1) next = static_cast<int>(hist[raw ? rows_raw_of(m0 + per) : m0 + per]);
   int local = 0;
 #pragma unroll
   for (int j = 0; j < per / 4; ++j) {            // rotated so that eight threads read eight different bank groups
@@ -275,10 +278,15 @@ __device__ __forceinline__ void pack_bins(uint32_t* hist, int limit, RowsShared&
       sh.t = t;
       sh.above = above;
       sh.total = above + in_bin;
-      hist[rows_raw_of(t)] = packed_bin(above, crossing(t, above, in_bin, in_next));
+      hist[raw ? rows_raw_of(t) : t] = packed_bin(above, crossing(t, above, in_bin, in_next));
     }
   }
   __syncthreads();
+}
+
+template <int NT>
+__device__ __forceinline__ void pack_bins(uint32_t* hist, bool raw, int limit, RowsShared& sh, int* warp_tot) {
+  pack_bins_and_cut<NT>(hist, raw, limit, sh, warp_tot, NoCut{});
 }
 
 // Scores of a group: the more, the less a score's share of the second sweep's slots is (prefill batches of 5.5 and 16 Ki scores:
@@ -877,7 +885,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     }
     // ---- threshold ----
     // (The thread that finds the threshold digit works the cut out too: by all threads it took 120 instructions of every warp.)
-    pack_bins<NT, true>(merged, k, sh, sh.warp_tot[0], [&](int t, int above, int in_bin, int in_next) {
+    pack_bins_and_cut<NT>(merged, true, k, sh, sh.warp_tot[0], [&](int t, int above, int in_bin, int in_next) {
       const int keep = kept_in_digit<T>(in_bin, k - above, kCap - above);
       int spread;
       sh.cut = (static_cast<uint32_t>(t) << kRowsShift) +
@@ -1018,7 +1026,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
         atomicOr(&sh.low_bits, low_bits);
       }
     }
-    pack_bins<NT, false>(hist, n, sh, sh.warp_tot[2], [](int, int, int in_bin, int) { return in_bin; });
+    pack_bins<NT>(hist, false, n, sh, sh.warp_tot[2]);
 #pragma unroll
     for (int j = 0; j < PER; ++j)
       if (pos[j] >= 0) where[j] = hist[(key_bits(bits[j]) - base) >> shift];

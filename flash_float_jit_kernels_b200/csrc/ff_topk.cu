@@ -40,6 +40,9 @@ bool self_seed_enabled() {
   return env == nullptr || atoi(env) != 0;
 }
 
+// Polls after which a CTA of a plainly launched split row gives a wait for the others up; set through ff_topk_set_wait_limit.
+std::atomic<int> g_wait_limit{ff::kGiveUpAfter};
+
 constexpr int kMaxDevices = 64;
 std::once_flag g_init_once[kMaxDevices];
 int g_init_rc[kMaxDevices];
@@ -200,21 +203,21 @@ int choose_cluster(int device, int32_t B, int64_t L_width, int32_t k) {
 }
 
 // Rows that are long and few are split over several clusters (groups) so that all SMs sweep them; that needs the
-// caller's zero-filled workspace and a cooperative launch (all CTAs of a row wait for each other through
-// global memory).  Returns the number of clusters per row and may lower `cluster`.
+// caller's zero-filled workspace, since all CTAs of a row wait for each other through
+// global memory.  Returns the number of clusters per row and may lower `cluster`.
 //
-// Clusters of two: 74 of them fit, on all 148 SMs (of eight only 15, on 120), and rows that need no histogram have no
-// use for wider ones (B = 1, 8 Mi columns 19.4 -> 18.6 us, B = 4, 1 Mi, k = 512 15.7 -> 14.7).
-//   * Rows that make their own guess are swept once: split rows of 256 Ki columns take 13.2 us (B = 2), 13.4 (B = 4), 14.8
-//     (B = 8), 17.5 (B = 16) in a graph, against 14.4, 14.5, 17.1 and 23.3 in one cluster each.  The guess needs about 200 hits
+// Clusters of ONE CTA, launched plainly (kGiveUpAfter): a cooperative launch outside a graph starts on a 2.048 us beat behind the
+// kernel in front of it (call by call, clusters of two in a cooperative launch : now, 1 x 1 Mi 14.3 : 12.8 us, 1 x 8 Mi 18.4 :
+// 18.2, 4 x 1 Mi, k = 512, 14.4 : 13.0), and clusters of two leave SMs over where the batch does not divide 74 (4 x 1 Mi 13.0 : 12.7).
+//   * Rows that make their own guess are swept once: split rows of 256 Ki columns take 13.5 us (B = 2), 13.8 (B = 4), 14.5
+//     (B = 8), 16.2 (B = 16), against 14.5, 14.7, 16.5 and 23.3 in one cluster each.  The guess needs about 200 hits
 //     in the CTAs' samples (seed_plan), 27 of them from one CTA at most.
-//   * A cooperative launch that is not replayed from a graph starts on a 2.048 us beat behind the kernel in front of it, and
-//     short rows of a ragged batch make no guess (12 ragged rows of 192 Ki bf16 columns 22.7 us split, 15.1 in clusters).
-//     So eager calls and 16-bit scores are split from 256 Ki + 64 k columns up (B = 4, eager, split : clusters, 256 Ki
-//     16.4 : 15.0 us full and 17.1 : 14.9 ragged, 384 Ki 16.6 : 16.8 and 17.4 : 17.2, 512 Ki 16.6 : 18.2 and 16.7 : 17.3),
-//     captured fp32 calls from 128 Ki + 32 k (192 Ki 13.3 : 14.1 full, 14.5 : 14.1 ragged), and so are batches whose clusters
-//     have fewer than eight CTAs (B = 16, 192 Ki, eager 18.8 : 21.2 and 20.4 : 19.6).  With guesses, which leave less to gain,
-//     only very long rows or a single row.
+//   * Short rows of a ragged batch make no guess.  So rows of 16-bit scores are split from 256 Ki + 64 k columns up (8 ragged rows of
+//     320 Ki 20.5 us split, 16.8 in clusters), fp32 rows from 128 Ki + 32 k (k = 512, split : clusters, 4 x 160 Ki 11.0 : 13.7
+//     full and 10.9 : 12.5 ragged), but call by call and for larger k only beyond 256 Ki (k = 2048, 12 x 192 Ki 14.9 : 16.0 full and
+//     17.3 : 16.3 ragged, 4 x 320 Ki 13.9 : 16.4 and 15.4 : 15.4).  Batches whose clusters
+//     have fewer than eight CTAs go by the first of these (B = 16, 192 Ki 18.8 : 21.2 and 20.4 : 19.6).  With guesses, which leave less
+//     to gain, only very long rows or a single row.
 //   * Rows that have to be swept twice are split if very long, or if one row has the GPU.
 constexpr int64_t kGroupMinWidthSingle = 131072;
 constexpr int64_t kGroupMinWidthHinted = 65536;
@@ -245,9 +248,8 @@ int choose_groups(int device, int32_t B, int64_t L_width, int32_t k, size_t work
   const bool automatic = g == 0;
   if (automatic) {
     if (g_cluster_override.load() != 0) return 1;
-    c = cp ? 8 : 2;
-    const int log2c = cp ? 3 : 1;
-    g = g_active_clusters[device][log2c] / B;
+    c = cp ? 8 : 1;
+    g = g_active_clusters[device][cp ? 3 : 0] / B;
     if (cp && g > 16) g = 16;
     const int64_t by_size = L_width / (static_cast<int64_t>(c) * (cp ? 1024 : 512));   // at least so many columns per CTA
     if (g > by_size) g = static_cast<int>(by_size);
@@ -255,10 +257,11 @@ int choose_groups(int device, int32_t B, int64_t L_width, int32_t k, size_t work
     if (cp) {
       worth = worth || (L_width >= (hinted ? kGroupMinWidthHinted : kGroupMinWidthSingle) && g >= 8);
     } else if (hinted) {
-      worth = worth || (B == 1 && L_width >= kGroupMinWidthHinted) || (B > 4 && g >= *cluster && L_width >= 524288);
+      worth = worth || (B == 1 && L_width >= kGroupMinWidthHinted) || (B > 4 && g >= 2 * *cluster && L_width >= 524288);
     } else {
-      const int64_t least = (captured && per_unit == 4) || *cluster < 8 ? 131072 + 32 * static_cast<int64_t>(k)
-                                                                         : 262144 + 64 * static_cast<int64_t>(k);
+      const int64_t least = *cluster < 8 || (per_unit == 4 && (captured || k <= 1024)) ? 131072 + 32 * static_cast<int64_t>(k)
+                            : per_unit == 4                                            ? 262144 + 1
+                                                                                       : 262144 + 64 * static_cast<int64_t>(k);
       worth = worth || (self_seed_enabled() && L_width >= least && own_guess_likely(L_width, k, g * c, per_unit)) ||
               (B == 1 && L_width >= kGroupMinWidthSingle);
     }
@@ -290,10 +293,19 @@ int launch(const ff::TopkParams& p, int cluster, cudaStream_t stream, int dtype 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  ff::TopkParams q = p;
+  // A row split over clusters that has no guess makes its own (FF_TOPK_SELF_SEED=0 or
+  // ff_topk_set_self_seed(0) switch that off); the code lives in the instantiation with guesses.
+  if (!HAS_MAP && groups > 1 && self_seed_enabled()) q.self_seed = 1;
+  const bool hints = q.hint_in != nullptr || q.hint_out != nullptr || q.self_seed != 0;
+  const bool split = groups > 1;
   // Cooperative whenever CTAs of the launch wait for each other through global memory: rows split
   // over clusters, and the single-kernel context-parallel step (its CTAs poll for entries that
-  // CTAs of the same launch on the peers store), so that residency is guaranteed, not inferred.
-  if (groups > 1 || p.push_fused != 0) {
+  // CTAs of the same launch on the peers store), so that residency is guaranteed, not inferred.  Except for rows split over
+  // single CTAs by the kernel with guesses, which finishes a row whose CTAs do not run together all the same (kGiveUpAfter).
+  const bool plain_split = !HAS_MAP && split && hints && cluster == 1 && q.push_world == 0;
+  if (plain_split) q.wait_limit = g_wait_limit.load(std::memory_order_relaxed);
+  if ((split && !plain_split) || p.push_fused != 0) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeCooperative;
     attr[cfg.numAttrs].val.cooperative = 1;
     ++cfg.numAttrs;
@@ -303,18 +315,12 @@ int launch(const ff::TopkParams& p, int cluster, cudaStream_t stream, int dtype 
     attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++cfg.numAttrs;
   }
-  ff::TopkParams q = p;
   q.trace = g_trace.load(std::memory_order_relaxed);
   q.block_base = 0;
   q.grid_ctas = static_cast<int32_t>(cfg.gridDim.x);
 
   // one instantiation per mode: the plain select carries no code of the others
   cudaError_t e;
-  // A row split over clusters that has no guess makes its own (FF_TOPK_SELF_SEED=0 or
-  // ff_topk_set_self_seed(0) switch that off); the code lives in the instantiation with guesses.
-  if (!HAS_MAP && groups > 1 && self_seed_enabled()) q.self_seed = 1;
-  const bool hints = q.hint_in != nullptr || q.hint_out != nullptr || q.self_seed != 0;
-  const bool split = groups > 1;
   if (!HAS_MAP && dtype == FF_DTYPE_BF16 && hints && split)
     e = cudaLaunchKernelEx(&cfg, ff::topk_cluster_kernel<false, ff::kModeHintedSplit, __nv_bfloat16>, q);
   else if (!HAS_MAP && dtype == FF_DTYPE_F16 && hints && split)
@@ -570,6 +576,11 @@ int ff_topk_set_self_seed(int32_t on) {
 
 int ff_topk_set_programmatic_launch(int32_t on) {
   g_programmatic.store(on < 0 ? -1 : (on != 0 ? 1 : 0));
+  return 0;
+}
+
+int ff_topk_set_wait_limit(int32_t polls) {
+  g_wait_limit.store(polls > 0 ? polls : ff::kGiveUpAfter);
   return 0;
 }
 

@@ -121,7 +121,9 @@ struct TopkParams {
   unsigned char* handover;     // or null: per row kHandoverRowBytes {count, readers, pad to 64 B, uint64 entries[kSortCap]}:
                                // the producer of the scores has already listed every score not below hint_in[row]
   int32_t self_seed;           // 1: a row split over clusters that has no guess makes its own (see seed_own_guess)
-  int32_t groups;              // clusters per row (> 1 needs workspace and a cooperative launch)
+  int32_t groups;              // clusters per row (> 1 needs workspace, and a cooperative launch or a wait_limit)
+  int32_t wait_limit;          // rows split over single CTAs without a cooperative launch: polls after which a CTA gives a wait
+                               // for the others up, so that the last one left selects the row alone; 0: never
   uint32_t* workspace;         // zero-filled global scratch, kWsRowWords words per row
   PeerPtrs push_peers;         // context-parallel send: results go to these exchange buffers
   int32_t push_world;          // > 0 switches the push on

@@ -435,6 +435,7 @@ struct ClusterShared {
   int cand_count;
   int push_base;
   int hint_total;    // survivors of all CTAs of the cluster in a hinted attempt
+  int lost;          // an entry of the row's survivor list never came
   int flag;          // row-barrier result / last-CTA flag
   int big_count;     // elements of large buckets queued in the finish
   uint32_t fin_red[5];   // finish: max / min key, max / min index half, differing key bits of the survivors
@@ -548,7 +549,8 @@ __device__ __forceinline__ void scan_tile(uint32_t tile, int units, int first_un
 // Per-row scratch in global memory (all zero between launches; the kernel
 // leaves it zeroed).  Word offsets:
 //   [0, 6)   arrivals at the histogram barrier of digit level 0..5
-//   [6]      arrivals at the survivor barrier      [7] CTAs that are done
+//   [6]      arrivals at the survivor barrier
+//   [7]      CTAs that are done (low half), and those of them that gave a wait up (high half)
 //   [8]      survivors appended so far
 //   [10,11]  hinted attempt: one 64-bit word, low half survivors appended, high half CTAs that have reserved
 //   [64, 320) first digit level only: the row's histogram summed in groups of 32 bins
@@ -568,16 +570,26 @@ static_assert(kWsSeedWord % 2 == 0, "the accumulator is a 64-bit word");
 constexpr int kWsRowWords = kWsSeedWord + kWsSeedWords;
 constexpr int kSpinLimit = 1 << 21;   // bounded polling of a row barrier (about a second)
 
-// All `expected` CTAs of a row meet here (they are co-resident: cooperative
-// launch).  Thread 0 publishes this CTA's earlier global writes and polls the
+// The CTAs of a row split over clusters wait for each other.  Two ways to be sure that such a row is finished:
+//   * a cooperative launch: all CTAs run at the same time.  Outside a graph it starts on a 2.048 us beat behind the kernel in
+//     front of it (1 x 1 Mi columns 14.3 us call by call, 12.7 in a graph);
+//   * p.wait_limit (rows split over single CTAs that take a guess): a plain launch.  The GPU starts the CTAs of one grid before
+//     those of the next, so they normally run together too (1 x 1 Mi 12.6 us), but nothing promises it: a kernel on a
+//     stream of higher priority may take the rest of the SMs and wait for these.  So a CTA whose wait runs out counts itself out
+//     as having given up, without writing, and leaves its SM; whoever counts itself out last, when all others have
+//     left the scratch, sees that and selects the row alone (redo_row_alone).  CTAs that did not give up have seen
+//     everybody's survivors, so what they write is what it writes.
+constexpr int kGiveUpAfter = 1 << 14;   // polls, about ten milliseconds
+
+// All `expected` CTAs of a row meet here.  Thread 0 publishes this CTA's earlier global writes and polls the
 // arrival counter; returns false if the poll limit ran out.
-__device__ __forceinline__ bool row_barrier(uint32_t* counter, uint32_t expected, int* flag) {
+__device__ __forceinline__ bool row_barrier(uint32_t* counter, uint32_t expected, int* flag, int limit) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
     atomicAdd(counter, 1u);
     int ok = 0;
-    for (int i = 0; i < kSpinLimit; ++i) {
+    for (int i = 0; i < limit; ++i) {
       uint32_t v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
       if (v >= expected) {
@@ -594,7 +606,7 @@ __device__ __forceinline__ bool row_barrier(uint32_t* counter, uint32_t expected
 // Copies the first n entries of a global survivor list into shared memory.  The list is zero
 // between launches and no composite is zero, so an entry is valid as soon as it is non-zero:
 // each thread polls its own entries (bounded), and no barrier or fence follows the writers.
-__device__ __forceinline__ bool load_list_validated(const uint64_t* glist, int n, uint64_t* dst) {
+__device__ __forceinline__ bool load_list_validated(const uint64_t* glist, int n, uint64_t* dst, int limit) {
   // all of a thread's entries are requested before the first one is looked at (the list has at
   // most kSortCap entries: kSortCap / kThreads per thread); only missing ones are polled again
   constexpr int kPer = kSortCap / kThreads;
@@ -610,7 +622,7 @@ __device__ __forceinline__ bool load_list_validated(const uint64_t* glist, int n
   for (int j = 0; j < kPer; ++j) {
     const int i = static_cast<int>(threadIdx.x) + j * kThreads;
     if (i < n) {
-      for (int spin = 0; v[j] == 0ull && spin < kSpinLimit; ++spin)
+      for (int spin = 0; v[j] == 0ull && spin < limit; ++spin)
         asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(v[j]) : "l"(glist + i) : "memory");
       if (v[j] == 0ull) ok = false;
       dst[i] = v[j];
@@ -627,7 +639,7 @@ __device__ __forceinline__ bool load_list_validated(const uint64_t* glist, int n
 __device__ __forceinline__ void merge_and_scan(cg::cluster_group& cluster, int C, int rank,
                                                uint32_t* hist, uint32_t* merged, int nbins, int r,
                                                bool raw0, ClusterShared& sh, const TopkParams& p, bool tr,
-                                               int G, uint32_t* ws, int level, bool& timed_out,
+                                               int G, uint32_t* ws, int level, bool& timed_out, int limit,
                                                int counted = -1) {
   // counted: how many elements the histograms of the whole row hold at this level (first level: the
   // row's length), or -1 if not known
@@ -731,14 +743,14 @@ __device__ __forceinline__ void merge_and_scan(cg::cluster_group& cluster, int C
       }
     }
     if (!self_counting) {
-      if (!row_barrier(ws + level, static_cast<uint32_t>(G * C), &sh.flag)) timed_out = true;
+      if (!row_barrier(ws + level, static_cast<uint32_t>(G * C), &sh.flag, limit)) timed_out = true;
     }
     if (two_step) {
       int val = 0, total = 0, excl = 0;
       if (self_counting) {
         // the poll is the coarse scan itself: read, sum, repeat until the sum is complete (bounded)
         bool complete = false;
-        for (int spin = 0; spin < (kSpinLimit >> 6) && !complete; ++spin) {
+        for (int spin = 0; spin < (limit >> 6) + 1 && !complete; ++spin) {
           uint32_t w = 0u;
           // acquire: a complete coarse sum makes the fine bins added before it visible (the CTA
           // barriers of the scan below carry that on to the lanes that read the fine bins)
@@ -1040,7 +1052,7 @@ template <typename T>
 // SMs, unlike the cycle stamps of the other slots) when the sample has landed, when this CTA's
 // estimate goes out, and when all CTAs' estimates are in.
 __device__ __noinline__ SeedResult seed_own_guess(uint32_t tile0, int n0, int* flag, uint32_t* scratch, uint32_t* ws,
-                                                  float p_frac, int n_share, int my_share,
+                                                  float p_frac, int n_share, int my_share, int limit,
                                                   unsigned long long* tr = nullptr) {
   constexpr int kPU = Elem<T>::kPerUnit;
   const int tid = threadIdx.x;
@@ -1131,7 +1143,7 @@ __device__ __noinline__ SeedResult seed_own_guess(uint32_t tile0, int n0, int* f
     atomicAdd(acc, add);
     unsigned long long v = 0ull;
     int spin = 0;
-    for (; spin < kSpinLimit; ++spin) {
+    for (; spin < limit; ++spin) {
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(acc) : "memory");
       if (static_cast<int>(v >> 54) >= n_share) break;
     }
@@ -1139,8 +1151,8 @@ __device__ __noinline__ SeedResult seed_own_guess(uint32_t tile0, int n0, int* f
     const int valid = static_cast<int>((v >> 44) & 1023ull);
     // the mean of the keys (keys are close to linear in the score over so narrow a range)
     uint32_t mean = 0u;
-    if (spin < kSpinLimit && 2 * valid >= n_share) mean = static_cast<uint32_t>((v & ((1ull << 44) - 1ull)) / static_cast<unsigned long long>(valid));
-    *flag = spin < kSpinLimit ? 1 : 0;
+    if (spin < limit && 2 * valid >= n_share) mean = static_cast<uint32_t>((v & ((1ull << 44) - 1ull)) / static_cast<unsigned long long>(valid));
+    *flag = spin < limit ? 1 : 0;
     scratch[0] = mean;
   }
   __syncthreads();
@@ -1227,7 +1239,7 @@ constexpr int kModeSplit = 8;
 constexpr int kModeHintedSplit = kModeHinted | kModeSplit;
 
 // Returns true when the row's output has been written by the survivor exchange of a
-// context-parallel step (then the caller has no runs to merge).
+// context-parallel step (then the caller has no runs to merge); kModeSplit: when this CTA has to select the row alone.
 template <bool HAS_MAP, int MODE, typename T>
 __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char* smem, ClusterShared& sh,
                                               const PushCtx& push) {
@@ -1256,6 +1268,9 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
   uint32_t* ws = G > 1 ? p.workspace + static_cast<size_t>(row) * kWsRowWords : nullptr;
   const int tid = threadIdx.x;
   const int k = p.k;
+  const bool may_give_up = kSplit && p.wait_limit != 0;
+  const int wait_limit = may_give_up ? p.wait_limit : kSpinLimit;
+  bool lost = false;        // a wait for the row's other CTAs ran out
 
   // ---- row geometry (uniform over the cluster) ---------------------------
   const int rs = p.row_starts != nullptr ? p.row_starts[row] : 0;
@@ -1357,6 +1372,7 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
     sh.sort_count = 0;
     sh.cand_count = 0;
     sh.hint_total = 0;
+    sh.lost = 0;
     sh.fin_red[0] = 0u;
     sh.fin_red[1] = 0xffffffffu;
     sh.fin_red[2] = 0u;
@@ -1404,7 +1420,7 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
           fallback = true;
         } else {
           const int n0 = seed_sample_ready(ts, sp, false);
-          const SeedResult sr = seed_own_guess<T>(ts.ring, n0, &sh.flag, hist, ws, sp.p, n_share, my_share);
+          const SeedResult sr = seed_own_guess<T>(ts.ring, n0, &sh.flag, hist, ws, sp.p, n_share, my_share, kSpinLimit);
           if (sr.code == 2) ts.timed_out = true;
           FF_TRACE(p, 21);
           if (sr.code != 1) {
@@ -1696,9 +1712,9 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
       // the chunk's first tile or two (they stay in the ring for the sweep that follows)
       const int n0 = seed_sample_ready(ts, sp, true);
       const SeedResult sr = seed_own_guess<T>(
-          ts.ring, n0, &sh.flag, hist, ws, sp.p, n_share, my_share,
+          ts.ring, n0, &sh.flag, hist, ws, sp.p, n_share, my_share, wait_limit,
           p.trace != nullptr ? p.trace + static_cast<size_t>(blockIdx.x) * kTraceSlots : nullptr);
-      if (sr.code == 2) ts.timed_out = true;
+      if (sr.code == 2) lost = true;
       if (sr.code == 1) {
         hint = sr.guess;
         use_hint = true;
@@ -1735,15 +1751,15 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
       if (tid == 0) {
         unsigned long long v = 0ull;
         int spin = 0;
-        for (; spin < kSpinLimit; ++spin) {
+        for (; spin < wait_limit; ++spin) {
           asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(ws + 10) : "memory");
           if (static_cast<uint32_t>(v >> 32) >= static_cast<uint32_t>(n_share)) break;
         }
-        sh.flag = spin < kSpinLimit ? 1 : 0;
+        sh.flag = spin < wait_limit ? 1 : 0;
         sh.push_base = static_cast<int>(static_cast<uint32_t>(v));
       }
       __syncthreads();
-      if (!sh.flag) ts.timed_out = true;
+      if (!sh.flag) lost = true;
       total = sh.push_base;
     } else if (C > 1) {
       cluster.sync();
@@ -1752,24 +1768,24 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
       total = sh.sort_count;
     }
     hinted_total = G > 1 ? min(total, kSortCap) : 0;
-    if (total >= k && total <= kSortCap) {
+    if (total >= k && total <= kSortCap && !(lost && may_give_up)) {
       hinted_done = true;
       expected_total = total;
       floor_comp = static_cast<uint64_t>(key_of(hint)) << 32;
       if (G > 1) {
         const uint64_t* gsurv = reinterpret_cast<const uint64_t*>(ws + kWsHeaderWords + kWsHistWords + kWsListWords);
-        if (!load_list_validated(gsurv, total, sortbuf)) ts.timed_out = true;
+        if (!load_list_validated(gsurv, total, sortbuf, wait_limit)) sh.lost = 1;
         if (my_share == 0 && tid == 0) sh.sort_count = total;
       }
     } else {
       // a caller's guess that did not fit is reported; the row's own guess is its own business
-      if (!self_seeded && p.status != nullptr && tid == 0 && my_share == 0) atomicOr(p.status, 8);
+      if (!self_seeded && !lost && p.status != nullptr && tid == 0 && my_share == 0) atomicOr(p.status, 8);
       if (tid == 0) sh.sort_count = 0;
     }
     if (tid == 0) sh.stage_count = 0;
     __syncthreads();
   }
-  if (!hinted_done) {
+  if (!hinted_done && !(lost && may_give_up)) {
   // ---- level 0: 13-bit histogram of the whole chunk -----------------------
   for (int i = tid; i < kMaxBins; i += kThreads) hist[i] = 0u;
   __syncthreads();
@@ -1809,7 +1825,8 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
       merge_two_step(cluster, C, hist, merged, r, sh, p);
     } else {
       merge_and_scan(cluster, C, rank, hist, merged, 1 << bits, r, raw0, sh, p, level == 0, G, ws, level,
-                     ts.timed_out, (level == 0 && !HAS_MAP) ? len : -1);
+                     lost, wait_limit, (level == 0 && !HAS_MAP) ? len : -1);
+      if (lost && may_give_up) break;
     }
     levels_used = level + 1;
     FF_TRACE(p, 2 + 3 * level);
@@ -1938,21 +1955,22 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
 
   if (G > 1) {
     const int n_load = (!hinted_done && ok) ? min(expected_total, kSortCap) : 0;
-    if (!hinted_done) {
+    if (!hinted_done && !(lost && may_give_up)) {
       // no barrier: the histogram told every CTA how many survivors to expect, and entries validate themselves
       const uint64_t* gsurv = reinterpret_cast<const uint64_t*>(ws + kWsHeaderWords + kWsHistWords);
-      if (!load_list_validated(gsurv, n_load, sortbuf)) ts.timed_out = true;
+      if (!load_list_validated(gsurv, n_load, sortbuf, wait_limit)) sh.lost = 1;
       __syncthreads();
       if (my_share == 0 && tid == 0) sh.sort_count = static_cast<int>(__ldcg(ws + 8));   // all of them have been reserved by now
     }
     __syncthreads();
+    lost = lost || sh.lost != 0;
     // Last use of the scratch: this CTA counts itself out; the CTA that does so last zeroes the
     // scratch for the next launch.  The atomic is issued here and its result looked at only when
     // the row is finished (leave_scratch below), so its round trip is off the critical path.
     n_plain_to_clear = hinted_done ? 0 : (ok ? n_load : kSortCap);
     if (tid == kScratchThread) {
       __threadfence();
-      counted_out_before = atomicAdd(ws + 7, 1u);
+      counted_out_before = atomicAdd(ws + 7, lost && may_give_up ? 0x10001u : 1u);
     }
   } else if (C > 1) {
     if (!hinted_done) cluster.sync();   // every survivor has landed in every CTA's list
@@ -1961,21 +1979,29 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
   }
   FF_TRACE(p, 20);
 
-  auto leave_scratch = [&]() {
-    if (G <= 1) return;
-    if (tid == kScratchThread) sh.flag = counted_out_before == static_cast<uint32_t>(n_share - 1) ? 1 : 0;
+  // Returns whether this CTA has to select the row alone.
+  auto leave_scratch = [&]() -> bool {
+    if (G <= 1) return false;
+    if (tid == kScratchThread)
+      sh.flag = (counted_out_before & 0xffffu) != static_cast<uint32_t>(n_share - 1) ? 0
+                : may_give_up && (lost || counted_out_before > 0xffffu)              ? 2
+                                                                                     : 1;
     __syncthreads();
+    const bool alone = sh.flag == 2;   // (then somebody may have left anything anywhere)
     if (sh.flag) {
-      for (int i = tid; i < kWsHeaderWords + levels_used * kMaxBins; i += kThreads) ws[i] = 0u;
+      for (int i = tid; i < kWsHeaderWords + (alone ? kNumLevels : levels_used) * kMaxBins; i += kThreads) ws[i] = 0u;
       // the lists must read as empty for the next launch (a failed select may have left any number of entries)
       uint32_t* lists = ws + kWsHeaderWords + kWsHistWords;
-      for (int i = tid; i < 2 * n_plain_to_clear; i += kThreads) lists[i] = 0u;
-      for (int i = tid; i < 2 * hinted_total; i += kThreads) lists[kWsListWords + i] = 0u;
+      for (int i = tid; i < (alone ? kWsListWords : 2 * n_plain_to_clear); i += kThreads) lists[i] = 0u;
+      for (int i = tid; i < (alone ? kWsListWords : 2 * hinted_total); i += kThreads) lists[kWsListWords + i] = 0u;
       if (kHinted && p.self_seed != 0) {
         if (tid < 2) ws[kWsSeedWord + tid] = 0u;
       }
     }
+    return alone;
   };
+  if (lost && may_give_up) return leave_scratch();   // (every copy that was asked for has been waited for: the waits lie behind whole sweeps or samples)
+  if (lost) ts.timed_out = true;
   if (ts.timed_out && p.status != nullptr && tid == 0) atomicOr(p.status, 2);
   if (!ok) {
     if (p.status != nullptr && tid == 0 && my_share == 0) atomicOr(p.status, 4);
@@ -1983,8 +2009,8 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
     if (my_share == 0) {
       for (int j = tid; j < k; j += kThreads) emit<kPush>(p, push, row, j, -1, 0u, HAS_MAP, table_row);
     }
-    leave_scratch();
-    return false;
+    const bool alone = leave_scratch();
+    return kSplit && alone;
   }
   const int n_surv = min(expected_total, kSortCap);
   const int hint_rank = min(n_surv, hint_target_rank(k)) - 1;
@@ -2067,8 +2093,8 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
       }
     }
     FF_TRACE(p, 25);
-    leave_scratch();
-    return sx_done;
+    const bool alone = leave_scratch();
+    return kSplit ? alone : sx_done;
   }
 
   // ---- finish: rank the n_surv survivors and write the first k ------------------
@@ -2262,8 +2288,34 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
     }
   }
   FF_TRACE(p, 25);
-  leave_scratch();
-  return sx_done;
+  const bool alone = leave_scratch();
+  return kSplit ? alone : sx_done;
+}
+
+// The row of a CTA that was the last to leave its scratch, some having given up a wait: one CTA selects it from the scores.
+// (By value: a reference would have every CTA keep its parameters in local memory, 16.1 instead of 12.7 us for 1 x 1 Mi.)
+template <typename T>
+__device__ __noinline__ void redo_row_alone(const TopkParams p, unsigned char* smem, ClusterShared& sh) {
+  TopkParams q = p;
+  const int row = (static_cast<int>(blockIdx.x) - p.block_base) / p.groups;
+  q.block_base = static_cast<int32_t>(blockIdx.x) - row;   // (the row of CTA b is b - block_base there)
+  q.groups = 1;
+  q.workspace = nullptr;
+  q.self_seed = 0;
+  q.hint_in = nullptr;
+  q.handover = nullptr;
+  q.wait_limit = 0;
+  q.trace = nullptr;
+  __syncthreads();   // every thread has left the first attempt, whose copies have all arrived
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(&sh.bars[s])) : "memory");
+      asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_addr(&sh.ebars[s])) : "memory");
+    }
+  }
+  __syncthreads();
+  const PushCtx push = {0, 0u};
+  (void)topk_row_body<false, kModeHinted, T>(q, smem, sh, push);
 }
 
 // One CTA's whole job for one rank: the row body, and in context-parallel send mode the step
@@ -2283,6 +2335,10 @@ __device__ __forceinline__ void topk_cta(const TopkParams& p, unsigned char* sme
     push.off = (static_cast<int64_t>(push.step & 1u) * p.push_world + p.push_rank) * p.push_slot_words;
   }
   const bool written = topk_row_body<HAS_MAP, MODE, T>(p, smem, sh, push);
+  if constexpr ((MODE & kModeSplit) != 0) {
+    if (__builtin_expect(written, 0)) redo_row_alone<T>(p, smem, sh);
+    return;
+  }
   if (kPush && !HAS_MAP && p.push_world > 0) {
     FF_TRACE(p, 32);
     // Every CTA read the step long ago; the one that counts itself last advances the counter.

@@ -312,6 +312,13 @@ int ff_topk_set_self_seed(int32_t on);
  * launches with the cluster attribute only, topk_indexer_radix.cu:1195-1233). */
 int ff_topk_set_programmatic_launch(int32_t on);
 
+/* Rows split over single CTAs are launched without the promise that all of them run at the same time.  They normally do;
+ * a CTA that has waited for the others for `polls` reads of memory (about a microsecond each; default 16,384) leaves, and the
+ * last CTA to leave selects the row alone, so that the result is exact either way.  polls <= 0: the default.
+ * Process-wide, for tests.  No reference counterpart (the reference's CTAs of one row are one cluster,
+ * topk_indexer_radix.cu:1195-1233). */
+int ff_topk_set_wait_limit(int32_t polls);
+
 /* The cluster size the automatic policy picks for (B, L_width, k) on the
  * current device (after overrides) when a row stays inside ONE cluster (no
  * workspace).  For the shape of an actual launch use ff_topk_policy_launch_shape. */
@@ -321,9 +328,8 @@ int32_t ff_topk_policy_cluster_size(int32_t B, int64_t L_width, int32_t k);
  * (hinted != 0) uses for (B, L_width, k) on the current device: out2[0] = CTAs
  * per cluster, out2[1] = clusters per row (more than one only with workspace of
  * ff_topk_workspace_bytes; pass has_workspace = 0 for a call without).  The
- * grid is B * out2[0] * out2[1] CTAs.  A captured launch of fp32 scores may split rows of
- * small batches where this one does not (from 128 Ki + 32 k instead of 256 Ki + 64 k columns: a
- * cooperative launch outside a graph starts late).  Plays the role of reading the reference's
+ * grid is B * out2[0] * out2[1] CTAs.  A captured launch of fp32 scores with k > 1024
+ * may split rows of small batches where this one does not (from 128 Ki + 32 k instead of 256 Ki columns).  Plays the role of reading the reference's
  * split policy off its launcher (topk_indexer_radix.cu:1309-1321). */
 int ff_topk_policy_launch_shape(int32_t B, int64_t L_width, int32_t k, int32_t has_workspace, int32_t hinted,
                                 int32_t* out2);

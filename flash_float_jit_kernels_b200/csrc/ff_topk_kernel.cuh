@@ -394,17 +394,16 @@ __device__ __forceinline__ typename HitMask<T>::type tile_hits(uint32_t tile, in
   constexpr int kPU = Elem<T>::kPerUnit;
   using Mask = typename HitMask<T>::type;
   Mask hits = 0;
+  // (Rolled: a row goes through this code a few times, and fetching eight units' worth of it took longer than running two of them
+  // four times.  1 x 8 Mi columns 16.9 us, unrolled by four 16.6, by two 16.2.)
+#pragma unroll 2
+  for (int lu = static_cast<int>(threadIdx.x), shift = 0; lu < units; lu += kThreads, shift += kPU) {
+    float v[kPU];
+    unpack_unit<T>(lds_u4(tile + 16u * static_cast<uint32_t>(lu)), v);
+    uint32_t h = 0u;
 #pragma unroll
-  for (int j = 0; j < kTileUnits / kThreads; ++j) {
-    const int lu = static_cast<int>(threadIdx.x) + j * kThreads;
-    if (lu < units) {
-      float v[kPU];
-      unpack_unit<T>(lds_u4(tile + 16u * static_cast<uint32_t>(lu)), v);
-      uint32_t h = 0u;
-#pragma unroll
-      for (int e = 0; e < kPU; ++e) h |= (!(v[e] < vmin) ? 1u : 0u) << e;
-      hits |= static_cast<Mask>(h) << (kPU * j);
-    }
+    for (int e = 0; e < kPU; ++e) h |= (!(v[e] < vmin) ? 1u : 0u) << e;
+    hits |= static_cast<Mask>(h) << shift;
   }
   return hits;
 }
@@ -960,6 +959,8 @@ struct SeedPlan {
   float p;         // target / length
   int n_use;       // 16-byte units of a CTA's first tile that it looks at
 };
+// log(1 - p) for p up to a quarter, to a thousandth.
+__device__ __forceinline__ float log1m(float p) { return -p * (1.f + p * (0.5f + p * (0.3333333f + p * (0.25f + 0.3f * p)))); }
 // Row-level decision, from quantities every CTA of the row computes alike.
 // len_for_p: the length the target count refers to (the whole row's in a context-parallel step,
 // where `len` is the shard's).
@@ -974,7 +975,7 @@ __device__ __forceinline__ SeedPlan seed_plan(int len, int mis, int per_unit, in
   const int target = min(ranks > 1 ? k + (k >> 1) : n_share < 16 ? k + (k >> 2) + (k >> 3) + 64 : k + (k >> 2) + 64,
                          kSortCap - (kSortCap >> 3));
   if (len_for_p <= 0) len_for_p = len;
-  sp.p = static_cast<float>(target) / static_cast<float>(len_for_p);
+  sp.p = __fdividef(static_cast<float>(target), static_cast<float>(len_for_p));
   sp.n_use = 0;
   if (n_share > kThreads || len_for_p < 4 * target) return sp;   // (the accumulator's counters hold up to 1023)
   const int U = static_cast<int>((static_cast<int64_t>(len) + mis + per_unit - 1) / per_unit);
@@ -984,7 +985,7 @@ __device__ __forceinline__ SeedPlan seed_plan(int len, int mis, int per_unit, in
   auto rho_of = [&](int units) {
     const int lanes = min(kThreads, units);
     const float g = static_cast<float>(per_unit) * static_cast<float>(units) / static_cast<float>(lanes);
-    return static_cast<float>(lanes) * (1.f - __expf(g * log1pf(-sp.p)));
+    return static_cast<float>(lanes) * (1.f - __expf(g * log1m(sp.p)));
   };
   float rho = rho_of(n0);
   if ((rho < 4.5f || rho * static_cast<float>(n_share) * static_cast<float>(ranks) < 400.f) && per > kTileUnits) {
@@ -996,10 +997,10 @@ __device__ __forceinline__ SeedPlan seed_plan(int len, int mis, int per_unit, in
   if (rho > 28.f) {
     // more hits than the kept 32 can show: look at as much of the tile as lets 27 of the threads' maxima reach the
     // wanted score (fewer units than threads where one unit per thread would show more)
-    const float g = log1pf(-27.f / static_cast<float>(kThreads)) / log1pf(-sp.p);   // scores per thread
+    const float g = __fdividef(log1m(27.f / static_cast<float>(kThreads)), log1m(sp.p));   // scores per thread
     const int units = static_cast<int>(g >= static_cast<float>(per_unit)
                                            ? g * static_cast<float>(kThreads / per_unit)
-                                           : 27.f / (1.f - __expf(static_cast<float>(per_unit) * log1pf(-sp.p))));
+                                           : __fdividef(27.f, 1.f - __expf(static_cast<float>(per_unit) * log1m(sp.p))));
     n0 = min(n0, max(units, 64));
     rho = rho_of(n0);
   }
@@ -1073,7 +1074,7 @@ __device__ __noinline__ SeedResult seed_own_guess(uint32_t tile0, int n0, int* f
   float pos = 0.f;
   if (lanes >= 32) {
     const float g = static_cast<float>(kPU) * static_cast<float>(n0) / static_cast<float>(lanes);
-    const float rho = static_cast<float>(lanes) * (1.f - __expf(g * log1pf(-p_frac)));
+    const float rho = static_cast<float>(lanes) * (1.f - __expf(g * log1m(p_frac)));
     pos = fminf(fmaxf(rho - 0.5f, 0.f), 30.99f);
   }
   // ---- largest score per thread over the first tile of the chunk ----
@@ -1081,16 +1082,13 @@ __device__ __noinline__ SeedResult seed_own_guess(uint32_t tile0, int n0, int* f
   if (n0 > 0) {
     float m = __uint_as_float(0xff800000u);
     bool any = false;
+#pragma unroll 4
+    for (int lu = tid; lu < n0; lu += kThreads) {   // (the ring's two stages are contiguous)
+      float v[kPU];
+      unpack_unit<T>(lds_u4(tile0 + 16u * static_cast<uint32_t>(lu)), v);
 #pragma unroll
-    for (int j = 0; j < 2 * kTileUnits / kThreads; ++j) {   // (the ring's two stages are contiguous)
-      const int lu = tid + j * kThreads;
-      if (lu < n0) {
-        float v[kPU];
-        unpack_unit<T>(lds_u4(tile0 + 16u * static_cast<uint32_t>(lu)), v);
-#pragma unroll
-        for (int e = 0; e < kPU; ++e) m = fmaxf(m, v[e]);   // (NaN scores are left out of the estimate)
-        any = true;
-      }
+      for (int e = 0; e < kPU; ++e) m = fmaxf(m, v[e]);   // (NaN scores are left out of the estimate)
+      any = true;
     }
     if (any) mkey = key_of(m);
   }
@@ -1151,7 +1149,7 @@ __device__ __noinline__ SeedResult seed_own_guess(uint32_t tile0, int n0, int* f
     const int valid = static_cast<int>((v >> 44) & 1023ull);
     // the mean of the keys (keys are close to linear in the score over so narrow a range)
     uint32_t mean = 0u;
-    if (spin < limit && 2 * valid >= n_share) mean = static_cast<uint32_t>((v & ((1ull << 44) - 1ull)) / static_cast<unsigned long long>(valid));
+    if (spin < limit && 2 * valid >= n_share) mean = static_cast<uint32_t>(__fdividef(static_cast<float>(v & ((1ull << 44) - 1ull)), static_cast<float>(valid)));
     *flag = spin < limit ? 1 : 0;
     scratch[0] = mean;
   }
@@ -1386,6 +1384,9 @@ __device__ __forceinline__ bool topk_row_body(const TopkParams& p, unsigned char
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
   }
+
+  // The first tile is on its way while the rest is set up and the guess is planned (every path of such a row sweeps it).
+  if (kSplit && G > 1 && p.handover == nullptr && ts.n_tiles > 0) stream_fetch(ts, 0);
 
   // ---- context-parallel step by exchange of survivors ----------------------------------------
   // Instead of ranking its own candidates, sending the sorted run and merging runs, every rank

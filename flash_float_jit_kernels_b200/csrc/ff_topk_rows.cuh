@@ -114,7 +114,7 @@ struct RowsShared {
   uint32_t kmin, kmax;     // bounds of the survivors' keys (rebuilt bins only)
   int last_pos;            // a crowded lowest bin of those: last position,
   uint32_t low_bits;       // and OR of the keys' distances from the smallest
-  uint32_t max_bucket;     // survivors in the largest finish bin
+  uint32_t max_bucket;     // survivors in the largest finish bin, if more than five
 };
 
 // Sum of v over all threads of higher index; `total`: over all threads.  One barrier; calls that
@@ -419,7 +419,9 @@ __device__ __forceinline__ int warp_inclusive(int v) {
 // Sweep 2: every score not below vmin (EXACT: whose composite is not below floor_comp) goes to the list.
 // `g` is the row's first group, still in registers.  A warp takes a group of its lanes' at a time: a scan over the lanes' hit
 // counts, one shared atomic for the warp's slots, and predicated stores (no hit mask: testing a score
-// again is one instruction, picking its bit out of a mask three).
+// again is one instruction, picking its bit out of a mask three.  Rows with few hits too: going by hits, with one hit of every lane a
+// round, took 11.5 instead of 10.8 us for 59 rows of 60 Ki with guesses, k = 512, 20.9 instead of 20.4 for 64 x 128 Ki in clusters of
+// four, and only 23.6 instead of 24.2 for 90 x 128 Ki.)
 template <typename T, int NT, int S, int CAP, bool EXACT>
 __device__ __forceinline__ void collect_row(const Chunk<T>& c, RowGroup<T, NT, S>& g, float vmin, uint64_t floor_comp,
                                             RowList<CAP> list, RowsShared& sh) {
@@ -472,53 +474,6 @@ __device__ __forceinline__ void collect_row(const Chunk<T>& c, RowGroup<T, NT, S
       if (at < CAP) {
         list.put(at, x, pos);
       }
-    }
-  }
-}
-
-// Sweep 2 of a row in which few scores are hits: a warp's lanes store one hit each per round, for as many rounds as
-// one of them has hits among its 16 scores, reading the score again instead of going through the registers.
-template <typename T>
-__device__ __forceinline__ float score_at(const T* p) {
-  if constexpr (Elem<T>::kPerUnit == 4) return __ldg(p);
-  else return Elem<T>::from_bits16(__ldg(reinterpret_cast<const unsigned short*>(p)));
-}
-template <typename T, int NT, int S, int CAP>
-__device__ __noinline__ void collect_row_sparse(const Chunk<T>& c, float vmin, RowList<CAP> list, RowsShared& sh) {
-  using Group = RowGroup<T, NT, S>;
-  const int lane = threadIdx.x & 31;
-#pragma unroll 1
-  for (int u0 = c.fb; u0 < c.fe; u0 += Group::kStep) {
-    Group g;
-    g.load(c, u0);
-    const int pos0 = Group::position(c, u0);
-    uint32_t hits = 0u;
-    auto test = [&](float x, int e) {
-      if (!(x < vmin)) hits |= 1u << e;
-    };
-    if (u0 + Group::kStep <= c.fe) g.template each<true>(c, u0, test); else g.template each<false>(c, u0, test);
-    const int total = static_cast<int>(__reduce_add_sync(0xffffffffu, static_cast<uint32_t>(__popc(hits))));
-    if (total == 0) continue;
-    int base = 0;
-    if (lane == 0) base = atomicAdd(&sh.count, total);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base + total > CAP) continue;
-    for (uint32_t more = __ballot_sync(0xffffffffu, hits != 0u); more != 0u; more = __ballot_sync(0xffffffffu, hits != 0u)) {
-      if (hits != 0u) {
-        const int e = __ffs(static_cast<int>(hits)) - 1;
-        hits &= hits - 1u;
-        const int pos = pos0 + Group::distance(e);
-        list.put(base + __popc(more & ((1u << lane) - 1u)), score_at(c.abase + (pos + c.mis)), pos);
-      }
-      base += __popc(more);
-    }
-  }
-  if (c.head || c.tail) {   // (uniform)
-    float x = 0.f;
-    const int pos = partial_element(c, x);
-    if (pos >= 0 && !(x < vmin)) {
-      const int at = atomicAdd(&sh.count, 1);
-      if (at < CAP) list.put(at, x, pos);
     }
   }
 }
@@ -810,9 +765,6 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     if (CLUSTER) cluster_barrier();
   };
 
-  // Where so few scores are hits, going by hits instead of by scores is faster (1 x 128 Ki, one CTA: 23.8 -> 21.5 us; 64 x
-  // 128 Ki, k = 512, four CTAs a row: 21.4 -> 20.2), with four CTAs on an SM (256 threads) it is not.
-  const bool sparse = NT > 256 && len / k > (CLUSTER ? 128 : 48);
   int n = 0;                    // survivors in the list
   bool listed = false;          // ... found with a guess
   if constexpr (HINTS) {
@@ -836,12 +788,9 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
         header[0] = header[1] = 0u;   // empty for the producer's next launch
       }
     } else if (use) {
-      if (sparse) collect_row_sparse<T, NT, kGroup, kCap>(chunk, hint, own_list, sh);
-      else {
-        Group g;
-        g.load(chunk, chunk.fb);
-        collect_row<T, NT, kGroup, kCap, false>(chunk, g, hint, 0ull, own_list, sh);
-      }
+      Group g;
+      g.load(chunk, chunk.fb);
+      collect_row<T, NT, kGroup, kCap, false>(chunk, g, hint, 0ull, own_list, sh);
       n = gather();
       listed = n >= k && n <= kCap;
       if (!listed) {
@@ -900,8 +849,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
     bool exact = bin_key > 0xff800000u || sh.max_bin > kPackMax || keep < k - above ||
                  (sh.total > kCap && 8 * sh.max_bin > 7 * sh.total);
     if (!exact) {
-      if (sparse) collect_row_sparse<T, NT, kGroup, kCap>(chunk, prefilter_value(sh.cut), own_list, sh);
-      else if (HINTS) collect_row_again<T, NT, kGroup, kCap>(chunk, prefilter_value(sh.cut), own_list, sh);   // (rare: out of the way)
+      if (HINTS) collect_row_again<T, NT, kGroup, kCap>(chunk, prefilter_value(sh.cut), own_list, sh);   // (rare: out of the way)
       else collect_row<T, NT, kGroup, kCap, false>(chunk, first, prefilter_value(sh.cut), 0ull, own_list, sh);
       n = gather();
       span = above + keep;
@@ -1104,8 +1052,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
       local += (v[q].x + v[q].y) + (v[q].z + v[q].w);
       largest = max(max(max(v[q].x, v[q].y), max(v[q].z, v[q].w)), largest);
     }
-    largest = __reduce_max_sync(0xffffffffu, largest);
-    if ((tid & 31) == 0) atomicMax(&sh.max_bucket, largest);
+    if (largest > 5u) atomicMax(&sh.max_bucket, largest);   // (up to five are ranked the same way)
     int total;
     const int after = suffix_exclusive<NT>(static_cast<int>(local), sh.warp_tot[1], total);
     uint32_t start = static_cast<uint32_t>(total - after) - local;
@@ -1138,7 +1085,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   const uint32_t max_bucket = sh.max_bucket;
   if (max_bucket <= 5u) {
     rank_blocks<NT, rows_block_slots(PER), 4>(sorted, n, ranked);
-  } else if (max_bucket <= 7u) {
+  } else if (!HINTS && max_bucket <= 7u) {   // (with guesses the code of it takes longer to pass than it saves)
     rank_blocks<NT, rows_block_slots(PER), 6>(sorted, n, ranked);
   } else {
     rank_crowded<NT, PER>(sorted, bins, 2 * span, n, ranked, p.status);

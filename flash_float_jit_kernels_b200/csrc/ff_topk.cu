@@ -349,13 +349,15 @@ int launch(const ff::TopkParams& p, int cluster, cudaStream_t stream, int dtype 
 }
 
 // The one-CTA-per-row kernels (ff_topk_rows.cuh), by score type, CTA size and guesses.
-// Lists of 2,560 and 3,072 survivors: k, a margin inside the threshold digit, room to spare; a caller's guess may
+// Lists of 2,512 to 3,072 survivors: k, a margin inside the threshold digit, room to spare; a caller's guess may
 // let 4,096 through.
 // A shape is the threads per CTA, negative and with the cluster size in front of it for a cluster per row
 // (-80512: eight CTAs of 512 threads).
 int shape_threads(int shape) { return (shape < 0 ? -shape : shape) % 10000; }
 int shape_cluster(int shape) { return shape < 0 ? -shape / 10000 : 1; }
-int rows_cap(int shape, bool hints) { return hints ? ff::kSortCap : shape_threads(shape) == 1024 ? 1024 * 3 : 256 * 10; }
+int rows_cap(int shape, bool hints) {
+  return hints ? ff::kSortCap : shape_threads(shape) == 1024 ? ff::rows_list_cap(1024, 3) : shape < 0 ? ff::rows_list_cap(512, 5) : ff::rows_list_cap(256, 10);
+}
 int rows_block(int shape, bool hints) { return shape_threads(shape) == 256 && hints ? 512 : shape_threads(shape); }
 template <typename T>
 RowsKernel rows_kernel(int shape, bool hints) {

@@ -50,13 +50,17 @@ constexpr int kRowsBins = 1 << kRowsBits;
 constexpr int kRowsShift = 32 - kRowsBits;
 
 // Shared memory of a CTA whose list holds `cap` survivors, in two regions:
-//   histogram, then the survivors bucket by bucket (64 bits each)
 //   list (64 bits each), then two finish bins per survivor (32 bits each), then the ranked positions
+//   histogram, then the survivors bucket by bucket (64 bits each)
 // and in a cluster the row's histogram and this CTA's own list behind them.
-constexpr int kRankPad = 8;                       // slots in front of and behind the sorted survivors
+constexpr int kRankPad = 8;                       // slots in front of the sorted survivors, and half of those behind them
 __host__ __device__ constexpr int rows_table_bytes(int cap) {
-  return kRowsBins * 4 > (cap + 2 * kRankPad) * 8 ? kRowsBins * 4 : (cap + 2 * kRankPad) * 8;
+  return kRowsBins * 4 > (cap + 3 * kRankPad) * 8 ? kRowsBins * 4 : (cap + 3 * kRankPad) * 8;
 }
+// Survivors the list of NT threads with PER places each takes.  Where four CTAs share an SM, 48 fewer than there are places: with those
+// the four do not fit 164 KiB, the next size that an SM divides its memory by is 196, and of the L1 that is left fewer page-table
+// entries are hits (1,024 rows of 4.1 Ki scores with page table 28.5 us, before the survivors were sorted 27.8).
+__host__ __device__ constexpr int rows_list_cap(int nt, int per) { return nt == 256 ? nt * per - 48 : nt * per; }
 __host__ __device__ constexpr int rows_smem_bytes(int cap, bool cluster) {
   return rows_table_bytes(cap) + cap * 8 + (cluster ? kRowsBins * 4 + cap * 8 : 0);
 }
@@ -531,7 +535,7 @@ __host__ __device__ constexpr int rows_block_slots(int per) { return per >= 8 ? 
 // the smallest and the largest word.)
 template <int NT, int BLOCK, int W>
 __device__ __forceinline__ void rank_blocks(const uint64_t* sorted, int n, int32_t* ranked) {
-  static_assert(BLOCK % 2 == 1 && W <= kRankPad, "conflict-free loads, inside the padding");
+  static_assert(BLOCK % 2 == 1 && W <= kRankPad && BLOCK + W - 1 <= 2 * kRankPad, "conflict-free loads, inside the padding");
 #pragma unroll 1
   for (int s0 = static_cast<int>(threadIdx.x) * BLOCK; s0 < n; s0 += NT * BLOCK) {
     uint64_t e[BLOCK + 2 * W];
@@ -576,7 +580,7 @@ __device__ __noinline__ void rank_crowded(const uint64_t* sorted, const uint32_t
       const uint64_t own = sorted[slot];
       const uint32_t first = b == 0 ? 0u : bins[b - 1], end = bins[b];
       rank[j] = first;
-      if (FF_IN_RANGE(p, static_cast<int>(end) - 1, PER * NT, 17)) {
+      if (FF_IN_RANGE(p, static_cast<int>(end) - 1, rows_list_cap(NT, PER), 17)) {
 #pragma unroll 1
         for (uint32_t q = first; q < end; ++q) rank[j] += sorted[q] < own ? 1u : 0u;
       }
@@ -586,7 +590,7 @@ __device__ __noinline__ void rank_crowded(const uint64_t* sorted, const uint32_t
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
     const int slot = static_cast<int>(threadIdx.x) + j * NT;
-    if (slot < n && FF_IN_RANGE(p, rank[j], PER * NT, 18)) ranked[rank[j]] = static_cast<int32_t>(static_cast<uint32_t>(sorted[slot]));
+    if (slot < n && FF_IN_RANGE(p, rank[j], rows_list_cap(NT, PER), 18)) ranked[rank[j]] = static_cast<int32_t>(static_cast<uint32_t>(sorted[slot]));
   }
   (void)p;
 }
@@ -603,13 +607,13 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   constexpr int kGroup = rows_group(CLUSTER, HINTS);
   using Group = RowGroup<T, NT, kGroup>;
   constexpr int kPU = Elem<T>::kPerUnit;
-  constexpr int kCap = PER * NT;
-  uint32_t* hist = reinterpret_cast<uint32_t*>(smem);
-  uint64_t* sorted = reinterpret_cast<uint64_t*>(smem) + kRankPad;           // kCap survivors, bucket by bucket
-  const RowList<kCap> list = {reinterpret_cast<float*>(smem + rows_table_bytes(kCap))};
+  constexpr int kCap = rows_list_cap(NT, PER);
+  const RowList<kCap> list = {reinterpret_cast<float*>(smem)};
+  uint32_t* hist = reinterpret_cast<uint32_t*>(smem + kCap * 8);
+  uint64_t* sorted = reinterpret_cast<uint64_t*>(hist) + kRankPad;           // kCap survivors, bucket by bucket
   uint32_t* bins = reinterpret_cast<uint32_t*>(list.x);                      // 2 * kCap finish bins
   int32_t* ranked = reinterpret_cast<int32_t*>(list.x);                      // kCap positions
-  uint32_t* merged = CLUSTER ? reinterpret_cast<uint32_t*>(list.x + 2 * kCap) : hist;
+  uint32_t* merged = CLUSTER ? hist + rows_table_bytes(kCap) / 4 : hist;
   const RowList<kCap> own_list = {CLUSTER ? reinterpret_cast<float*>(merged + kRowsBins) : list.x};
   const uint32_t C = CLUSTER ? cluster_size() : 1u, rank = CLUSTER ? cluster_rank() : 0u;
   const int tid = threadIdx.x;
@@ -905,7 +909,7 @@ __global__ void __launch_bounds__(NT, CTAS) topk_rows_kernel(const RowsParams p)
   };
 #pragma unroll
   for (int j = kHalf; j < PER; ++j) pos[j] = -1;
-  mine([&](int j) {   // (behind the n survivors the list holds anything)
+  mine([&](int j) {   // (behind the n survivors the list, and the table behind it, hold anything)
     const uint2 entry = reinterpret_cast<const uint2*>(list.x)[tid + j * NT];
     pos[j] = tid + j * NT < n ? static_cast<int32_t>(entry.y) : -1;
     bits[j] = __float_as_uint(__fadd_rn(__uint_as_float(entry.x), 0.0f));

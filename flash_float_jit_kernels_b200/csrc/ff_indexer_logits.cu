@@ -396,11 +396,14 @@ __global__ void __launch_bounds__(kThreads, 2) indexer_logits_kernel(const Param
 //     its first key, where the copy fills in zeros);
 //   * one thread issues the tensor-core instructions;
 //   * four epilogue warps as above; in front of their first tile they also write the -inf of a fresh result.
-// Bound by the K bytes: 64 full rows of 131,072 keys 179.7 us (6.16 TB/s, 94 % of the measured copy peak), lengths
-// U[8192, 131072] 98.6 us (5.93 TB/s).  Shares of up to 32 tiles dealt out by the hardware (indexer_logits_kernel: each
+// Bound by the K bytes: batches of 64 ragged rows in turn (lengths U[4096, 131072], about 600 MB a call), 104 us, 5.8 TB/s with what is
+// written, 89 % of the measured copy peak; four and five tiles in flight per CTA alike, three 1 % slower, two 4 %, one CTA on an SM with six or
+// eight 30 %, three CTAs with two or three 1 to 3 %.  Four, because small calls like fewer (a step of 16 rows of 40,000 keys 24.2 us
+// with four, 24.8 with five).
+// Shares of up to 32 tiles dealt out by the hardware (indexer_logits_kernel: each
 // share sets up barriers and tensor memory, loads q and fills its pipeline again, and the last wave is ragged)
 // took 180.8 and 114.9 us, and 14.5 instead of 10.7 us for 16 ragged rows of 40,000.
-constexpr int kRunStages = 5;
+constexpr int kRunStages = 4;
 constexpr int kRunMaxRows = FF_INDEXER_MAX_FILL_ROWS;
 constexpr int kRunThreads = (kEpilogueWarps + 2) * 32;
 constexpr int kRunProducerWarp = kEpilogueWarps + 1;
@@ -498,6 +501,8 @@ __global__ void __launch_bounds__(kRunThreads, 2) indexer_logits_run_kernel(cons
     }
     sh.timed_out = 0;
     sh.prefix[0] = 0;
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&k_map) : "memory");   // (parameters of this launch)
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&q_map) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -164,12 +164,12 @@ def test_rows_that_end_at_a_group(oracle, B, L, k):
 
 @pytest.mark.parametrize("B,L,k", [(18, 16384, 2048), (160, 5461, 2048), (18, 40960, 1024), (160, 4000, 300)])
 @pytest.mark.parametrize("guess", [False, True])
-def test_buckets_of_two_to_ten(oracle, B, L, k, guess):
+def test_buckets_of_one_to_a_dozen(oracle, B, L, k, guess):
     """Every score occurs r times, far apart and with a full mantissa, so that the largest bucket holds r and a few more: ranks
-    from the neighbours up to four and up to six slots away, and from a bucket that is looked up."""
+    from the neighbours up to four and up to eight slots away, and from a bucket that is looked up."""
     from flash_float_jit_kernels_b200 import new_threshold_hint
     g = torch.Generator().manual_seed(B + L)
-    s = torch.stack([torch.randn((L // (1 + i % 9) + 1,), generator=g).repeat(10)[:L] for i in range(B)])
+    s = torch.stack([torch.randn((L // (1 + i % 11) + 1,), generator=g).repeat(12)[:L] for i in range(B)])
     lengths = torch.full((B,), L, dtype=torch.int32)
     hint = new_threshold_hint(B, "cuda") if guess else None
     for _ in range(2 if guess else 1):

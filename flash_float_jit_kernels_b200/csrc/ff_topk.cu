@@ -207,7 +207,7 @@ int choose_cluster(int device, int32_t B, int64_t L_width, int32_t k) {
 // global memory.  Returns the number of clusters per row and may lower `cluster`.
 //
 // Clusters of ONE CTA, launched plainly (kGiveUpAfter): a cooperative launch outside a graph starts on a 2.048 us beat behind the
-// kernel in front of it (call by call, clusters of two in a cooperative launch : now, 1 x 1 Mi 14.3 : 12.8 us, 1 x 8 Mi 18.4 :
+// kernel in front of it (call by call, clusters of two in a cooperative launch : this, when it came, 1 x 1 Mi 14.3 : 12.8 us, 1 x 8 Mi 18.4 :
 // 18.2, 4 x 1 Mi, k = 512, 14.4 : 13.0), and clusters of two leave SMs over where the batch does not divide 74 (4 x 1 Mi 13.0 : 12.7).
 //   * Rows that make their own guess are swept once: split rows of 256 Ki columns take 13.5 us (B = 2), 13.8 (B = 4), 14.5
 //     (B = 8), 16.2 (B = 16), against 14.5, 14.7, 16.5 and 23.3 in one cluster each.  The guess needs about 200 hits
@@ -421,7 +421,8 @@ int launch_rows(const ff::TopkParams& p, int shape, cudaStream_t stream, int dty
 }
 
 // Shape of topk_rows_kernel for this batch, or 0: the kernel of ff_topk_kernel.cuh (also whenever a launch shape is
-// forced; `split`: that one would split the row over several clusters; `half`: 16-bit scores).  Measured on B200, k = 2048, us in
+// forced; `split`: that one would split the row over several clusters; `half`: 16-bit scores).  Measured on B200, k = 2048 (before the
+// finish ranked survivors among their neighbours, since when the shapes of topk_rows_kernel take 5 to 15 % less; no line moved), us in
 // a graph, full rows N(0, 1) / ragged rows of logits (lengths from 4 Ki up):
 //   * more rows than SMs: four CTAs of 256 threads per SM (296 rows of 16 Ki: 14.6 against 18.9 with one CTA of 1024), unless
 //     the rows are long: at four to an SM they do not stay in L2 for the second sweep (297 rows of 128 Ki 100.8 / 71.0 against

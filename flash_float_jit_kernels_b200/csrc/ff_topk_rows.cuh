@@ -13,9 +13,9 @@
 //             of neighbours that are not; indices leave through shared memory
 //
 // What bounds it: batches of many rows keep issue slots and the shared-memory pipe about 60 % busy each (4,096 rows of 5,461
-// scores, k = 2048: 88.2 us; 104.3 with survivors ranked by a walk of each one's bucket, sixteen scores to a group of the sweeps and
+// scores, k = 2048: 88.6 us, 15,300 warp instructions and 3,950 shared-memory wavefronts per row; 103.7 with survivors ranked by a walk of each one's bucket, sixteen scores to a group of the sweeps and
 // the cut worked out by every thread; the kernel of ff_topk_kernel.cuh, one row per SM, took 455); a single row is a chain of
-// eight phases, 8.7 us for 16 Ki scores (9.1; 12.5 in a cluster of sixteen CTAs of the other kernel).  Hence 64 registers and
+// eight phases, 8.5 us for 16 Ki scores (9.1; 12.5 in a cluster of sixteen CTAs of the other kernel).  Hence 64 registers and
 // 40 KiB per row, four rows on an SM.
 #pragma once
 
